@@ -212,3 +212,75 @@ _REL = {"gemm": 7e-3, "mlp": 7e-3, "fp8": 7e-3, "mx": 7e-3, "bs": 7e-3, "ring": 
 
 def tolerance(case):
     return {"rel": _REL[case["path"]]}
+
+
+def _q64(x, rows, pow2=False):
+    """bf16 [r, K] -> the fp64 values of its e4m3 form with one scale per ``rows`` rows and 128
+    columns (fp32 scales amax / 448, rounded up to a power of two with ``pow2``): the quantisation
+    is part of the measured call, so the exact result is that of the quantised operands."""
+    r, k = x.shape
+    pad = (-r) % rows
+    f = torch.nn.functional.pad(x.float(), (0, 0, 0, pad)).view((r + pad) // rows, rows, k // 128, 128)
+    amax = f.abs().amax(dim=(1, 3), keepdim=True)
+    # a tensor divided by a number is multiplied by its reciprocal on a GPU; divide in earnest
+    s = torch.where(amax > 0, amax / torch.full_like(amax, 448.0), torch.ones_like(amax))
+    if pow2:
+        m, e = torch.frexp(s)                        # s = m * 2^e, m in [0.5, 1)
+        s = torch.ldexp(torch.ones_like(s), torch.where(m == 0.5, e - 1, e))
+    q = (f * (1.0 / s)).to(torch.float8_e4m3fn)
+    return (q.double() * s.double()).view(r + pad, k)[:r]
+
+
+def _attention64(q, k, v, causal, q_offset):
+    """(o, lse) of [B, S, H, 128] tensors in 64 bits, one head and 2048 queries at a time."""
+    b, sq, hq, d = q.shape
+    skv, hkv = k.shape[1], k.shape[2]
+    o = torch.empty(b, sq, hq, d, dtype=torch.float64, device=q.device)
+    lse = torch.empty(b, hq, sq, dtype=torch.float64, device=q.device)
+    cols = torch.arange(skv, device=q.device)
+    for bi in range(b):
+        for h in range(hq):
+            kh, vh = (t[bi, :, h // (hq // hkv)].double() for t in (k, v))
+            for r in range(0, sq, 2048):
+                s = q[bi, r:r + 2048, h].double() @ kh.t() / math.sqrt(d)
+                if causal:
+                    rows = torch.arange(r, r + s.shape[0], device=q.device)[:, None] + q_offset
+                    s.masked_fill_(cols[None, :] > rows, float("-inf"))
+                ls = torch.logsumexp(s, dim=-1)
+                lse[bi, h, r:r + 2048] = ls
+                o[bi, r:r + 2048, h] = torch.exp(s - ls[:, None]) @ vh
+    return o, lse
+
+
+def exact(case, seed):
+    path = case["path"]
+    s = prepare(case, seed)
+    if path == "gemm":
+        return s.x.double() @ s.w.double().t()
+    if path == "fp8":
+        return s.alpha * (s.x.double() @ s.w.double().t())
+    if path in ("mx", "bs"):
+        # the weight as prepare() drew it, right after the activation
+        dev = s.x.device
+        g = torch.Generator(device=dev).manual_seed(seed)
+        torch.randn(case["m"], case["k"], device=dev, generator=g)
+        w = (torch.randn(case["n"], case["k"], device=dev, generator=g) * 0.02).bfloat16()
+        return _q64(s.x, 1, path == "mx") @ _q64(w, 128, path == "mx").t()
+    if path == "mlp":
+        return (s.x.double() @ s.layer.w1.double().t()) @ s.layer.w2.double().t()
+    if path == "ring":
+        return _attention64(s.q, s.op.k_local(), s.op.v_local(), s.causal, 0)
+    if path == "attn":
+        return _attention64(s.q, s.k, s.v, s.causal, s.q_offset)
+    w1, w2 = s.layer.weights()
+    top, idx = torch.topk(torch.softmax(s.logits.double(), dim=1), s.topk, dim=1)
+    weight = top / top.sum(dim=1, keepdim=True)
+    x = _q64(s.x, 1)
+    y = torch.zeros_like(x)
+    inter = case["inter"]
+    for e in range(case["experts"]):
+        t, k = (idx == e).nonzero(as_tuple=True)
+        h = x[t] @ w1[e].double().t()
+        o = (torch.nn.functional.silu(h[:, :inter]) * h[:, inter:]) @ w2[e].double().t()
+        y.index_add_(0, t, o * weight[t, k][:, None])
+    return y
