@@ -113,7 +113,10 @@ def quantize_blockscaled_pow2(x: torch.Tensor, row_block: int = 1):
     q = torch.empty(rows, K, dtype=torch.float8_e4m3fn, device=x.device)
     s = torch.empty((rows + row_block - 1) // row_block, K // 128, dtype=torch.float32,
                     device=x.device)
-    sf = torch.full(((K // 128 + 3) // 4, rows), 0x7f7f7f7f, dtype=torch.int32, device=x.device)
+    sf_shape = ((K // 128 + 3) // 4, rows)
+    # one scale per row: the kernel writes whole words, missing blocks of a ragged K included
+    sf = torch.empty(sf_shape, dtype=torch.int32, device=x.device) if row_block == 1 else \
+        torch.full(sf_shape, 0x7f7f7f7f, dtype=torch.int32, device=x.device)
     rc = lib.cb_quant_blockscaled_pow2(N.ptr(x), N.ptr(q), N.ptr(s), N.ptr(sf), rows,
                                        C.c_longlong(rows), K, row_block, N.stream_ptr())
     if rc != 0:

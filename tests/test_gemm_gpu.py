@@ -190,3 +190,37 @@ def test_fp8_gemm_with_hardware_block_scales(native_lib, shape, pair):
     assert int(status[0].item()) == 0, hex(int(status[0].item()) & 0xffffffff)
     ref = _bs_reference(aq, as_, bq, bs)
     _check(out, ref, 1e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,k", [(1, 128), (3, 640), (4, 512), (37, 384), (130, 1152)])
+@pytest.mark.parametrize("pow2", [False, True])
+def test_quantize_rows_is_exact(native_lib, rows, k, pow2):
+    """The warp-per-512-columns kernel at ragged row groups and K groups: scales, e4m3 bytes and
+    packed words equal the formula bit for bit (zero and huge blocks among them)."""
+    from commbench_b200.ops.gemm import quantize_blockscaled, quantize_blockscaled_pow2
+
+    g = torch.Generator(device="cuda").manual_seed(rows * 1000 + k)
+    x = (torch.randn(rows, k, device="cuda", generator=g)
+         * torch.logspace(-6, 6, rows, device="cuda")[:, None]).bfloat16()
+    x[0, :128] = 0
+    x[-1, -1] = 3e38
+    f = x.float().view(rows, k // 128, 128)
+    amax = f.abs().amax(dim=-1)
+    s = torch.where(amax > 0, amax / torch.full_like(amax, 448.0), torch.ones_like(amax))
+    if pow2:
+        m, e = torch.frexp(s)
+        s = torch.ldexp(torch.ones_like(s), torch.where(m == 0.5, e - 1, e))
+    # the kernel saturates, torch's cast may not: clamp in fp32 first
+    ref = (f * (1.0 / s)[..., None]).clamp(-448, 448).to(torch.float8_e4m3fn).view(rows, k)
+    if pow2:
+        q, sc, sf = quantize_blockscaled_pow2(x, 1)
+        kg = (k // 128 + 3) // 4
+        byte = torch.full((rows, kg * 4), 127, dtype=torch.uint8, device="cuda")
+        byte[:, :k // 128] = (torch.frexp(s)[1] + 126).to(torch.uint8)
+        words = byte.view(rows, kg, 4).permute(1, 0, 2).contiguous().view(torch.int32).view(kg, rows)
+        assert torch.equal(sf, words)
+    else:
+        q, sc = quantize_blockscaled(x, 1)
+    assert torch.equal(sc, s)
+    assert torch.equal(q.view(torch.uint8), ref.view(torch.uint8))
