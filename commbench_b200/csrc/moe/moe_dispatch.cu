@@ -16,14 +16,26 @@ void set_last_error(const std::string& s);
 
 enum : uint32_t { PH_MOE_ARRIVE2 = 48, PH_MOE_COMBINE2 = 49 };
 
+// Eight e4m3 values times their block's scale, as bf16.
+__device__ __forceinline__ uint4 expand_fp8x8(uint2 raw, float s) {
+  const __nv_fp8x2_storage_t* p8 = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
+  uint4 o;
+  __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p8[i], __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+    ob[i] = __floats2bfloat162_rn(f.x * s, f.y * s);
+  }
+  return o;
+}
+
 struct MoeSendArgs {
   const __nv_bfloat16* x;     // [T, H] this rank's tokens
   const int* topk_idx;        // [T*K]
-  const float* topk_w;        // [T*K]
-  const int* sorted_pair;     // [T*K] pairs in expert-major order
-  const int* src_pair_base;   // [E]
-  const int* my_counts;       // [E] selections of each expert among my tokens
+  const int* slot;            // [T*K] position of a selection among this rank's of the same expert
   const int* send_row_base;   // [E] first destination row
+  __nv_bfloat16* a_out;       // bf16 [max_rows, H] grouped-GEMM input of THIS rank
   uint8_t* recv_x[CB_MAX_RANKS];      // fp8 [max_rows, H] on each rank
   float* recv_scale[CB_MAX_RANKS];    // [max_rows, H/128]
   int2* recv_meta[CB_MAX_RANKS];      // [max_rows] {source rank, source pair index}
@@ -33,9 +45,14 @@ struct MoeSendArgs {
   int per_token;              // 1: one copy of a token per destination RANK (see the kernel)
 };
 
-// grid (E, slices).  Warp per row: load the token's bf16 row, per-128-channel
-// absmax -> scale, quantise to e4m3, write 8 bytes per lane to the destination
-// row; the CTA then releases once and bumps the expert's arrival counter.
+// Token-major dispatch: a warp loads up to 1024 columns of a token ONCE, quantises them ONCE
+// (per-128-channel absmax -> scale -> e4m3) and writes them to every row that the token's K
+// selections have; all slices of a token belong to one CTA, which releases once at the end and then
+// bumps the arrival counter of every expert it wrote rows for.
+//
+// Rows for another rank go there as fp8 plus scales.  Rows for an expert of THIS rank never take
+// the fp8 detour through memory: the quantised values, expanded to bf16 exactly as the receive
+// kernel would, are written straight into the grouped GEMM's input.
 //
 // per_token = 0 (expanded layout): every (token, expert) selection carries its own copy of the
 // token, written at its final row of the destination's per-expert receive buffer.
@@ -47,84 +64,120 @@ struct MoeSendArgs {
 // second count exchange is needed - sent by the first of the token's selections that lives on
 // that rank; every selection still writes its {source rank, pair} word at its final row, and the
 // receive kernel expands from there.
+//
+// Bound by the bytes written.  At 4096 tokens, top-8 of 32 local experts, H = 7168 an expert-major
+// grid (every selection loads and quantises its token again, 128 CTAs) took 417 us and the receive
+// kernel's expansion 253 us; this kernel takes 115 us (528 MB, 4.6 TB/s) and the receive kernel only
+// marks padding.
+static constexpr int kSendCols = 1024;   // columns per warp and step: 4 x 16 bytes per lane
 __global__ void __launch_bounds__(256)
     moe_dispatch_send_kernel(const __grid_constant__ MoeSendArgs a) {
   pdl_wait();                // chained with programmatic dependent launch: see prim/pdl.cuh
   pdl_launch_dependents();
-  const int e = blockIdx.x;
+  extern __shared__ int sent[];    // [E] rows this CTA has written per expert
   const int El = a.E / a.world;
-  const int dst = e / El;
-  const int cnt = a.my_counts[e];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int warps = blockDim.x >> 5;
-  const int nvec = a.H / 8;        // 16-byte vectors per row
   const int groups = a.H / 128;
-  int handled = 0;
-  for (int r = blockIdx.y * warps + warp; r < cnt; r += gridDim.y * warps) {
-    const int pair = a.sorted_pair[a.src_pair_base[e] + r];
-    const int token = pair / a.K;
-    const long long row = static_cast<long long>(a.send_row_base[e]) + r;
-    if (row >= a.max_rows) continue;  // plan kernel already reported the overflow
-    long long drow = row;
-    bool send = true;                 // the same for every lane: `pair` belongs to the warp
-    if (a.per_token) {
-      const int k = pair - token * a.K;
-      const int lo = dst * El, hi = lo + El;
-      for (int kk = 0; kk < k; ++kk) {
-        const int ee = a.topk_idx[token * a.K + kk];
-        if (ee >= lo && ee < hi) send = false;     // an earlier selection already sends the token
-      }
-      drow = static_cast<long long>(a.rank) * a.T + token;
-    }
-    const uint4* __restrict__ src =
-        reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(token) * a.H);
-    uint2* __restrict__ dq = reinterpret_cast<uint2*>(a.recv_x[dst] + drow * a.H);
-    float* __restrict__ ds = a.recv_scale[dst] + drow * groups;
-    // H is a multiple of 256, so every lane makes the same number of trips (the shuffles below
-    // need the whole warp); four rows of loads in flight per lane.
-#pragma unroll 4
-    for (int v = lane; send && v < nvec; v += 32) {
-      const uint4 raw = src[v];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-      float f[8];
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 t = __bfloat1622float2(h[i]);
-        f[2 * i] = t.x;
-        f[2 * i + 1] = t.y;
-        amax = fmaxf(amax, fmaxf(fabsf(t.x), fabsf(t.y)));
-      }
-      // 16 lanes share one 128-channel group
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      const float scale = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
-      const float inv = 1.0f / scale;
-      uint32_t w[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(
-            make_float2(f[4 * i] * inv, f[4 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-        const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(
-            make_float2(f[4 * i + 2] * inv, f[4 * i + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-        w[i] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
-      }
-      dq[v] = make_uint2(w[0], w[1]);
-      if ((lane & 15) == 0) ds[v / 16] = scale;
-    }
-    if (lane == 0) a.recv_meta[dst][row] = make_int2(a.rank, pair);
-    ++handled;
-  }
-  // CTA-wide count of rows written, one release, one counter bump.
-  __shared__ int total;
-  if (threadIdx.x == 0) total = 0;
+  const int slices = (a.H + kSendCols - 1) / kSendCols;
+  for (int e = threadIdx.x; e < a.E; e += blockDim.x) sent[e] = 0;
   __syncthreads();
-  if (lane == 0 && handled > 0) atomicAdd(&total, handled);
-  __syncthreads();
-  if (threadIdx.x == 0 && total > 0) {
-    fence_acq_rel_sys();
-    red_relaxed_sys_add(a.arrived[dst] + (e - dst * El), static_cast<uint32_t>(total));
+  // Tokens of a CTA: so many at a time that their slices fill the 8 warps.
+  const int batch = slices < 8 ? 8 / slices : 1;
+  for (int t0 = blockIdx.x * batch; t0 < a.T; t0 += gridDim.x * batch) {
+    const int n = min(batch, a.T - t0) * slices;
+    for (int unit = warp; unit < n; unit += 8) {
+      const int token = t0 + unit / slices, slice = unit % slices;
+      // H is a multiple of 256: a 256-column group is whole or absent for all lanes.
+      const uint4* __restrict__ src =
+          reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(token) * a.H + slice * kSendCols);
+      const int ng = min(kSendCols, a.H - slice * kSendCols) / 256;
+      uint4 raw[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        raw[g] = g < ng ? __ldg(src + g * 32 + lane) : make_uint4(0, 0, 0, 0);
+      uint2 q[4];
+      float sc[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[g]);
+        __nv_bfloat162 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])),
+                                   __hmax2(__habs2(h[2]), __habs2(h[3])));
+        // 16 lanes share one 128-channel group
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m = __hmax2(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float2 mf = __bfloat1622float2(m);
+        const float amax = fmaxf(fmaxf(0.f, mf.x), mf.y);
+        sc[g] = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
+        const float inv = 1.0f / sc[g];
+        uint32_t w[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 v0 = __bfloat1622float2(h[2 * i]), v1 = __bfloat1622float2(h[2 * i + 1]);
+          const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(
+              make_float2(v0.x * inv, v0.y * inv), __NV_SATFINITE, __NV_E4M3);
+          const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(
+              make_float2(v1.x * inv, v1.y * inv), __NV_SATFINITE, __NV_E4M3);
+          w[i] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+        }
+        q[g] = make_uint2(w[0], w[1]);
+        raw[g] = expand_fp8x8(q[g], sc[g]);   // what a row of this rank gets
+      }
+      unsigned ranks_sent = 0u;   // per_token: other ranks that have the token already
+      for (int k0 = 0; k0 < a.K; k0 += 32) {
+        // lane l holds selection k0 + l: expert, destination row, whether the payload goes there
+        int e = -1, row = 0;
+        if (k0 + lane < a.K) {
+          const int pair = token * a.K + k0 + lane;
+          e = a.topk_idx[pair];
+          if (e >= a.E) e = -1;
+          if (e >= 0) {
+            row = a.send_row_base[e] + a.slot[pair];
+            if (row >= a.max_rows) e = -1;   // the plan kernel already reported the overflow
+          }
+        }
+        const int dst = e >= 0 ? e / El : -1;
+        bool payload = e >= 0;
+        if (a.per_token) {                   // an earlier selection on that rank sends the token
+          const unsigned same = __match_any_sync(0xffffffffu, dst);
+          if (dst >= 0 && dst != a.rank)
+            payload = (same & ((1u << lane) - 1u)) == 0u && ((ranks_sent >> dst) & 1u) == 0u;
+          ranks_sent |= __reduce_or_sync(0xffffffffu, dst >= 0 ? 1u << dst : 0u);
+        }
+        if (slice == 0 && e >= 0) {
+          a.recv_meta[dst][row] = make_int2(a.rank, token * a.K + k0 + lane);
+          atomicAdd(&sent[e], 1);
+        }
+        for (unsigned left = __ballot_sync(0xffffffffu, payload); left != 0u; left &= left - 1u) {
+          const int l = __ffs(left) - 1;
+          const int d = __shfl_sync(0xffffffffu, dst, l);
+          const long long r = __shfl_sync(0xffffffffu, row, l);
+          if (d == a.rank) {
+            uint4* out = reinterpret_cast<uint4*>(a.a_out + r * a.H + slice * kSendCols);
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              if (g < ng) out[g * 32 + lane] = raw[g];
+          } else {
+            const long long dr = a.per_token ? static_cast<long long>(a.rank) * a.T + token : r;
+            uint2* dq = reinterpret_cast<uint2*>(a.recv_x[d] + dr * a.H + slice * kSendCols);
+            float* ds = a.recv_scale[d] + dr * groups + slice * (kSendCols / 128) + (lane >> 4);
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              if (g < ng) {
+                dq[g * 32 + lane] = q[g];
+                if ((lane & 15) == 0) ds[2 * g] = sc[g];
+              }
+          }
+        }
+      }
+    }
   }
+  // One release of everything this CTA wrote, then the counters.
+  __syncthreads();
+  if (threadIdx.x == 0) fence_acq_rel_sys();
+  __syncthreads();
+  for (int e = threadIdx.x; e < a.E; e += blockDim.x)
+    if (sent[e] > 0)
+      red_relaxed_sys_add(a.arrived[e / El] + e % El, static_cast<uint32_t>(sent[e]));
 }
 
 struct MoeRecvArgs {
@@ -142,11 +195,13 @@ struct MoeRecvArgs {
   int per_token;              // 1: rows were sent once per token and rank; expand them here
   int T, K;                   // tokens per rank and selections per token (per_token only)
   int stage_rows;             // rows of recv_x / recv_scale (per_token only: world * T)
+  int rank;                   // rows of this source rank are in a_out already (dispatch kernel)
 };
 
-// grid (El, slices).  Waits until the expert's rows are all in, then
-// dequantises them to bf16; padding rows (up to the next multiple of 128) are
-// zeroed and marked with source rank -1 so later stages skip them.
+// grid (El, slices).  Waits until the expert's rows are all in, then expands the rows that came
+// from other ranks to bf16; this rank's own rows were written by its dispatch kernel.  Padding
+// rows (up to the next multiple of 128) are marked with source rank -1 so later stages skip them;
+// what they hold does not matter, since no row of a product depends on another row of A.
 // With `ctas_done` set, the last CTA of an expert to finish clears that expert's arrival
 // counter, so no separate fill launch is needed between two calls.  This is early enough: a peer
 // cannot send rows of its NEXT call before it has this rank's combine rows of the current one,
@@ -184,40 +239,38 @@ __global__ void __launch_bounds__(256)
   const int warps = blockDim.x >> 5;
   const int nvec = a.H / 8;
   const int groups = a.H / 128;
-  for (int r = blockIdx.y * warps + warp; all_ok && r < padded; r += gridDim.y * warps) {
-    const long long row = static_cast<long long>(base) + r;
-    if (row >= a.max_rows) continue;
-    uint4* __restrict__ out = reinterpret_cast<uint4*>(a.a_out + row * a.H);
-    if (r >= expect) {
-      for (int v = lane; v < nvec; v += 32) out[v] = make_uint4(0, 0, 0, 0);
-      if (lane == 0) a.recv_meta[row] = make_int2(-1, -1);
-      continue;
-    }
-    long long srow = row;
-    if (a.per_token) {
-      const int2 m = __ldcg(a.recv_meta + row);          // {source rank, source pair}
-      srow = static_cast<long long>(m.x) * a.T + m.y / a.K;
-      if (m.x < 0 || m.y < 0 || srow >= a.stage_rows) {   // never written: leave a zero row
-        for (int v = lane; v < nvec; v += 32) out[v] = make_uint4(0, 0, 0, 0);
-        continue;
+  // A warp's rows are `stride` apart; its lanes look at 32 of them at a time and the warp then
+  // expands those that need it.
+  const int stride = gridDim.y * warps;
+  for (int r0 = blockIdx.y * warps + warp; all_ok && r0 < padded; r0 += 32 * stride) {
+    const long long my = r0 + static_cast<long long>(lane) * stride;
+    int2 m = make_int2(-1, -1);
+    bool work = false;
+    if (my < padded && base + my < a.max_rows) {
+      if (my >= expect) {
+        a.recv_meta[base + my] = m;
+      } else {
+        m = __ldcg(a.recv_meta + base + my);             // {source rank, source pair}
+        work = m.x != a.rank;
       }
     }
-    const uint2* __restrict__ q = reinterpret_cast<const uint2*>(a.recv_x + srow * a.H);
-    const float* __restrict__ sc = a.recv_scale + srow * groups;
+    for (unsigned left = __ballot_sync(0xffffffffu, work); left != 0u; left &= left - 1u) {
+      const int l = __ffs(left) - 1;
+      const long long row = base + r0 + static_cast<long long>(l) * stride;
+      uint4* __restrict__ out = reinterpret_cast<uint4*>(a.a_out + row * a.H);
+      long long srow = row;
+      if (a.per_token) {
+        const int src = __shfl_sync(0xffffffffu, m.x, l), pair = __shfl_sync(0xffffffffu, m.y, l);
+        srow = static_cast<long long>(src) * a.T + pair / a.K;
+        if (src < 0 || pair < 0 || srow >= a.stage_rows) {   // never written: leave a zero row
+          for (int v = lane; v < nvec; v += 32) out[v] = make_uint4(0, 0, 0, 0);
+          continue;
+        }
+      }
+      const uint2* __restrict__ q = reinterpret_cast<const uint2*>(a.recv_x + srow * a.H);
+      const float* __restrict__ sc = a.recv_scale + srow * groups;
 #pragma unroll 4
-    for (int v = lane; v < nvec; v += 32) {
-      const uint2 raw = __ldcg(q + v);
-      const float s = __ldcg(sc + v / 16);
-      const __nv_fp8x2_storage_t* p8 = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
-      uint4 o;
-      __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p8[i], __NV_E4M3);
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-        ob[i] = __floats2bfloat162_rn(f.x * s, f.y * s);
-      }
-      out[v] = o;
+      for (int v = lane; v < nvec; v += 32) out[v] = expand_fp8x8(__ldcg(q + v), __ldcg(sc + v / 16));
     }
   }
   if (a.ctas_done != nullptr) {
@@ -341,13 +394,18 @@ extern "C" {
 int cb_sizeof_moe_send_args() { return static_cast<int>(sizeof(MoeSendArgs)); }
 int cb_sizeof_moe_recv_args() { return static_cast<int>(sizeof(MoeRecvArgs)); }
 
-int cb_moe_dispatch_send(const MoeSendArgs* a, int slices, void* stream) {
-  if (a->H % 256 != 0 || a->E % a->world != 0) {
-    set_last_error("dispatch: hidden must be a multiple of 256 and experts divisible by ranks");
+int cb_moe_dispatch_send(const MoeSendArgs* a, int max_ctas, void* stream) {
+  if (a->H % 256 != 0 || a->E % a->world != 0 || a->E > 1024 || a->T < 1 || a->K < 1) {
+    set_last_error("dispatch: hidden must be a multiple of 256, experts (at most 1024) divisible "
+                   "by ranks, at least one token and selection");
     return -1;
   }
-  dim3 grid(a->E, slices < 1 ? 1 : slices);
-  return launch_pdl(moe_dispatch_send_kernel, grid, dim3(256), 0,
+  const int slices = (a->H + kSendCols - 1) / kSendCols;
+  const int batch = slices < 8 ? 8 / slices : 1;
+  int ctas = (a->T + batch - 1) / batch;
+  if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
+  if (ctas < 1) ctas = 1;
+  return launch_pdl(moe_dispatch_send_kernel, dim3(ctas), dim3(256), a->E * sizeof(int),
                     static_cast<cudaStream_t>(stream), *a) == cudaSuccess
              ? 0
              : -1;

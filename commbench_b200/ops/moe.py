@@ -3,7 +3,7 @@ grouped GEMM (SwiGLU) -> grouped GEMM with the combine send fused into its epilo
 weighted combine reduction.
 
 Per call and rank the kernels are (all from ``csrc/moe``):
-  router_topk, moe_slots, [count all-gather], moe_plan, moe_sort_pairs, dispatch_send,
+  router_topk, moe_slots, [count all-gather], moe_plan, dispatch_send,
   recv_dequant, grouped_gemm(up; silu(gate) * up in its epilogue unless ``fused_swiglu`` is off,
   then a separate swiglu kernel), grouped_gemm(down, scatter), combine_reduce.
 No host synchronisation happens between them: the receive side learns the row counts from
@@ -37,9 +37,8 @@ _P8 = C.c_void_p * N.MAX_RANKS
 
 class _SendArgs(C.Structure):
     _fields_ = [
-        ("x", C.c_void_p), ("topk_idx", C.c_void_p), ("topk_w", C.c_void_p),
-        ("sorted_pair", C.c_void_p), ("src_pair_base", C.c_void_p), ("my_counts", C.c_void_p),
-        ("send_row_base", C.c_void_p),
+        ("x", C.c_void_p), ("topk_idx", C.c_void_p), ("slot", C.c_void_p),
+        ("send_row_base", C.c_void_p), ("a_out", C.c_void_p),
         ("recv_x", _P8), ("recv_scale", _P8), ("recv_meta", _P8), ("arrived", _P8),
         ("rank", C.c_int), ("world", C.c_int), ("T", C.c_int), ("K", C.c_int), ("H", C.c_int),
         ("E", C.c_int), ("max_rows", C.c_int), ("status", C.c_void_p), ("per_token", C.c_int),
@@ -53,6 +52,7 @@ class _RecvArgs(C.Structure):
         ("recv_base", C.c_void_p), ("H", C.c_int), ("max_rows", C.c_int),
         ("timeout_ns", C.c_ulonglong), ("status", C.c_void_p), ("ctas_done", C.c_void_p),
         ("per_token", C.c_int), ("T", C.c_int), ("K", C.c_int), ("stage_rows", C.c_int),
+        ("rank", C.c_int),
     ]
 
 
@@ -118,13 +118,11 @@ class _RankState:
         self.slot = torch.empty(L.T * L.K, **i32)
         self.counts = torch.zeros(L.E, **i32)
         self.send_row_base = torch.empty(L.E, **i32)
-        self.src_pair_base = torch.empty(L.E, **i32)
         self.recv_expected = torch.empty(L.El, **i32)
         self.recv_base = torch.empty(L.El + 1, **i32)
         self.mblk_expert = torch.zeros(L.max_rows // 128, **i32)
         self.n_mblocks = torch.zeros(1, **i32)
         self.n_rows = torch.zeros(1, **i32)
-        self.sorted_pair = torch.empty(L.T * L.K, **i32)
         self.a = torch.empty(L.max_rows, L.H, dtype=torch.bfloat16, device=dev)
         self.h1 = None if L.fused_swiglu else \
             torch.empty(L.max_rows, 2 * L.I, dtype=torch.bfloat16, device=dev)
@@ -228,8 +226,7 @@ class MoELayer:
         ``bias0`` / ``bias1``: optional [T, H] bf16 tensors added in the combine reduction (a
         shared expert's output, a residual).  Returns y [T, H] bf16 (list in emulation).
 
-        The small kernels of the layer (slots, plan, pair sort, dispatch, receive, combine
-        reduction) are chained with programmatic dependent launch: each may be scheduled while
+        The small kernels of the layer (slots, plan, dispatch, receive, combine reduction) are chained with programmatic dependent launch: each may be scheduled while
         its predecessor still runs and waits on the device for it."""
         lib, W, E, K, T, H, I = self.lib, self.W, self.E, self.K, self.T, self.H, self.I
         if not self.emu:
@@ -249,21 +246,18 @@ class MoELayer:
         else:
             counts_all = [coll.all_gather(self.ctx, self.states[0].counts.view(1, E)).contiguous()]
         self._mark("slots+count_gather")
-        # 3. plan + sorted pairs (one launch)
-        for st, idx, ca in zip(self.states, topk_idx, counts_all):
-            N.check(lib.cb_moe_plan_sort(N.ptr(ca), W, E, st.r, N.ptr(idx), N.ptr(st.slot), n_pairs,
-                                         N.ptr(st.sorted_pair), N.ptr(st.send_row_base),
-                                         N.ptr(st.src_pair_base), N.ptr(st.recv_expected),
-                                         N.ptr(st.recv_base), N.ptr(st.mblk_expert),
-                                         N.ptr(st.n_mblocks), self.max_rows,
-                                         C.c_void_p(self._status(st)), sp), "cb_moe_plan_sort")
-        self._mark("plan+sort")
+        # 3. plan
+        for st, ca in zip(self.states, counts_all):
+            N.check(lib.cb_moe_plan(N.ptr(ca), W, E, st.r, N.ptr(st.send_row_base),
+                                    N.ptr(st.recv_expected), N.ptr(st.recv_base),
+                                    N.ptr(st.mblk_expert), N.ptr(st.n_mblocks), self.max_rows,
+                                    C.c_void_p(self._status(st)), sp), "cb_moe_plan")
+        self._mark("plan")
         # 4. dispatch push (quantise + send + per-expert arrival counters)
-        for st, x, idx, w in zip(self.states, xs, topk_idx, topk_w):
+        for st, x, idx in zip(self.states, xs, topk_idx):
             a = _SendArgs()
-            a.x, a.topk_idx, a.topk_w = x.data_ptr(), idx.data_ptr(), w.data_ptr()
-            a.sorted_pair, a.src_pair_base = st.sorted_pair.data_ptr(), st.src_pair_base.data_ptr()
-            a.my_counts, a.send_row_base = st.counts.data_ptr(), st.send_row_base.data_ptr()
+            a.x, a.topk_idx, a.slot = x.data_ptr(), idx.data_ptr(), st.slot.data_ptr()
+            a.send_row_base, a.a_out = st.send_row_base.data_ptr(), st.a.data_ptr()
             for r in range(N.MAX_RANKS):
                 ok = r < W
                 a.recv_x[r] = self.recv_x.ptrs[r] if ok else 0
@@ -272,9 +266,10 @@ class MoELayer:
                 a.arrived[r] = self.arrived.ptrs[r] if ok else 0
             a.rank, a.world, a.T, a.K, a.H, a.E, a.max_rows = st.r, W, T, K, H, E, self.max_rows
             a.status, a.per_token = self._status(st), int(self.per_token)
-            N.check(lib.cb_moe_dispatch_send(C.byref(a), 4, sp), "cb_moe_dispatch_send")
+            # four CTAs per SM at most: each releases its rows and bumps the counters once
+            N.check(lib.cb_moe_dispatch_send(C.byref(a), 4 * self.sms, sp), "cb_moe_dispatch_send")
         self._mark("dispatch_send")
-        # 5. receive: wait per expert, dequantise to bf16, mark padding rows
+        # 5. receive: wait per expert, dequantise other ranks' rows to bf16, mark padding rows
         for st in self.states:
             ra = _RecvArgs()
             ra.recv_x = self._local(self.recv_x, st).data_ptr()
@@ -287,6 +282,7 @@ class MoELayer:
             ra.timeout_ns, ra.status = self.ctx.timeout_ns, self._status(st)
             ra.ctas_done = st.recv_ctas.data_ptr()    # the kernel re-arms the arrival counters
             ra.per_token, ra.T, ra.K, ra.stage_rows = int(self.per_token), T, K, self.stage_rows
+            ra.rank = st.r
             # about two CTAs per SM: the kernel streams max_rows * H bytes in and twice that out
             slices = max(4, -(-2 * self.sms // self.El))
             N.check(lib.cb_moe_recv_dequant(C.byref(ra), self.El, slices, sp), "cb_moe_recv_dequant")
@@ -337,7 +333,7 @@ class MoELayer:
 
     @property
     def launches_per_call(self) -> int:
-        # slots, count all-gather, plan+sort, dispatch, receive, two grouped GEMMs, combine
+        # slots, count all-gather, plan, dispatch, receive, two grouped GEMMs, combine
         # reduction; the unfused form adds the row count and the SwiGLU kernel
         return 8 if self.fused_swiglu else 10
 

@@ -100,3 +100,36 @@ def test_expert_sort_is_a_stable_sort(native_lib, n, E):
     assert torch.equal(sp[:order.numel()].long(), order)
     assert bool((sp[order.numel():] == -1).all())
     assert torch.equal(counts.long(), torch.bincount(idx[valid].long(), minlength=E))
+
+
+@pytest.mark.parametrize("dispatch", ["per_pair", "per_token"])
+@pytest.mark.parametrize("T,H,K,world", [(1, 256, 1, 1), (33, 2304, 5, 2), (19, 7168, 8, 1),
+                                         (9, 1024, 40, 2)])
+def test_moe_dispatch_edges(native_lib, T, H, K, world, dispatch):
+    """Dispatch kernel at its edges: one token, hidden sizes of one, several and a ragged number
+    of 1024-column slices, more than 32 selections, masked and repeated experts; rows for the own
+    rank go straight to the GEMM input, the others through the fp8 buffers.  3e-2 of the largest
+    value, as in the layer test above."""
+    from commbench_b200.ops.moe import MoELayer, reference_moe
+    from commbench_b200.runtime.context import EmuContext
+
+    I, E = 256, 8
+    ctx = EmuContext(world)
+    layer = MoELayer(ctx, T, H, I, E, K, capacity_factor=2.0 * world, dispatch=dispatch)
+    w1_all = torch.cat([layer.weights(r)[0] for r in range(world)])
+    w2_all = torch.cat([layer.weights(r)[1] for r in range(world)])
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    xs = [torch.randn(T, H, device="cuda", generator=g).bfloat16() for _ in range(world)]
+    idxs = [torch.randint(0, E, (T, K), device="cuda", generator=g, dtype=torch.int32)
+            for _ in range(world)]
+    ws = [torch.rand(T, K, device="cuda", generator=g) + 0.1 for _ in range(world)]
+    for idx in idxs:
+        idx[::3, K - 1] = -1
+    for _ in range(2):
+        ys = layer.forward(xs, idxs, ws)
+    ctx.check_status()
+    for r in range(world):
+        wr = torch.where(idxs[r] >= 0, ws[r], torch.zeros_like(ws[r]))
+        ref = reference_moe(xs[r], idxs[r], wr, w1_all, w2_all, I)
+        err = (ys[r].float() - ref).abs().max().item()
+        assert err / (ref.abs().max().item() + 1e-6) < 3e-2, (r, err)
