@@ -39,35 +39,35 @@ enum : uint32_t { PH_MOE_ARRIVE = 48, PH_MOE_COMBINE = 49 };
 
 // ------------------------------------------------------------------- router
 // One warp per token: softmax over E logits, top-K by repeated arg-max,
-// weights renormalised to sum to 1.  E <= 1024.
+// weights renormalised to sum to 1.  kPer = logits per lane, E <= 32 * kPer <= 1024: a compile-time
+// count keeps the row in registers (a run-time one put it in local memory).
+template <int kPer>
 __global__ void router_topk_kernel(const float* __restrict__ logits, int T, int E, int K,
                                    int* __restrict__ topk_idx, float* __restrict__ topk_w) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= T) return;
   const float* row = logits + static_cast<size_t>(warp) * E;
-  float v[32];
-  const int per = (E + 31) / 32;
+  float v[kPer];
   float mx = -INFINITY;
-  for (int i = 0; i < per; ++i) {
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
     const int e = i * 32 + lane;
     v[i] = e < E ? row[e] : -INFINITY;
     mx = fmaxf(mx, v[i]);
   }
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float sum = 0.f;
-  for (int i = 0; i < per; ++i) {
-    v[i] = (i * 32 + lane) < E ? __expf(v[i] - mx) : -1.f;
-    if (v[i] > 0.f) sum += v[i];
-  }
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  // the softmax denominator cancels in the renormalisation
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) v[i] = (i * 32 + lane) < E ? __expf(v[i] - mx) : -1.f;
   float picked_sum = 0.f;
   float my_w = 0.f;
   int my_e = -1;
   for (int k = 0; k < K; ++k) {
     float best = -1.f;
     int best_e = 0x7fffffff;
-    for (int i = 0; i < per; ++i) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
       const int e = i * 32 + lane;
       if (v[i] > best) {
         best = v[i];
@@ -82,7 +82,9 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int T, int 
         best_e = oe;
       }
     }
-    if ((best_e & 31) == lane) v[best_e >> 5] = -1.f;  // remove the winner
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      if (best_e == i * 32 + lane) v[i] = -1.f;        // remove the winner
     picked_sum += best;
     if (lane == k) {
       my_w = best;
@@ -93,7 +95,6 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int T, int 
     topk_idx[static_cast<size_t>(warp) * K + lane] = my_e;
     topk_w[static_cast<size_t>(warp) * K + lane] = my_w / picked_sum;
   }
-  (void)sum;  // softmax denominator cancels in the renormalisation
 }
 
 // ------------------------------------------------------------ dispatch layout
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kSlotWarps * 32)
   const int per_warp = ((n_pairs + kSlotWarps - 1) / kSlotWarps + 31) / 32 * 32;
   const int begin = min(warp * per_warp, n_pairs), end = min(begin + per_warp, n_pairs);
   int hits = 0;
-#pragma unroll 4
+#pragma unroll 16
   for (int base = begin; base < end; base += 32) {
     const int i = base + lane;
     hits += (i < end && topk_idx[i] == e) ? 1 : 0;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(kSlotWarps * 32)
     for (int w = 0; w < kSlotWarps; ++w) total += chunk_hits[w];
     counts[e] = total;
   }
+#pragma unroll 16
   for (int base = begin; base < end; base += 32) {
     const int i = base + lane;
     const bool hit = i < end && topk_idx[i] == e;
@@ -237,7 +239,12 @@ int cb_moe_router_topk(const void* logits, int T, int E, int K, void* topk_idx, 
   }
   const int threads = 256;
   const int blocks = (T * 32 + threads - 1) / threads;
-  router_topk_kernel<<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(
+  auto* kernel = E <= 32    ? router_topk_kernel<1>
+                 : E <= 64  ? router_topk_kernel<2>
+                 : E <= 128 ? router_topk_kernel<4>
+                 : E <= 256 ? router_topk_kernel<8>
+                            : router_topk_kernel<32>;
+  kernel<<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const float*>(logits), T, E, K, static_cast<int*>(topk_idx),
       static_cast<float*>(topk_w));
   return cudaGetLastError() == cudaSuccess ? 0 : -1;

@@ -243,6 +243,8 @@ class MoELayer:
         # 2. count matrix on every rank
         if self.emu:
             counts_all = [torch.stack([s.counts for s in self.states]).contiguous()] * W
+        elif W == 1:
+            counts_all = [self.states[0].counts]
         else:
             counts_all = [coll.all_gather(self.ctx, self.states[0].counts.view(1, E)).contiguous()]
         self._mark("slots+count_gather")
@@ -333,9 +335,9 @@ class MoELayer:
 
     @property
     def launches_per_call(self) -> int:
-        # slots, count all-gather, plan, dispatch, receive, two grouped GEMMs, combine
-        # reduction; the unfused form adds the row count and the SwiGLU kernel
-        return 8 if self.fused_swiglu else 10
+        # slots, count all-gather (not on a single real rank), plan, dispatch, receive, two grouped
+        # GEMMs, combine reduction; the unfused form adds the row count and the SwiGLU kernel
+        return (8 if self.fused_swiglu else 10) - int(self.W == 1 and not self.emu)
 
 
 def dispatch_rows(topk_idx: torch.Tensor, num_experts: int, world: int, per_token: bool) -> list[int]:
