@@ -89,6 +89,24 @@ def available() -> bool:
     return _LIB_PATH.exists()
 
 
+# Entry points of the per-call operators take plain integers for pointers: declared argument types
+# spare a ctypes object per argument.
+_P, _I, _F, _L = C.c_void_p, C.c_int, C.c_float, C.c_longlong
+_HOT_ARGTYPES = {
+    "cb_gemm_bf16": [_P, _P, _P, _I, _I, _I, _F, _I, _I, _P, _P],
+    "cb_gemm_fp8": [_P, _P, _P, _I, _I, _I, _F, _I, _I, _P, _P],
+    "cb_gemm_fp8_mx": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P],
+    "cb_gemm_fp8_blockscaled": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _I, _P, _P],
+    "cb_quant_blockscaled": [_P, _P, _P, _L, _I, _I, _P],
+    "cb_quant_blockscaled_pow2": [_P, _P, _P, _P, _I, _L, _I, _I, _P],
+    "cb_attn_fwd": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P],
+    "cb_attn_fwd4": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P],
+    "cb_moe_router_topk": [_P, _I, _I, _I, _P, _P, _P],
+    "cb_moe_slots": [_P, _I, _I, _P, _P, _P],
+    "cb_moe_plan": [_P, _I, _I, _I, _P, _P, _P, _P, _P, _I, _P, _P],
+}
+
+
 def load():
     """Returns the loaded library, building it first only if CB200_AUTOBUILD=1."""
     global _lib
@@ -107,6 +125,8 @@ def load():
     lib.cb_last_error.restype = C.c_char_p
     for name in ("cb_symm_round_size",):
         getattr(lib, name).restype = C.c_longlong
+    for name, args in _HOT_ARGTYPES.items():
+        getattr(lib, name).argtypes = args
     if lib.cb_sizeof_coll_args() != C.sizeof(CollArgs):
         raise NativeError(
             f"CollArgs layout mismatch: C {lib.cb_sizeof_coll_args()} vs ctypes {C.sizeof(CollArgs)}")
@@ -130,8 +150,15 @@ def ptr(t) -> C.c_void_p:
     return C.c_void_p(0 if t is None else t.data_ptr())
 
 
-def stream_ptr(stream=None) -> C.c_void_p:
+def raw_stream(stream=None) -> int:
+    """Handle of ``stream``, or of the current stream of the current device.  The raw query costs
+    0.3 us where building the ``torch.cuda.Stream`` object costs 3.5."""
+    if stream is not None:
+        return stream.cuda_stream
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def stream_ptr(stream=None) -> C.c_void_p:
+    return C.c_void_p(raw_stream(stream))

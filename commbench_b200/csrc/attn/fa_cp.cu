@@ -1,4 +1,5 @@
 // The context-parallel attention kernel (fa_cp.cuh) and its launch helper.
+#include "../gemm/launch.h"
 #include "cp_launch.h"
 #include "fa_cp.cuh"
 
@@ -18,16 +19,12 @@ static int g_cp_poly = 0;
 
 template <int kPoly>
 static int cp_launch_t(const FaCpParams& p, int grid, cudaStream_t st) {
-  static bool attr_set = false;
-  cudaError_t e = cudaSuccess;
-  if (!attr_set) {
-    e = cudaFuncSetAttribute(fa_cp_kernel<kPoly>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             CP_SMEM);
-    if (e != cudaSuccess) {
-      set_last_error(std::string("cudaFuncSetAttribute(fa_cp): ") + cudaGetErrorString(e));
-      return -1;
-    }
-    attr_set = true;
+  static std::atomic<uint64_t> smem_done{0};
+  cudaError_t e =
+      allow_smem(reinterpret_cast<const void*>(fa_cp_kernel<kPoly>), CP_SMEM, smem_done);
+  if (e != cudaSuccess) {
+    set_last_error(std::string("cudaFuncSetAttribute(fa_cp): ") + cudaGetErrorString(e));
+    return -1;
   }
   fa_cp_kernel<kPoly><<<grid, CP_THREADS, CP_SMEM, st>>>(p);
   e = cudaGetLastError();

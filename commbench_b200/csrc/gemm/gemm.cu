@@ -146,9 +146,9 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
     p.raster_group = grp;
   }
   {
-    cudaError_t e = cudaFuncSetAttribute(gemm_plain_kernel<Cfg>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg::SMEM_BYTES);
+    static std::atomic<uint64_t> smem_done{0};
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(gemm_plain_kernel<Cfg>),
+                               Cfg::SMEM_BYTES, smem_done);
     if (e != cudaSuccess) {
       set_last_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
       return -1;

@@ -7,8 +7,24 @@
 // datasets/example051_thunderkitten_ag_gemm_easy/nv/empty_thunderkitten_ag_gemm.cu:271-308).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <atomic>
 
 namespace cb {
+
+// Opt-in to `bytes` of dynamic shared memory, once per kernel and device: `done` is the kernel's own
+// bit mask of devices (the attribute is idempotent, so a race only sets it twice).
+inline cudaError_t allow_smem(const void* kernel, int bytes, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+  if ((done.load(std::memory_order_relaxed) & bit) != 0) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
 
 template <class... KArgs, class... Args>
 inline cudaError_t launch_gemm_kernel(void (*kernel)(KArgs...), int grid, int threads, int smem,

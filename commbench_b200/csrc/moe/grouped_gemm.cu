@@ -19,6 +19,7 @@
 
 #include <string>
 
+#include "../gemm/launch.h"
 #include "../gemm/tmap_host.h"
 #include "../prim/barrier.cuh"
 #include "../symm/driver_api.h"
@@ -117,9 +118,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
 
 template <class Cfg, bool kDown, bool kGatedUp = false>
 static int launch_grouped(const GroupedParams& p, int ctas, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<Cfg, kDown, kGatedUp>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Cfg::SMEM_BYTES);
+  static std::atomic<uint64_t> smem_done{0};
+  cudaError_t e = allow_smem(
+      reinterpret_cast<const void*>(grouped_gemm_kernel<Cfg, kDown, kGatedUp>), Cfg::SMEM_BYTES,
+      smem_done);
   if (e != cudaSuccess) {
     set_last_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     return -1;

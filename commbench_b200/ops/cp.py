@@ -51,16 +51,15 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: 
     if out is None:
         out = torch.empty_like(q)
     if lse is None:
-        lse = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
+        lse = q.new_empty((B, Hq, Sq), dtype=torch.float32)
     sc = scale if scale is not None else 1.0 / math.sqrt(D)
     if impl is None:
         impl = get_config().attn_impl
     fn = {1: lib.cb_attn_fwd, 4: lib.cb_attn_fwd4}.get(impl)
     if fn is None:
         raise CommError(f"unknown attention kernel {impl} (1 or 4)")
-    rc = fn(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(lse), B, Sq, Skv, Hq, Hkv,
-            q_offset, kv_offset, int(causal), C.c_float(sc), C.c_void_p(status_ptr),
-            N.stream_ptr(stream))
+    rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, Sq, Skv, Hq,
+            Hkv, q_offset, kv_offset, int(causal), sc, status_ptr, N.raw_stream(stream))
     if rc != 0:
         raise CommError(f"attention launch failed: {N.last_error()}")
     return out, lse
@@ -210,9 +209,7 @@ class RingAttention(_CpBase):
         d.rank, d.world, d.B, d.s_local, d.hq, d.hkv = r, self.W, self.B, self.Sl, self.Hq, self.Hkv
         d.causal, d.zigzag, d.num_comm, d.scale = int(causal), int(self.zigzag), self.num_comm, scale
         d.q, d.o, d.lse = q.data_ptr(), o.data_ptr(), (lse.data_ptr() if lse is not None else 0)
-        for x in range(N.MAX_RANKS):
-            d.k_slots[x] = self.k_ptrs[x] if x < self.W else 0
-            d.v_slots[x] = self.v_ptrs[x] if x < self.W else 0
+        d.k_slots, d.v_slots = _P8(*self.k_ptrs), _P8(*self.v_ptrs)
         d.flags, d.sched = self.flags[i].data_ptr(), self.sched[i].data_ptr()
         d.copies = self.copies[i].data_ptr()
         d.calls = self.calls
@@ -248,8 +245,7 @@ class RingAttention(_CpBase):
                     tuple(qi.shape) == (self.B, self.Sl, self.Hq, 128)):
                 raise CommError("q must be a contiguous bf16 tensor [B, S_local, Hq, 128]")
             o = (out[i] if self.emu else out) if out is not None else torch.empty_like(qi)
-            lse = torch.empty(self.B, self.Hq, self.Sl, dtype=torch.float32, device=qi.device) \
-                if want_lse else None
+            lse = qi.new_empty((self.B, self.Hq, self.Sl), dtype=torch.float32) if want_lse else None
             self._launch(i, r, qi, o, lse, causal, sc, stream)
             outs.append(o)
             lses.append(lse)

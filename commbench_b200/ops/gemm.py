@@ -9,6 +9,7 @@ empty_thunderkitten_gemm_ar.cu:84-191).
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import torch
 
@@ -24,6 +25,11 @@ def _check(t: torch.Tensor, name: str):
         raise GemmError(f"{name} must be a contiguous, 16-byte aligned 2-D CUDA tensor")
 
 
+@functools.lru_cache(maxsize=None)
+def _sm_count(device: torch.device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, alpha: float = 1.0,
          bn: int = 0, max_ctas: int = 0, status_ptr: int = 0, stream=None) -> torch.Tensor:
     """``out[M,N] = alpha * a[M,K] @ b[N,K].T`` on the tcgen05 kernel (no library GEMM)."""
@@ -35,18 +41,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, alph
     if K != K2:
         raise GemmError(f"inner dimensions differ: {K} vs {K2}")
     if out is None:
-        out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
-    _check(out, "out")
-    if out.dtype != torch.bfloat16 or tuple(out.shape) != (M, Nn):
-        raise GemmError("out must be bf16 [M, N]")
-    if a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16:
+        out = a.new_empty((M, Nn), dtype=torch.bfloat16)
+    else:
+        _check(out, "out")
+        if out.dtype != torch.bfloat16 or tuple(out.shape) != (M, Nn):
+            raise GemmError("out must be bf16 [M, N]")
+    dt = a.dtype
+    if dt == torch.bfloat16 and b.dtype == dt:
         fn = lib.cb_gemm_bf16
-    elif a.dtype == torch.float8_e4m3fn and b.dtype == torch.float8_e4m3fn:
+    elif dt == torch.float8_e4m3fn and b.dtype == dt:
         fn = lib.cb_gemm_fp8
     else:
         raise GemmError(f"unsupported dtypes {a.dtype} x {b.dtype}")
-    rc = fn(N.ptr(a), N.ptr(b), N.ptr(out), M, Nn, K, C.c_float(alpha), bn, max_ctas,
-            C.c_void_p(status_ptr), N.stream_ptr(stream))
+    rc = fn(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, alpha, bn, max_ctas, status_ptr,
+            N.raw_stream(stream))
     if rc != 0:
         raise GemmError(f"gemm launch failed: {N.last_error()}")
     return out
@@ -90,11 +98,10 @@ def quantize_blockscaled(x: torch.Tensor, row_block: int = 1):
     lib = N.load()
     _check(x, "x")
     rows, K = x.shape
-    q = torch.empty(rows, K, dtype=torch.float8_e4m3fn, device=x.device)
-    s = torch.empty((rows + row_block - 1) // row_block, K // 128, dtype=torch.float32,
-                    device=x.device)
-    rc = lib.cb_quant_blockscaled(N.ptr(x), N.ptr(q), N.ptr(s), C.c_longlong(rows), K, row_block,
-                                  N.stream_ptr())
+    q = x.new_empty((rows, K), dtype=torch.float8_e4m3fn)
+    s = x.new_empty(((rows + row_block - 1) // row_block, K // 128), dtype=torch.float32)
+    rc = lib.cb_quant_blockscaled(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, K, row_block,
+                                  N.raw_stream())
     if rc != 0:
         raise GemmError(N.last_error())
     return q, s
@@ -110,15 +117,14 @@ def quantize_blockscaled_pow2(x: torch.Tensor, row_block: int = 1):
     lib = N.load()
     _check(x, "x")
     rows, K = x.shape
-    q = torch.empty(rows, K, dtype=torch.float8_e4m3fn, device=x.device)
-    s = torch.empty((rows + row_block - 1) // row_block, K // 128, dtype=torch.float32,
-                    device=x.device)
+    q = x.new_empty((rows, K), dtype=torch.float8_e4m3fn)
+    s = x.new_empty(((rows + row_block - 1) // row_block, K // 128), dtype=torch.float32)
     sf_shape = ((K // 128 + 3) // 4, rows)
     # one scale per row: the kernel writes whole words, missing blocks of a ragged K included
-    sf = torch.empty(sf_shape, dtype=torch.int32, device=x.device) if row_block == 1 else \
+    sf = x.new_empty(sf_shape, dtype=torch.int32) if row_block == 1 else \
         torch.full(sf_shape, 0x7f7f7f7f, dtype=torch.int32, device=x.device)
-    rc = lib.cb_quant_blockscaled_pow2(N.ptr(x), N.ptr(q), N.ptr(s), N.ptr(sf), rows,
-                                       C.c_longlong(rows), K, row_block, N.stream_ptr())
+    rc = lib.cb_quant_blockscaled_pow2(x.data_ptr(), q.data_ptr(), s.data_ptr(), sf.data_ptr(), rows,
+                                       rows, K, row_block, N.raw_stream())
     if rc != 0:
         raise GemmError(N.last_error())
     return q, s, sf
@@ -150,12 +156,13 @@ def gemm_fp8_mx(a_q, a_sf, b_q, b_sf, out=None, alpha: float = 1.0, pair: bool =
         if not (t.dtype == torch.int32 and t.is_contiguous() and tuple(t.shape) == (kg, rows)):
             raise GemmError(f"{name} must be a contiguous int32 tensor [{kg}, {rows}]")
     if out is None:
-        out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a_q.device)
-    _check(out, "out")
+        out = a_q.new_empty((M, Nn), dtype=torch.bfloat16)
+    else:
+        _check(out, "out")
     # pair: a CTA pair per 256 x 192 tile (default, fastest); otherwise one CTA per 128 x 192
-    rc = lib.cb_gemm_fp8_mx(N.ptr(a_q), N.ptr(a_sf), N.ptr(b_q), N.ptr(b_sf), N.ptr(out), M, Nn, K,
-                            C.c_float(alpha), 0 if pair else -1, C.c_void_p(status_ptr),
-                            N.stream_ptr(stream))
+    rc = lib.cb_gemm_fp8_mx(a_q.data_ptr(), a_sf.data_ptr(), b_q.data_ptr(), b_sf.data_ptr(),
+                            out.data_ptr(), M, Nn, K, alpha, 0 if pair else -1, status_ptr,
+                            N.raw_stream(stream))
     if rc != 0:
         raise GemmError(f"gemm launch failed: {N.last_error()}")
     return out
@@ -194,14 +201,15 @@ def gemm_fp8_blockscaled(a_q, a_s, b_q, b_s, out=None, alpha: float = 1.0, pair:
             and b_s.dtype == torch.float32):
         raise GemmError("scales must be contiguous fp32 tensors")
     if out is None:
-        out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a_q.device)
-    _check(out, "out")
+        out = a_q.new_empty((M, Nn), dtype=torch.bfloat16)
+    else:
+        _check(out, "out")
     if pair is None:
-        nsm = torch.cuda.get_device_properties(a_q.device).multi_processor_count
+        nsm = _sm_count(a_q.device)
         pair = ((M + 255) // 256) * ((Nn + 255) // 256) * 2 >= nsm
-    rc = lib.cb_gemm_fp8_blockscaled(N.ptr(a_q), N.ptr(a_s), N.ptr(b_q), N.ptr(b_s), N.ptr(out), M,
-                                     Nn, K, C.c_float(alpha), int(bool(pair)), max_ctas,
-                                     C.c_void_p(status_ptr), N.stream_ptr(stream))
+    rc = lib.cb_gemm_fp8_blockscaled(a_q.data_ptr(), a_s.data_ptr(), b_q.data_ptr(), b_s.data_ptr(),
+                                     out.data_ptr(), M, Nn, K, alpha, int(bool(pair)), max_ctas,
+                                     status_ptr, N.raw_stream(stream))
     if rc != 0:
         raise GemmError(f"gemm launch failed: {N.last_error()}")
     return out

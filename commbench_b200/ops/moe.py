@@ -73,10 +73,10 @@ def router_topk(logits: torch.Tensor, k: int):
     lib = N.load()
     T, E = logits.shape
     logits = logits.float().contiguous()
-    idx = torch.empty(T, k, dtype=torch.int32, device=logits.device)
-    w = torch.empty(T, k, dtype=torch.float32, device=logits.device)
-    N.check(lib.cb_moe_router_topk(N.ptr(logits), T, E, k, N.ptr(idx), N.ptr(w), N.stream_ptr()),
-            "cb_moe_router_topk")
+    idx = logits.new_empty((T, k), dtype=torch.int32)
+    w = logits.new_empty((T, k))
+    N.check(lib.cb_moe_router_topk(logits.data_ptr(), T, E, k, idx.data_ptr(), w.data_ptr(),
+                                   N.raw_stream()), "cb_moe_router_topk")
     return idx, w
 
 
@@ -260,12 +260,8 @@ class MoELayer:
             a = _SendArgs()
             a.x, a.topk_idx, a.slot = x.data_ptr(), idx.data_ptr(), st.slot.data_ptr()
             a.send_row_base, a.a_out = st.send_row_base.data_ptr(), st.a.data_ptr()
-            for r in range(N.MAX_RANKS):
-                ok = r < W
-                a.recv_x[r] = self.recv_x.ptrs[r] if ok else 0
-                a.recv_scale[r] = self.recv_scale.ptrs[r] if ok else 0
-                a.recv_meta[r] = self.recv_meta.ptrs[r] if ok else 0
-                a.arrived[r] = self.arrived.ptrs[r] if ok else 0
+            a.recv_x, a.recv_scale = _P8(*self.recv_x.ptrs), _P8(*self.recv_scale.ptrs)
+            a.recv_meta, a.arrived = _P8(*self.recv_meta.ptrs), _P8(*self.arrived.ptrs)
             a.rank, a.world, a.T, a.K, a.H, a.E, a.max_rows = st.r, W, T, K, H, E, self.max_rows
             a.status, a.per_token = self._status(st), int(self.per_token)
             # four CTAs per SM at most: each releases its rows and bumps the counters once
@@ -313,9 +309,7 @@ class MoELayer:
             d2.a, d2.b, d2.c = st.s.data_ptr(), st.w2.data_ptr(), 0
             d2.mblk_expert, d2.n_mblocks = st.mblk_expert.data_ptr(), st.n_mblocks.data_ptr()
             d2.recv_meta = self._local(self.recv_meta, st).data_ptr()
-            for r in range(N.MAX_RANKS):
-                d2.combine_peer[r] = self.combine.ptrs[r] if r < W else 0
-                d2.done_peer[r] = self.done.ptrs[r] if r < W else 0
+            d2.combine_peer, d2.done_peer = _P8(*self.combine.ptrs), _P8(*self.done.ptrs)
             d2.done_ctas = st.done_ctas.data_ptr()
             d2.status = self._status(st)
             N.check(lib.cb_moe_grouped_gemm(C.byref(d2), sp), "grouped gemm (down)")
