@@ -101,6 +101,8 @@ _HOT_ARGTYPES = {
     "cb_quant_blockscaled_pow2": [_P, _P, _P, _P, _I, _L, _I, _I, _P],
     "cb_attn_fwd": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P],
     "cb_attn_fwd4": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P],
+    "cb_attn_split_bytes": [_I, _I, _I, _I, _I, _I, _I, _I],
+    "cb_attn_split": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _L, _P, _P],
     "cb_moe_router_topk": [_P, _I, _I, _I, _P, _P, _P],
     "cb_moe_slots": [_P, _I, _I, _P, _P, _P],
     "cb_moe_plan": [_P, _I, _I, _I, _P, _P, _P, _P, _P, _I, _P, _P],
@@ -123,7 +125,7 @@ def load():
                 "(or __graft_entry__.build()) first")
     lib = C.CDLL(str(_LIB_PATH), mode=C.RTLD_GLOBAL)
     lib.cb_last_error.restype = C.c_char_p
-    for name in ("cb_symm_round_size",):
+    for name in ("cb_symm_round_size", "cb_attn_split_bytes"):
         getattr(lib, name).restype = C.c_longlong
     for name, args in _HOT_ARGTYPES.items():
         getattr(lib, name).argtypes = args

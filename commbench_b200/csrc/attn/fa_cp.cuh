@@ -86,6 +86,87 @@ __device__ __forceinline__ float cp_max3(float a, float b, float c) {
   return d;
 }
 
+// One block of the online softmax: the 128 masked scores of this thread's row in `s` become the
+// bf16 probabilities s[0..63]; m_ref (log2 units) and l are the running reference maximum and sum.
+// The accumulator in tensor memory at `tO` is rescaled when the maximum has grown by more than
+// CP_RESCALE_THRESHOLD in any row of the warp (`rescale_o`: it holds something already).
+// kPoly: see fa_cp_kernel.  Warp-collective.
+template <int kPoly>
+__device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t tO, float scale_log2,
+                                                  bool need_mask, bool rescale_o, float& m_ref,
+                                                  float& l) {
+  float mx8[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    mx8[i] = fmaxf(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]));
+#pragma unroll
+  for (int i = 16; i < 128; i += 2)
+    mx8[(i >> 1) & 7] =
+        cp_max3(mx8[(i >> 1) & 7], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+  const float mx_all =
+      cp_max3(fmaxf(cp_max3(mx8[0], mx8[1], mx8[2]), cp_max3(mx8[3], mx8[4], mx8[5])),
+              mx8[6], mx8[7]);
+  const float mx_s = mx_all * scale_log2;
+  const bool grow =
+      mx_s > m_ref + CP_RESCALE_THRESHOLD || (m_ref == -INFINITY && mx_s > -INFINITY);
+  const bool any_grow = __any_sync(0xffffffffu, grow);
+  if (any_grow) {
+    const float m_new = fmaxf(m_ref, mx_s);
+    const float alpha = m_ref == -INFINITY ? 0.f : cp_ex2(m_ref - m_new);
+    m_ref = m_new;
+    l *= alpha;
+    if (rescale_o) {
+      // These scores being complete implies that the previous P V is: O is stable.
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(tO + c * 32u, o);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+        tmem_st_32x32(tO + c * 32u, o);
+      }
+    }
+  }
+  const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+  const uint64_t scale2 = cp_pack(scale_log2, scale_log2), negm2 = cp_pack(-m_use, -m_use);
+  uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
+  // The bf16 pairs go back into s[0..63]: element i is only written after s[2i], s[2i+1]
+  // have been consumed.
+#pragma unroll
+  for (int i = 0; i < 128; i += 2) {
+    const uint64_t y = cp_fma2(cp_pack_u(s[i], s[i + 1]), scale2, negm2);
+    float p0, p1;
+    if (kPoly > 0 && !need_mask && ((i >> 1) % (kPoly > 0 ? kPoly : 1)) == kPoly - 1) {
+      // 2^x on the FMA pipe: nearest-integer split with the 1.5 * 2^23 trick, a cubic on
+      // the fraction in [-0.5, 0.5] (relative error 7.5e-5, below bf16 rounding), the
+      // exponent added as an integer; inputs clamped to -126 so it cannot wrap.  Masked
+      // blocks keep the SFU everywhere: -inf must give an exact zero.
+      const float x0 = fmaxf(__uint_as_float(static_cast<uint32_t>(y)), -126.f);
+      const float x1 = fmaxf(__uint_as_float(static_cast<uint32_t>(y >> 32)), -126.f);
+      const uint64_t xx = cp_pack(x0, x1);
+      const uint64_t rr = cp_add2(xx, cp_pack(12582912.f, 12582912.f));
+      const uint64_t xf = cp_add2(rr, cp_pack(-12582912.f, -12582912.f));
+      const uint64_t fr = cp_fma2(xf, cp_pack(-1.f, -1.f), xx);
+      uint64_t qq = cp_fma2(fr, cp_pack(0.05517116f, 0.05517116f), cp_pack(0.24261014f, 0.24261014f));
+      qq = cp_fma2(qq, fr, cp_pack(0.69326097f, 0.69326097f));
+      qq = cp_fma2(qq, fr, cp_pack(0.99992812f, 0.99992812f));
+      p0 = __uint_as_float(static_cast<uint32_t>(qq) + (static_cast<uint32_t>(rr) << 23));
+      p1 = __uint_as_float(static_cast<uint32_t>(qq >> 32) + (static_cast<uint32_t>(rr >> 32) << 23));
+    } else {
+      p0 = cp_ex2(__uint_as_float(static_cast<uint32_t>(y)));
+      p1 = cp_ex2(__uint_as_float(static_cast<uint32_t>(y >> 32)));
+    }
+    sum4[(i >> 1) & 3] = cp_add2(sum4[(i >> 1) & 3], cp_pack(p0, p1));
+    __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+    s[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
+  }
+  {
+    const uint64_t a = cp_add2(cp_add2(sum4[0], sum4[1]), cp_add2(sum4[2], sum4[3]));
+    l += __uint_as_float(static_cast<uint32_t>(a)) + __uint_as_float(static_cast<uint32_t>(a >> 32));
+  }
+}
+
 // Walks the key blocks that a query tile pair attends to, segment by segment.  Every role of a
 // CTA runs its own copy and sees the same sequence.  Both tiles of the pair visit the same
 // blocks: a block that lies wholly in the future of the first tile (at most one per item, the
@@ -449,76 +530,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           for (int i = 0; i < 128; ++i)
             if (!(i < kv_left && (!p.causal || key0 + i <= q_pos))) s[i] = 0xff800000u;  // -inf
         }
-        float mx8[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          mx8[i] = fmaxf(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]));
-#pragma unroll
-        for (int i = 16; i < 128; i += 2)
-          mx8[(i >> 1) & 7] =
-              cp_max3(mx8[(i >> 1) & 7], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-        const float mx_all =
-            cp_max3(fmaxf(cp_max3(mx8[0], mx8[1], mx8[2]), cp_max3(mx8[3], mx8[4], mx8[5])),
-                    mx8[6], mx8[7]);
-        const float mx_s = mx_all * p.scale_log2;
-        const bool grow =
-            mx_s > m_ref + CP_RESCALE_THRESHOLD || (m_ref == -INFINITY && mx_s > -INFINITY);
-        const bool any_grow = __any_sync(0xffffffffu, grow);
-        if (any_grow) {
-          const float m_new = fmaxf(m_ref, mx_s);
-          const float alpha = m_ref == -INFINITY ? 0.f : cp_ex2(m_ref - m_new);
-          m_ref = m_new;
-          l *= alpha;
-          if (j > 0) {
-            // S_t(j) complete implies P_t(j-1) V_{j-1} complete: O_t is stable.
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-              uint32_t o[32];
-              tmem_ld_32x32(tO + c * 32u, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st_32x32(tO + c * 32u, o);
-            }
-          }
-        }
-        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-        const uint64_t scale2 = cp_pack(p.scale_log2, p.scale_log2), negm2 = cp_pack(-m_use, -m_use);
-        uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
-        // The bf16 pairs go back into s[0..63]: element i is only written after s[2i], s[2i+1]
-        // have been consumed.
-#pragma unroll
-        for (int i = 0; i < 128; i += 2) {
-          const uint64_t y = cp_fma2(cp_pack_u(s[i], s[i + 1]), scale2, negm2);
-          float p0, p1;
-          if (kPoly > 0 && !need_mask && ((i >> 1) % (kPoly > 0 ? kPoly : 1)) == kPoly - 1) {
-            // 2^x on the FMA pipe: nearest-integer split with the 1.5 * 2^23 trick, a cubic on
-            // the fraction in [-0.5, 0.5] (relative error 7.5e-5, below bf16 rounding), the
-            // exponent added as an integer; inputs clamped to -126 so it cannot wrap.  Masked
-            // blocks keep the SFU everywhere: -inf must give an exact zero.
-            const float x0 = fmaxf(__uint_as_float(static_cast<uint32_t>(y)), -126.f);
-            const float x1 = fmaxf(__uint_as_float(static_cast<uint32_t>(y >> 32)), -126.f);
-            const uint64_t xx = cp_pack(x0, x1);
-            const uint64_t rr = cp_add2(xx, cp_pack(12582912.f, 12582912.f));
-            const uint64_t xf = cp_add2(rr, cp_pack(-12582912.f, -12582912.f));
-            const uint64_t fr = cp_fma2(xf, cp_pack(-1.f, -1.f), xx);
-            uint64_t qq = cp_fma2(fr, cp_pack(0.05517116f, 0.05517116f), cp_pack(0.24261014f, 0.24261014f));
-            qq = cp_fma2(qq, fr, cp_pack(0.69326097f, 0.69326097f));
-            qq = cp_fma2(qq, fr, cp_pack(0.99992812f, 0.99992812f));
-            p0 = __uint_as_float(static_cast<uint32_t>(qq) + (static_cast<uint32_t>(rr) << 23));
-            p1 = __uint_as_float(static_cast<uint32_t>(qq >> 32) + (static_cast<uint32_t>(rr >> 32) << 23));
-          } else {
-            p0 = cp_ex2(__uint_as_float(static_cast<uint32_t>(y)));
-            p1 = cp_ex2(__uint_as_float(static_cast<uint32_t>(y >> 32)));
-          }
-          sum4[(i >> 1) & 3] = cp_add2(sum4[(i >> 1) & 3], cp_pack(p0, p1));
-          __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-          s[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
-        }
-        {
-          const uint64_t a = cp_add2(cp_add2(sum4[0], sum4[1]), cp_add2(sum4[2], sum4[3]));
-          l += __uint_as_float(static_cast<uint32_t>(a)) + __uint_as_float(static_cast<uint32_t>(a >> 32));
-        }
+        cp_online_softmax<kPoly>(s, tO, p.scale_log2, need_mask, j > 0, m_ref, l);
         // P_t(j): row r = lane r, keys 2c and 2c+1 in column c.
         tmem_st_32x32_at(tS, &s[0]);
         tmem_st_32x32_at(tS + 32u, &s[32]);

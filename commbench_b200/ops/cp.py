@@ -27,6 +27,29 @@ from ..utils.tracing import traced
 from . import collectives as coll
 
 
+def _split_attention(q, k, v, out, lse, causal, q_offset, kv_offset, sc, status_ptr, stream) -> bool:
+    """Runs the split-key kernel if the call is one for it - few query tiles: the keys are split
+    over the chip and the partial results merged - and says whether it did.  ``lse`` may be None."""
+    lib = N.load()
+    B, Sq, Hq, _ = q.shape
+    _, Skv, Hkv, _ = k.shape
+    nbytes = lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, q_offset, kv_offset, int(causal))
+    if nbytes < 0:
+        return False
+    ws = 0
+    if nbytes > 0:
+        buf = q.new_empty((nbytes,), dtype=torch.uint8)
+        if stream is not None:
+            buf.record_stream(stream)
+        ws = buf.data_ptr()
+    rc = lib.cb_attn_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                           lse.data_ptr() if lse is not None else 0, B, Sq, Skv, Hq, Hkv, q_offset,
+                           kv_offset, int(causal), sc, ws, nbytes, status_ptr, N.raw_stream(stream))
+    if rc != 0:
+        raise CommError(f"attention launch failed: {N.last_error()}")
+    return True
+
+
 @traced("cb200.flash_attention")
 def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: int = 0,
                     scale: float | None = None, out=None, lse=None, status_ptr: int = 0,
@@ -34,7 +57,8 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: 
     """One key/value chunk: returns (o [B,Sq,Hq,D] bf16 normalised, lse [B,Hq,Sq] fp32).
 
     ``impl`` selects the kernel (default from ``CB200_ATTN_IMPL``): 4 = two query tiles per
-    CTA with a softmax warp-group each, O and P in tensor memory (the product kernel);
+    CTA with a softmax warp-group each, O and P in tensor memory (the product kernel), or its
+    split-key form where the query tiles are too few to fill the chip;
     1 = the first design (one tile, O in registers), kept as a simple cross-check.
 
     ``q_offset`` / ``kv_offset`` are the global sequence positions of the first query / key;
@@ -58,6 +82,9 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: 
     fn = {1: lib.cb_attn_fwd, 4: lib.cb_attn_fwd4}.get(impl)
     if fn is None:
         raise CommError(f"unknown attention kernel {impl} (1 or 4)")
+    if impl == 4 and _split_attention(q, k, v, out, lse, causal, q_offset, kv_offset, sc, status_ptr,
+                                      stream):
+        return out, lse
     rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, Sq, Skv, Hq,
             Hkv, q_offset, kv_offset, int(causal), sc, status_ptr, N.raw_stream(stream))
     if rc != 0:
@@ -190,6 +217,9 @@ class RingAttention(_CpBase):
         self.v_t, self.v_ptrs = self._sym(nbytes)
         self.k_buf = [t[:nbytes].view(torch.bfloat16).view(shape) for t in self.k_t]
         self.v_buf = [t[:nbytes].view(torch.bfloat16).view(shape) for t in self.v_t]
+        own = list(self._ranks())
+        self._k_own = [t[:, r] for t, r in zip(self.k_buf, own)]
+        self._v_own = [t[:, r] for t, r in zip(self.v_buf, own)]
         self._local_state(self.lib.cb_ring_attn_copy_bytes())
         torch.cuda.synchronize(ctx.device)
         if not self.emu:
@@ -197,12 +227,10 @@ class RingAttention(_CpBase):
 
     def k_local(self, i: int = 0) -> torch.Tensor:
         """This rank's own key slot, ``[B, S_local, Hkv, 128]`` (a view of symmetric memory)."""
-        r = i if self.emu else self.ctx.rank
-        return self.k_buf[i][:, r]
+        return self._k_own[i]
 
     def v_local(self, i: int = 0) -> torch.Tensor:
-        r = i if self.emu else self.ctx.rank
-        return self.v_buf[i][:, r]
+        return self._v_own[i]
 
     def _launch(self, i, r, q, o, lse, causal, scale, stream):
         d = _RingDesc()
@@ -227,10 +255,11 @@ class RingAttention(_CpBase):
         sc = scale if scale is not None else 1.0 / math.sqrt(128)
         outs, lses = [], []
         for i, _ in enumerate(self._ranks()):
-            if ks[i].data_ptr() != self.k_local(i).data_ptr():
-                self.k_local(i).copy_(ks[i])
-            if vs[i].data_ptr() != self.v_local(i).data_ptr():
-                self.v_local(i).copy_(vs[i])
+            k_own, v_own = self._k_own[i], self._v_own[i]
+            if ks[i].data_ptr() != k_own.data_ptr():
+                k_own.copy_(ks[i])
+            if vs[i].data_ptr() != v_own.data_ptr():
+                v_own.copy_(vs[i])
         # A plan change (causal <-> full) rewrites the piece list and renumbers the counters:
         # nothing of the old plan may still run, and the counters start again from zero.
         if self._plan_key != (bool(causal),):
@@ -246,7 +275,10 @@ class RingAttention(_CpBase):
                 raise CommError("q must be a contiguous bf16 tensor [B, S_local, Hq, 128]")
             o = (out[i] if self.emu else out) if out is not None else torch.empty_like(qi)
             lse = qi.new_empty((self.B, self.Hq, self.Sl), dtype=torch.float32) if want_lse else None
-            self._launch(i, r, qi, o, lse, causal, sc, stream)
+            # one rank: a plain local attention over its own slot
+            if self.W > 1 or not _split_attention(qi, self._k_own[i], self._v_own[i], o, lse,
+                                                  causal, 0, 0, sc, self._status_ptr(i), stream):
+                self._launch(i, r, qi, o, lse, causal, sc, stream)
             outs.append(o)
             lses.append(lse)
         self._barrier()                       # nobody overwrites a shard that is still being read

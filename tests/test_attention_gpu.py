@@ -137,3 +137,63 @@ def test_ulysses_attention_kernel_virtual_ranks(native_lib, world, causal):
         ctx.check_status()
         for r in range(world):
             assert torch.allclose(outs[r].float(), sh(ro, r), atol=2e-2, rtol=2e-2), (it, r)
+
+
+# (B, Sq, Skv, Hq, Hkv, q_offset, kv_offset): one block and one key; a group of one, three (no
+# divisor of 128) and 64; ragged keys; more items than CTAs; items cut over many CTAs; a query tile
+# that sees no key; several query tiles with a causal diagonal.
+SPLIT_SHAPES = [(1, 1, 1, 1, 1, 0, 0), (1, 1, 129, 4, 1, 128, 0), (3, 2, 1000, 6, 2, 998, 0),
+                (2, 1, 640, 128, 2, 639, 0), (40, 1, 300, 8, 8, 299, 0), (1, 1, 16384, 8, 1, 16383, 0),
+                (2, 4, 5000, 32, 8, 4996, 0), (1, 100, 260, 8, 2, 0, 70), (1, 300, 1077, 4, 1, 777, 0)]
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("shape", SPLIT_SHAPES)
+def test_split_key_attention_matches_reference(native_lib, shape, causal):
+    """Split-key kernel and merge against fp32.  o: rounding of the bf16 result (2^-9 of values of
+    order one) plus bf16 probabilities, 1e-2 of the largest value; lse is fp32 throughout, 1e-4."""
+    import ctypes as C
+    import math
+
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.cp import reference_attention
+
+    B, Sq, Skv, Hq, Hkv, qo, ko = shape
+    q, k, v = _qkv(B, Sq, Skv, Hq, Hkv, 31 + Skv)
+    lib = N.load()
+    nbytes = 64 << 20
+    ws = torch.full((nbytes,), 0xff, dtype=torch.uint8, device="cuda")     # NaN everywhere
+    o, lse = torch.empty_like(q), torch.empty(B, Hq, Sq, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    rc = lib.cb_attn_split(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(o), N.ptr(lse), B, Sq, Skv, Hq, Hkv,
+                           qo, ko, int(causal), C.c_float(1.0 / math.sqrt(128)), N.ptr(ws),
+                           C.c_longlong(nbytes), N.ptr(status), N.stream_ptr())
+    assert rc == 0, N.last_error()
+    ro, rl = reference_attention(q, k, v, causal=causal, q_offset=qo, kv_offset=ko)
+    assert int(status.abs().sum()) == 0
+    assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
+    seen = rl > float("-inf")
+    assert torch.equal(lse > float("-inf"), seen)
+    assert (lse - rl)[seen].abs().max() < 1e-4
+
+
+def test_split_and_pair_kernels_agree_on_the_public_call(native_lib):
+    """The size rule sends decode to the split kernel and a full prefill to the tile-pair kernel;
+    a workspace that is too small is refused."""
+    import ctypes as C
+
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.cp import flash_attention, reference_attention
+
+    lib = N.load()
+    assert lib.cb_attn_split_bytes(4, 1, 3000, 16, 4, 2999, 0, 1) > 0
+    assert lib.cb_attn_split_bytes(1, 16384, 16384, 32, 8, 0, 0, 1) == -1
+    q, k, v = _qkv(4, 1, 3000, 16, 4, 3)
+    o, lse = flash_attention(q, k, v, causal=True, q_offset=2999)
+    ro, rl = reference_attention(q, k, v, causal=True, q_offset=2999)
+    assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
+    assert (lse - rl).abs().max() < 1e-4
+    rc = lib.cb_attn_split(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(o), N.ptr(lse), 4, 1, 3000, 16, 4, 2999,
+                           0, 1, C.c_float(0.1), N.ptr(o), C.c_longlong(16), C.c_void_p(0),
+                           N.stream_ptr())
+    assert rc != 0 and "workspace" in N.last_error()
