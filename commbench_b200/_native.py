@@ -95,6 +95,7 @@ _P, _I, _F, _L = C.c_void_p, C.c_int, C.c_float, C.c_longlong
 _HOT_ARGTYPES = {
     "cb_gemm_bf16": [_P, _P, _P, _I, _I, _I, _F, _I, _I, _P, _P],
     "cb_gemm_fp8": [_P, _P, _P, _I, _I, _I, _F, _I, _I, _P, _P],
+    "cb_gemm_small": [_P, _P, _P, _I, _I, _I, _F, _I, _I, _I, _P, _P],
     "cb_gemm_fp8_mx": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P],
     "cb_gemm_fp8_blockscaled": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _I, _P, _P],
     "cb_quant_blockscaled": [_P, _P, _P, _L, _I, _I, _P],

@@ -6,6 +6,9 @@
 // `matmul::kernel` (datasets/example053_thunderkitten_gemm_ar_easy/nv/
 // empty_thunderkitten_gemm_ar.cu:84-191).
 #include "gemm_sm100.cuh"
+#include "gemm_small.cuh"
+
+#include <math.h>
 
 #include <string>
 
@@ -169,6 +172,134 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
   return 0;
 }
 
+// Which kernel and tile a GEMM runs on, by a model of its time in microseconds.  kbytes: bytes of one
+// K row (K x element size).  Per-128-byte-K-block times of a CTA that nothing else holds up, measured on
+// one m-block: persistent pairs on 256 x 256 tiles 0.30, the small kernel's 64 / 128 / 256-wide
+// tiles 0.16 / 0.22 / 0.34; all CTAs together draw at most 17 bytes a nanosecond x 1000 out of L2 (11
+// where rows do not start on 128-byte lines: every box row then touches two) and weights arrive
+// at 6 from memory.  GEMM_RULE_FIGURES
+struct GemmChoice {
+  int bn;      // persistent: 64 ... 512 as in cb_gemm_bf16; small kernel: its tile width
+  int split;   // 0: persistent kernel; else the small kernel's K splits
+};
+static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
+  const float nkb = static_cast<float>((kbytes + 127) / 128);
+  const float l2_rate = kbytes % 128 == 0 ? 17e6f : 11e6f;   // bytes per us
+  const float hbm_us = static_cast<float>(N) * static_cast<float>(kbytes) / 6e6f;
+  const long long m128 = (M + 127) / 128, m256 = (M + 255) / 256;
+  GemmChoice best = {512, 0};
+  float best_us = 1e30f;
+  const auto offer = [&](int bn, int split, float us) {
+    if (us < best_us) {
+      best_us = us;
+      best = {bn, split};
+    }
+  };
+  {  // persistent kernels: pairs on 256 x 256, single CTAs on 128 x 256
+    const long long pairs = m256 * ((N + 255) / 256), singles = m128 * ((N + 255) / 256);
+    const long long pw = (pairs + sms / 2 - 1) / (sms / 2), sw = (singles + sms - 1) / sms;
+    const float pair_ctas = 2.f * static_cast<float>(pairs < sms / 2 ? pairs : sms / 2);
+    const float single_ctas = static_cast<float>(singles < sms ? singles : sms);
+    const float pair_kb = fmaxf(0.30f, pair_ctas * 32768.f / l2_rate);
+    const float single_kb = fmaxf(0.36f, single_ctas * 49152.f / l2_rate);
+    offer(512, 0, 7.f + fmaxf(static_cast<float>(pw) * fmaxf(nkb * pair_kb, 2.5f), hbm_us));
+    offer(256, 0, 6.5f + fmaxf(static_cast<float>(sw) * fmaxf(nkb * single_kb, 2.5f), hbm_us));
+  }
+  const int a_rows = M < 128 ? (M + 7) / 8 * 8 : 128;
+  const int widths[3] = {64, 128, 256};
+  const bool lines = kbytes % 128 == 0;
+  const float kb_us[3] = {lines ? 0.16f : 0.18f, lines ? 0.22f : 0.30f, lines ? 0.34f : 0.50f};
+  for (int i = 0; i < 3; ++i)
+    for (int split = 1; split <= 8; split *= 2) {
+      if (static_cast<float>(split) > nkb) break;
+      const long long ctas = m128 * ((N + widths[i] - 1) / widths[i]) * split;
+      // one wave only; clusters do not pack a GPC's SMs completely
+      if (ctas > (split <= 2 ? sms : split == 4 ? sms * 9 / 10 : sms * 4 / 5)) break;
+      const float per_kb = fmaxf(kb_us[i], static_cast<float>(ctas) *
+                                               static_cast<float>(a_rows + widths[i]) * 128.f / l2_rate);
+      const float tile_kb = static_cast<float>(a_rows * widths[i]) * 4.f / 1024.f;
+      const float reduce = split == 1 ? 0.5f + tile_kb * 0.025f
+                                      : (split == 8 ? 3.7f : 1.7f) + tile_kb * 0.05f *
+                                            static_cast<float>(split - 1) / static_cast<float>(split);
+      const float steps = static_cast<float>((static_cast<int>(nkb) + split - 1) / split);
+      offer(widths[i], split, 2.7f + fmaxf(steps * per_kb, hbm_us) + reduce);
+    }
+  return best;
+}
+
+// Tile of the persistent kernels for a caller that limits the CTAs: pairs on 256 x 256 tiles when
+// there are plenty of them, narrower tiles for skinny problems.
+static int persistent_tile(int M, int N) {
+  const long long m_blocks = (M + 127) / 128;
+  if (static_cast<long long>((M + 255) / 256) * ((N + 255) / 256) * 2 >= sm_count()) return 512;
+  if (m_blocks * ((N + 255) / 256) >= sm_count()) return 256;
+  if (m_blocks * ((N + 127) / 128) >= sm_count()) return 128;
+  return 64;
+}
+
+template <int BN, bool FP8, int SPLIT>
+static int launch_small(const SmallParams& p, int tiles, cudaStream_t st) {
+  using Cfg = SmallCfg<BN, FP8>;
+  static std::atomic<uint64_t> smem_done{0};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(gemm_small_kernel<Cfg, SPLIT>),
+                             Cfg::SMEM_BYTES, smem_done);
+  if (e == cudaSuccess)
+    e = launch_gemm_kernel_pdl(gemm_small_kernel<Cfg, SPLIT>, tiles * SPLIT, Cfg::THREADS,
+                               Cfg::SMEM_BYTES, st, SPLIT, false, true, p);
+  if (e != cudaSuccess) {
+    set_last_error(std::string("gemm launch: ") + cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+template <int BN, bool FP8>
+static int run_small(const void* a, const void* b, void* c, int M, int N, int K, float alpha,
+                     int split, uint32_t* status, cudaStream_t st) {
+  using Cfg = SmallCfg<BN, FP8>;
+  SmallParams p;
+  const TmapDtype dt = FP8 ? TMAP_U8 : TMAP_BF16;
+  const unsigned long long pitch = static_cast<unsigned long long>(K) * (FP8 ? 1 : 2);
+  p.a_rows = M < Cfg::BM ? (M + 7) / 8 * 8 : Cfg::BM;
+  if (make_tmap_2d(&p.tm_a, a, dt, K, M, pitch, Cfg::BK, static_cast<unsigned>(p.a_rows), true))
+    return -1;
+  if (make_tmap_2d(&p.tm_b, b, dt, K, N, pitch, Cfg::BK, Cfg::BN, true)) return -1;
+  if ((reinterpret_cast<uintptr_t>(c) & 15u) != 0) {
+    set_last_error("gemm: C is not 16-byte aligned");
+    return -1;
+  }
+  p.c = static_cast<__nv_bfloat16*>(c);
+  p.M = M;
+  p.N = N;
+  p.num_m = (M + Cfg::BM - 1) / Cfg::BM;
+  p.num_kb = (K + Cfg::BK - 1) / Cfg::BK;
+  p.alpha = alpha;
+  p.status = status;
+  const int tiles = p.num_m * ((N + BN - 1) / BN);
+  if (split > p.num_kb) {
+    set_last_error("gemm: more K splits than K blocks");
+    return -1;
+  }
+  switch (split) {
+    case 1: return launch_small<BN, FP8, 1>(p, tiles, st);
+    case 2: return launch_small<BN, FP8, 2>(p, tiles, st);
+    case 4: return launch_small<BN, FP8, 4>(p, tiles, st);
+    case 8: return launch_small<BN, FP8, 8>(p, tiles, st);
+    default: set_last_error("gemm: K split must be 1, 2, 4 or 8"); return -1;
+  }
+}
+
+template <bool FP8>
+static int run_small_bn(const void* a, const void* b, void* c, int M, int N, int K, float alpha,
+                        int bn, int split, uint32_t* status, cudaStream_t st) {
+  switch (bn) {
+    case 64: return run_small<64, FP8>(a, b, c, M, N, K, alpha, split, status, st);
+    case 128: return run_small<128, FP8>(a, b, c, M, N, K, alpha, split, status, st);
+    case 256: return run_small<256, FP8>(a, b, c, M, N, K, alpha, split, status, st);
+    default: set_last_error("gemm: small tiles are 64, 128 or 256 wide"); return -1;
+  }
+}
+
 }  // namespace cb
 
 using namespace cb;
@@ -188,13 +319,10 @@ int cb_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, flo
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint32_t* s = static_cast<uint32_t*>(status);
   if (bn == 0) {
-    // Fill the machine: pairs on 256 x 256 tiles when there are plenty of them, narrower
-    // tiles for skinny problems.
-    const long long m_blocks = (M + 127) / 128;
-    if (((M + 255) / 256) * ((N + 255) / 256) * 2 >= sm_count()) bn = 512;
-    else if (m_blocks * ((N + 255) / 256) >= sm_count()) bn = 256;
-    else if (m_blocks * ((N + 127) / 128) >= sm_count()) bn = 128;
-    else bn = 64;
+    const GemmChoice g = choose_gemm(M, N, 2ll * K, sm_count());
+    if (g.split > 0 && max_ctas <= 0)
+      return run_small_bn<false>(a, b, c, M, N, K, alpha, g.bn, g.split, s, st);
+    bn = g.split > 0 ? persistent_tile(M, N) : g.bn;
   }
   switch (bn) {
     case 512:
@@ -211,6 +339,25 @@ int cb_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, flo
       set_last_error("cb_gemm_bf16: bn must be 0, 64, 128, 256, 384 or 512");
       return -1;
   }
+}
+
+// What bn = 0 picks: tile width + 1000 x K splits (0 splits: a persistent kernel).
+int cb_gemm_choice(int M, int N, int K, int fp8) {
+  const GemmChoice g = choose_gemm(M, N, static_cast<long long>(K) * (fp8 ? 1 : 2), sm_count());
+  return g.bn + 1000 * g.split;
+}
+
+// The split-K kernel with a given tile width (64, 128, 256) and number of K splits (1, 2, 4, 8).
+int cb_gemm_small(const void* a, const void* b, void* c, int M, int N, int K, float alpha, int fp8,
+                  int bn, int split, void* status, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || (K % (fp8 ? 16 : 8)) != 0 || (N % 8) != 0) {
+    set_last_error("cb_gemm_small: need M,N,K > 0, K % 8 == 0 (fp8: 16), N % 8 == 0");
+    return -1;
+  }
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  uint32_t* s = static_cast<uint32_t*>(status);
+  return fp8 ? run_small_bn<true>(a, b, c, M, N, K, alpha, bn, split, s, st)
+             : run_small_bn<false>(a, b, c, M, N, K, alpha, bn, split, s, st);
 }
 
 // cb_gemm_bf16 with the role trace switched on: `trace` = 8 x (number of SMs) 64-bit words
@@ -241,11 +388,10 @@ int cb_gemm_fp8(const void* a, const void* b, void* c, int M, int N, int K, floa
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint32_t* s = static_cast<uint32_t*>(status);
   if (bn == 0) {
-    const long long m_blocks = (M + 127) / 128;
-    if (((M + 255) / 256) * ((N + 255) / 256) * 2 >= sm_count()) bn = 512;
-    else if (m_blocks * ((N + 255) / 256) >= sm_count()) bn = 256;
-    else if (m_blocks * ((N + 127) / 128) >= sm_count()) bn = 128;
-    else bn = 64;
+    const GemmChoice g = choose_gemm(M, N, K, sm_count());
+    if (g.split > 0 && max_ctas <= 0)
+      return run_small_bn<true>(a, b, c, M, N, K, alpha, g.bn, g.split, s, st);
+    bn = g.split > 0 ? persistent_tile(M, N) : g.bn;
   }
   switch (bn) {
     case 512:

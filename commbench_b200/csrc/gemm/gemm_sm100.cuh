@@ -140,6 +140,8 @@ __device__ __forceinline__ bool mbar_wait_traced(uint64_t* bar, uint32_t parity,
                                                  long long* acc_cycles) {
   bool ok;
   if (!tracing) {
+    // Usual case: every lane sees the phase complete at its first try.
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) != 0) return true;
     ok = mbar_wait(bar, parity, abort_flag, status, detail);
   } else {
     // The whole call is timed: a try_wait may itself block for a while before it answers.

@@ -27,15 +27,15 @@ inline cudaError_t allow_smem(const void* kernel, int bytes, std::atomic<uint64_
 }
 
 template <class... KArgs, class... Args>
-inline cudaError_t launch_gemm_kernel(void (*kernel)(KArgs...), int grid, int threads, int smem,
-                                      cudaStream_t st, int cluster, bool cooperative,
-                                      Args... args) {
+inline cudaError_t launch_gemm_kernel_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem,
+                                          cudaStream_t st, int cluster, bool cooperative, bool pdl,
+                                          Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(static_cast<unsigned>(threads));
   cfg.dynamicSmemBytes = static_cast<size_t>(smem);
   cfg.stream = st;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   unsigned n = 0;
   if (cluster > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
@@ -49,9 +49,22 @@ inline cudaError_t launch_gemm_kernel(void (*kernel)(KArgs...), int grid, int th
     attr[n].val.cooperative = 1;
     ++n;
   }
+  if (pdl) {  // the kernel must call pdl_wait()
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   cfg.attrs = attr;
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <class... KArgs, class... Args>
+inline cudaError_t launch_gemm_kernel(void (*kernel)(KArgs...), int grid, int threads, int smem,
+                                      cudaStream_t st, int cluster, bool cooperative,
+                                      Args... args) {
+  return launch_gemm_kernel_pdl(kernel, grid, threads, smem, st, cluster, cooperative, false,
+                                args...);
 }
 
 }  // namespace cb

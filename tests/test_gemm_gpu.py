@@ -224,3 +224,59 @@ def test_quantize_rows_is_exact(native_lib, rows, k, pow2):
         q, sc = quantize_blockscaled(x, 1)
     assert torch.equal(sc, s)
     assert torch.equal(q.view(torch.uint8), ref.view(torch.uint8))
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("shape", [(1, 8, 1024), (7, 72, 1040), (128, 264, 1536), (129, 520, 1040),
+                                   (300, 136, 2064)])
+def test_small_gemm_splits(native_lib, shape, bn, split, fp8):
+    """Split-K kernel at the edges of its tiles: one row, ragged row groups, columns short of a
+    tile, a last K block of 16 elements, K blocks that do not divide by the splits or the ring
+    stage.  Against fp32: the bf16 result is off by at most half a unit (2^-9 of the value), the
+    fp32 sums by far less, so 2-norm 3e-3 and 1e-2 of the largest value.  Two runs give the same
+    bits; rows of C beyond M stay untouched."""
+    from commbench_b200 import _native as N
+
+    M, Nn, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + Nn + K)
+    a = torch.randn(M, K, device="cuda", generator=g).mul_(0.5).bfloat16()
+    b = torch.randn(Nn, K, device="cuda", generator=g).mul_(0.5).bfloat16()
+    if fp8:
+        a, b = a.to(torch.float8_e4m3fn), b.to(torch.float8_e4m3fn)
+    lib = N.load()
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    outs = []
+    for _ in range(2):
+        c = torch.full((M + 3, Nn), 7.0, device="cuda", dtype=torch.bfloat16)
+        rc = lib.cb_gemm_small(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, Nn, K, 0.5, int(fp8), bn,
+                               split, status.data_ptr(), N.raw_stream())
+        assert rc == 0, N.last_error()
+        outs.append(c)
+    ref = _ref(a, b, 0.5)
+    assert int(status.abs().sum()) == 0
+    assert torch.equal(outs[0], outs[1])
+    assert bool((outs[0][M:] == 7.0).all())
+    err = outs[0][:M].float() - ref
+    assert err.norm() <= 3e-3 * ref.norm()
+    assert err.abs().max() <= 1e-2 * ref.abs().max()
+
+
+def test_gemm_choice_covers_the_range(native_lib):
+    """The size rule: split K where tiles are few, the pair kernel where they are many; whatever it
+    picks is right (bf16 rounding, 2-norm 3e-3)."""
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.gemm import gemm
+
+    lib = N.load()
+    assert lib.cb_gemm_choice(48, 3584, 8192, 0) >= 2000          # split
+    assert lib.cb_gemm_choice(8192, 8192, 8192, 0) == 512         # persistent pairs
+    g = torch.Generator(device="cuda").manual_seed(9)
+    for M, Nn, K in [(1, 512, 8), (17, 4096, 4096), (129, 1032, 3080), (700, 2000, 520)]:
+        a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+        b = torch.randn(Nn, K, device="cuda", generator=g).bfloat16()
+        ref = _ref(a, b)
+        assert (gemm(a, b).float() - ref).norm() <= 3e-3 * ref.norm()
+        out = gemm(a, b, max_ctas=16)                             # a CTA limit keeps the persistent kernels
+        assert (out.float() - ref).norm() <= 3e-3 * ref.norm()
