@@ -132,24 +132,21 @@ struct GemmShape {
 
 // Warp-collective mbar_wait: every lane of a converged warp calls it and all of them get the
 // same answer (a lane that saw the barrier flip at the last moment must not go on alone to a
-// `.sync.aligned` instruction or an election while its neighbours give up).  With tracing on,
-// the waiting time is added to `*acc_cycles`.
+// `.sync.aligned` instruction or an election while its neighbours give up).  The usual case is one
+// try and one vote; the loop with its time limit is the slow path.  With tracing on (a lane may
+// trace while its neighbours do not, so nothing collective depends on it), the waiting time is
+// added to `*acc_cycles`.
 __device__ __forceinline__ bool mbar_wait_traced(uint64_t* bar, uint32_t parity,
                                                  volatile int* abort_flag, uint32_t* status,
                                                  uint32_t detail, bool tracing,
                                                  long long* acc_cycles) {
-  bool ok;
-  if (!tracing) {
-    // Usual case: every lane sees the phase complete at its first try.
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) != 0) return true;
-    ok = mbar_wait(bar, parity, abort_flag, status, detail);
-  } else {
-    // The whole call is timed: a try_wait may itself block for a while before it answers.
-    const long long t0 = clock64();
-    ok = mbar_wait(bar, parity, abort_flag, status, detail);
-    *acc_cycles += clock64() - t0;
-  }
-  return __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
+  // The whole call is timed: a try_wait may itself block for a while before it answers.
+  const long long t0 = tracing ? clock64() : 0;
+  bool ok = __all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) != 0;
+  if (!ok)
+    ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, detail) ? 1 : 0) != 0;
+  if (tracing) *acc_cycles += clock64() - t0;
+  return ok;
 }
 
 // Grouped rasterisation: consecutive tiles share a panel of up to `group` row

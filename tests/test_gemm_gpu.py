@@ -280,3 +280,16 @@ def test_gemm_choice_covers_the_range(native_lib):
         assert (gemm(a, b).float() - ref).norm() <= 3e-3 * ref.norm()
         out = gemm(a, b, max_ctas=16)                             # a CTA limit keeps the persistent kernels
         assert (out.float() - ref).norm() <= 3e-3 * ref.norm()
+
+
+@pytest.mark.parametrize("bn", [512, 256])
+def test_role_trace_runs_with_one_tracing_lane(native_lib, bn):
+    """Only lane 0 of the first epilogue warp traces: the waits, which are warp-collective, must not
+    depend on it."""
+    from commbench_b200.ops.gemm import gemm_role_trace
+
+    a = torch.randn(300, 1024, device="cuda").bfloat16()
+    b = torch.randn(520, 1024, device="cuda").bfloat16()
+    r = gemm_role_trace(a, b, bn)
+    assert r["mma_cycles"] > 0
+    assert all(0.0 <= v <= 1.0 for k, v in r.items() if k != "mma_cycles"), r
