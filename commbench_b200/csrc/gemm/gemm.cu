@@ -412,7 +412,8 @@ int cb_gemm_fp8(const void* a, const void* b, void* c, int M, int N, int K, floa
 // columns), b [N,K] e4m3 with b_scale [ceil(N/128), K/128] (one per 128 x 128 block); K % 128 == 0.
 // C = alpha * (a * a_scale) (b * b_scale)^T in bf16.  The quantised operands feed the tensor
 // cores directly; every 128-wide K block's partial sum is scaled and accumulated in fp32
-// registers.  pair != 0: CTA pairs (256 x 256 tiles), else one CTA per 128 x 256 tile.
+// registers.  One CTA per 128 x 256 tile; `pair` is accepted and makes no difference (a pair per
+// 256 x 256 tile was slower at every size, see gemm_sm100.cuh).
 int cb_gemm_fp8_blockscaled(const void* a, const void* a_scale, const void* b, const void* b_scale,
                             void* c, int M, int N, int K, float alpha, int pair, int max_ctas,
                             void* status, void* stream) {
@@ -425,9 +426,7 @@ int cb_gemm_fp8_blockscaled(const void* a, const void* a_scale, const void* b, c
   uint32_t* s = static_cast<uint32_t*>(status);
   const float* as = static_cast<const float*>(a_scale);
   const float* bs = static_cast<const float*>(b_scale);
-  if (pair)
-    return launch_plain<GemmCfg<256, 5, true, 2, true>>(a, b, c, M, N, K, alpha, s, max_ctas, st,
-                                                        nullptr, as, bs);
+  (void)pair;
   return launch_plain<GemmCfg<256, 3, true, 1, true>>(a, b, c, M, N, K, alpha, s, max_ctas, st,
                                                       nullptr, as, bs);
 }

@@ -9,7 +9,6 @@ empty_thunderkitten_gemm_ar.cu:84-191).
 from __future__ import annotations
 
 import ctypes as C
-import functools
 
 import torch
 
@@ -23,11 +22,6 @@ class GemmError(RuntimeError):
 def _check(t: torch.Tensor, name: str):
     if not (t.is_cuda and t.is_contiguous() and t.dim() == 2 and t.data_ptr() % 16 == 0):
         raise GemmError(f"{name} must be a contiguous, 16-byte aligned 2-D CUDA tensor")
-
-
-@functools.lru_cache(maxsize=None)
-def _sm_count(device: torch.device) -> int:
-    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, alpha: float = 1.0,
@@ -185,7 +179,8 @@ def gemm_fp8_blockscaled(a_q, a_s, b_q, b_s, out=None, alpha: float = 1.0, pair:
                          max_ctas: int = 0, status_ptr: int = 0, stream=None):
     """``out = (a_q * a_s [1x128 blocks]) @ (b_q * b_s [128x128 blocks]).T`` on the fp8 tensor
     cores: the quantised operands are the MMA operands, and every 128-wide K block's partial sum
-    is multiplied by its two scales and accumulated in fp32 registers inside the kernel."""
+    is multiplied by its two scales and accumulated in fp32 registers inside the kernel.
+    ``pair`` makes no difference any more: one CTA per tile is the faster form at every size."""
     lib = N.load()
     _check(a_q, "a_q")
     _check(b_q, "b_q")
@@ -204,9 +199,6 @@ def gemm_fp8_blockscaled(a_q, a_s, b_q, b_s, out=None, alpha: float = 1.0, pair:
         out = a_q.new_empty((M, Nn), dtype=torch.bfloat16)
     else:
         _check(out, "out")
-    if pair is None:
-        nsm = _sm_count(a_q.device)
-        pair = ((M + 255) // 256) * ((Nn + 255) // 256) * 2 >= nsm
     rc = lib.cb_gemm_fp8_blockscaled(a_q.data_ptr(), a_s.data_ptr(), b_q.data_ptr(), b_s.data_ptr(),
                                      out.data_ptr(), M, Nn, K, alpha, int(bool(pair)), max_ctas,
                                      status_ptr, N.raw_stream(stream))
