@@ -50,10 +50,12 @@
 // "UE8M0", chosen at quantisation) the tensor core applies them itself
 // (`tcgen05.mma.kind::mxf8f6f4.block_scale`), reading one scale byte per operand row and 32
 // K-elements from tensor memory, and the whole K loop accumulates in TMEM as in the unscaled
-// kernels.  Four scale warps (one per TMEM lane quadrant) fetch the bytes of the next K blocks
-// and store them into a ring of scale-factor columns beside the accumulators (tcgen05.st),
-// one slot per ring stage; tiles are 128 x 192 so that two accumulators and the ring fit
-// in the 512 columns.
+// kernels.  A scale word packs the exponents of four consecutive 128-wide K blocks of a row; the
+// hardware reads a word as the scales of four 32-wide steps and an instruction selects a byte, so the
+// packed words serve as they are, every step of K block j selecting byte j.  Four scale warps fetch
+// the words of the next groups of four K blocks and lay them out in shared memory; the MMA thread
+// copies a group into its scale-factor columns (tcgen05.cp) once, before its first MMA.  Tiles are
+// 192 columns wide so that two accumulators and the scale columns fit in the 512 columns.
 //
 // No load in this file is a cluster-multicast load.  Every wait is bounded: on a
 // time-out the CTA raises its abort word (and its partner's), every role leaves
@@ -73,8 +75,7 @@ template <int BN_, int STAGES_, bool FP8_, int PAIR_ = 1, bool BS_ = false, bool
 struct GemmCfg {
   static constexpr bool MX = MX_;             // power-of-two block scales applied by the tensor core
   static constexpr int SF_BASE = 2 * BN_;     // first scale-factor column in TMEM (MX)
-  static constexpr int SF_STRIDE = 16;        // columns per K block: 4 for A rows, up to 8 for B rows
-  static constexpr int SF_SLOTS = 8;          // K blocks of scale factors in TMEM: 2 groups of 4
+  static constexpr int SF_STRIDE = 16;        // columns per group: 4 for A rows, up to 8 for B rows
   static constexpr int PAIR = PAIR_;          // CTAs that share a tile (1, or 2 = a cluster)
   static constexpr bool BS = BS_;             // block-scaled fp8 with promotion in registers
   static constexpr int EPI_WARPS = BS_ ? 8 : 4;
@@ -92,18 +93,21 @@ struct GemmCfg {
   static constexpr int EPI_COLS = 64;                 // bf16 columns per store box (128 B)
   static constexpr int EPI_BUF_BYTES = 32 * 128;      // 32 rows x 128 B per warp and buffer
   static constexpr int EPI_BYTES = EPI_WARPS * 2 * EPI_BUF_BYTES;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024;
+  static constexpr int SF_GROUPS = 4;         // groups of 4 K blocks of scale factors on chip
+  static constexpr int SF_GROUP_BYTES = MX_ ? 3 * 512 : 0;   // A rows, B rows 0..127, B rows 128..255
+  static constexpr int SF_BYTES = SF_GROUPS * SF_GROUP_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + SF_BYTES + 1024;
   static constexpr int TMEM_COLS = MX_ ? 512 : 2 * BN;
   // Warp roles.  Plain: producer, MMA, 4 epilogue warps, signal warp.  Block-scaled: a
   // utility warp-group (producer, MMA, signal, one idle warp) that gives registers away and
   // two epilogue warp-groups that take them (setmaxnreg works on whole warp-groups).
   static constexpr int EPI_WARP0 = BS_ ? 4 : 2;
   static constexpr int SIGNAL_WARP = BS_ ? 2 : 6;
-  static constexpr int SCALE_WARP0 = 8;       // MX: warps 8..11 write scale factors
+  static constexpr int SCALE_WARP0 = 8;       // MX: warps 8..11 stage scale factors
   static constexpr int THREADS = (BS_ || MX_) ? 384 : 224;
   static_assert(!MX_ || (FP8_ && !BS_ && BN_ <= 192 &&
-                         2 * BN_ + SF_SLOTS * SF_STRIDE <= 512),
-                "hardware block scales: fp8, accumulators + scale ring within 512 TMEM columns");
+                         2 * BN_ + 4 * SF_STRIDE <= 512),
+                "hardware block scales: fp8, accumulators + scale slots within 512 TMEM columns");
   static_assert(!BS_ || (FP8_ && BN_ == 256 && PAIR_ == 1),
                 "block scales: fp8 operands, 256-column tiles, one CTA per tile");
   static_assert(PAIR_ == 1 || PAIR_ == 2, "one CTA or a pair per tile");
@@ -184,8 +188,8 @@ struct GemmCtl {
   uint64_t empty[STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
-  uint64_t sf_full[2];    // scale warps -> MMA thread: a group of 4 K blocks of scale factors is in TMEM
-  uint64_t sf_empty[2];   // MMA thread -> scale warps: the group's MMAs are done
+  uint64_t sf_full[4];    // scale warps -> MMA thread: a group of 4 K blocks of scale factors is staged
+  uint64_t sf_empty[4];   // MMA thread -> scale warps: the group's MMAs are done
   uint64_t sig_full[8];   // epilogue warps -> signal warp: a tile's stores were issued
   uint64_t sig_empty[8];  // signal warp -> epilogue warps: slot may be reused
   uint32_t tmem_base;
@@ -412,14 +416,16 @@ __device__ __forceinline__ void gemm_mma_bs(const P& p, const GemmShape& g, uint
   }
 }
 
-// MMA role with hardware block scales: as gemm_mma, plus the wait for the stage's scale
-// factors and the scale-factor operands of the instruction.
+// MMA role with hardware block scales: as gemm_mma, plus the copy of a group's scale factors to
+// TMEM and the scale-factor operands of the instruction.  Two K blocks per wait and election.
 template <class Cfg, class Policy, class P>
 __device__ __forceinline__ void gemm_mma_mx(const P& p, const GemmShape& g, uint8_t* ring,
-                                            GemmCtl<Cfg::STAGES>* ctl, uint32_t* status, int cta,
-                                            int num_ctas, uint32_t tmem_base) {
+                                            const uint8_t* sf_smem, GemmCtl<Cfg::STAGES>* ctl,
+                                            uint32_t* status, int cta, int num_ctas,
+                                            uint32_t tmem_base) {
   uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
   const int ntiles = Policy::num_tiles(p);
+  const uint64_t sf_desc0 = make_sf_copy_desc(smem_u32(sf_smem));
   const uint64_t a_desc0 = make_sw128_kmajor_desc(smem_u32(ring));
   constexpr uint64_t kStageStep = static_cast<uint64_t>(Cfg::STAGE_BYTES >> 4);
   constexpr uint64_t kBStep = static_cast<uint64_t>(Cfg::A_BYTES >> 4);
@@ -429,6 +435,29 @@ __device__ __forceinline__ void gemm_mma_mx(const P& p, const GemmShape& g, uint
   const uint32_t empty0_peer = Cfg::PAIR == 2 ? map_to_cta(empty0, 1) : 0u;
   const uint32_t tfull0_peer = Cfg::PAIR == 2 ? map_to_cta(tfull0, 1) : 0u;
   const uint32_t sfe0_peer = Cfg::PAIR == 2 ? map_to_cta(sfe0, 1) : 0u;
+  auto commit = [&](uint32_t local, uint32_t peer) {
+    if constexpr (Cfg::PAIR == 2) {
+      mma_commit_pair(local);
+      mma_commit_pair(peer);
+    } else {
+      mma_commit_addr(local);
+    }
+  };
+  // K block `j` of its group, in ring slot `st`: four K steps of 32, all with byte j of the columns.
+  auto issue = [&](uint32_t d_tmem, uint32_t sfa, uint32_t st, uint32_t j, uint32_t accumulate) {
+    const uint64_t a_desc = a_desc0 + st * kStageStep;
+    const uint64_t b_desc = a_desc + kBStep;
+    const uint32_t idesc = make_idesc_mx(Cfg::BM, Cfg::BN, 0u) | (j << 29) | (j << 4);
+#pragma unroll
+    for (int k = 0; k < Cfg::MMAS_PER_STAGE; ++k) {
+      const uint32_t accum = k > 0 ? 1u : accumulate;
+      if constexpr (Cfg::PAIR == 2)
+        mma_mxf8_ss_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, sfa, sfa + 4u, accum);
+      else
+        mma_mxf8_ss(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, sfa, sfa + 4u, accum);
+    }
+    commit(empty0 + st * 8u, empty0_peer + st * 8u);
+  };
   uint32_t gcount = 0;  // groups of 4 K blocks so far (a tile starts a new group)
   const bool tracing = g.trace != nullptr;  // [0] operands, [1] accumulator + scale factors
   long long w_full = 0, w_other = 0;
@@ -439,62 +468,50 @@ __device__ __forceinline__ void gemm_mma_mx(const P& p, const GemmShape& g, uint
       return;
     tc_fence_after_sync();
     const uint32_t d_tmem = tmem_base + acc * Cfg::BN;
-    for (int kb = 0; kb < g.num_k_blocks; ++kb) {
-      const uint32_t grp = gcount & 1u;
-      if ((kb & 3) == 0 &&
-          !mbar_wait_traced(&ctl->sf_full[grp], (gcount >> 1) & 1u, &ctl->abort_flag, status,
+    for (int kg = 0; kg < g.num_k_blocks; kg += 4, ++gcount) {
+      const uint32_t grp = gcount & 3u;
+      if (!mbar_wait_traced(&ctl->sf_full[grp], (gcount >> 2) & 1u, &ctl->abort_flag, status,
                             0x380 + grp, tracing, &w_other))
         return;
-      if (!mbar_wait_traced(&ctl->full[stage], phase, &ctl->abort_flag, status, 0x300 + stage,
-                            tracing, &w_full))
-        return;
-      tc_fence_after_sync();
-      const bool group_ends = (kb & 3) == 3 || kb == g.num_k_blocks - 1;
-      // Operands are computed by the whole (converged) warp, so they can live in uniform
-      // registers; only the asynchronous instructions themselves sit under the election.
-      const uint64_t a_desc = a_desc0 + stage * kStageStep;
-      const uint64_t b_desc = a_desc + kBStep;
-      const uint32_t sfa =
-          tmem_base + Cfg::SF_BASE + (grp * 4u + static_cast<uint32_t>(kb & 3)) * Cfg::SF_STRIDE;
-      const uint32_t sfb = sfa + 4u;
-      const uint32_t first = kb > 0 ? 1u : 0u;
-      if (elect_one()) {
-        // Four K steps of 32; step j takes byte j of the scale columns.
-        if constexpr (Cfg::PAIR == 2) {
-          mma_mxf8_ss_pair(d_tmem, a_desc, b_desc, make_idesc_mx(Cfg::BM, Cfg::BN, 0u), sfa, sfb, first);
-          mma_mxf8_ss_pair(d_tmem, a_desc + 2u, b_desc + 2u, make_idesc_mx(Cfg::BM, Cfg::BN, 1u), sfa, sfb, 1u);
-          mma_mxf8_ss_pair(d_tmem, a_desc + 4u, b_desc + 4u, make_idesc_mx(Cfg::BM, Cfg::BN, 2u), sfa, sfb, 1u);
-          mma_mxf8_ss_pair(d_tmem, a_desc + 6u, b_desc + 6u, make_idesc_mx(Cfg::BM, Cfg::BN, 3u), sfa, sfb, 1u);
-          mma_commit_pair(empty0 + stage * 8u);
-          mma_commit_pair(empty0_peer + stage * 8u);
-          if (group_ends) {  // the group's scale columns are free, in both CTAs
-            mma_commit_pair(sfe0 + grp * 8u);
-            mma_commit_pair(sfe0_peer + grp * 8u);
+      const uint32_t sfa = tmem_base + Cfg::SF_BASE + grp * Cfg::SF_STRIDE;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int left = g.num_k_blocks - kg - 2 * half;
+        if (left <= 0) break;
+        const bool two = left > 1;
+        const uint32_t stage1 = stage + 1 == Cfg::STAGES ? 0u : stage + 1u;
+        const uint32_t phase1 = stage + 1 == Cfg::STAGES ? phase ^ 1u : phase;
+        const long long t0 = tracing ? clock64() : 0;
+        const bool ok =
+            two ? mbar_wait_both(&ctl->full[stage], phase, 0x300 + stage, &ctl->full[stage1], phase1,
+                                 0x300 + stage1, &ctl->abort_flag, status)
+                : mbar_wait_traced(&ctl->full[stage], phase, &ctl->abort_flag, status, 0x300 + stage,
+                                   false, nullptr);
+        if (tracing) w_full += clock64() - t0;
+        if (!ok) return;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          if (half == 0) {
+            const uint64_t d = sf_desc0 + grp * static_cast<uint64_t>(Cfg::SF_GROUP_BYTES >> 4);
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+              if constexpr (Cfg::PAIR == 2) tmem_copy_sf_pair(sfa + part * 4u, d + part * 32u);
+              else tmem_copy_sf(sfa + part * 4u, d + part * 32u);
+            }
           }
-        } else {
-          mma_mxf8_ss(d_tmem, a_desc, b_desc, make_idesc_mx(Cfg::BM, Cfg::BN, 0u), sfa, sfb, first);
-          mma_mxf8_ss(d_tmem, a_desc + 2u, b_desc + 2u, make_idesc_mx(Cfg::BM, Cfg::BN, 1u), sfa, sfb, 1u);
-          mma_mxf8_ss(d_tmem, a_desc + 4u, b_desc + 4u, make_idesc_mx(Cfg::BM, Cfg::BN, 2u), sfa, sfb, 1u);
-          mma_mxf8_ss(d_tmem, a_desc + 6u, b_desc + 6u, make_idesc_mx(Cfg::BM, Cfg::BN, 3u), sfa, sfb, 1u);
-          mma_commit_addr(empty0 + stage * 8u);
-          if (group_ends) mma_commit_addr(sfe0 + grp * 8u);  // the group's scale columns are free
+          issue(d_tmem, sfa, stage, 2u * half, kg + half > 0 ? 1u : 0u);
+          if (two) issue(d_tmem, sfa, stage1, 2u * half + 1u, 1u);
+          if (half == 1 || left <= 2) commit(sfe0 + grp * 8u, sfe0_peer + grp * 8u);
         }
-      }
-      __syncwarp();
-      if (group_ends) ++gcount;
-      if (++stage == Cfg::STAGES) {
-        stage = 0;
-        phase ^= 1u;
-      }
-    }
-    if (elect_one()) {
-      if constexpr (Cfg::PAIR == 2) {
-        mma_commit_pair(tfull0 + acc * 8u);
-        mma_commit_pair(tfull0_peer + acc * 8u);
-      } else {
-        mma_commit_addr(tfull0 + acc * 8u);
+        __syncwarp();
+        for (int i = 0; i < (two ? 2 : 1); ++i)
+          if (++stage == Cfg::STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
       }
     }
+    if (elect_one()) commit(tfull0 + acc * 8u, tfull0_peer + acc * 8u);
     __syncwarp();
     acc ^= 1u;
     if (acc == 0u) acc_phase ^= 1u;
@@ -520,29 +537,28 @@ __device__ __forceinline__ const uint32_t* tile_a_sf(const P& p, const GemmShape
   }
 }
 
-// Scale warp (one per TMEM lane quadrant; all four write the same data, the layout wants it
-// replicated): lane l holds rows l, l+32, l+64, l+96 of A and l, l+32, ... of the B tile.  It
-// works in groups of four K blocks - one 32-bit load per row brings their four exponent bytes,
-// the next group's loads in flight meanwhile - and two groups of TMEM columns alternate: wait
-// until the MMAs of the group's previous use are done, store 4 x (4 + 8) columns, one
-// tcgen05.wait::st, one arrival.
+// Scale warp w of four: every fourth group of 4 K blocks, staged in slot w.  Lane l holds the words of
+// rows l, l+32, l+64, l+96 of A and l, l+32, ... of the B tile, and stores them as 3 x 16 bytes, the
+// order in which tcgen05.cp spreads 512 bytes over lanes and columns.  The loads of a group are
+// issued before the wait for its slot, so with four warps four groups of loads are in flight.
+// (The columns used to be written by tcgen05.st, bytes replicated for every K block: a group's trip from
+// free to filled was longer than the MMAs in between and the MMA warp waited 40 % of its time.
+// 8192 x 3584 x 8192: 243 us then, 179 now, plain fp8 162.)
 template <class Cfg, class Policy, class P>
-__device__ __forceinline__ void gemm_scale_writer(const P& p, const GemmShape& g,
+__device__ __forceinline__ void gemm_scale_stager(const P& p, const GemmShape& g, uint8_t* sf_smem,
                                                   GemmCtl<Cfg::STAGES>* ctl, uint32_t* status,
-                                                  int cta, int num_ctas, uint32_t tmem_base,
-                                                  uint32_t warp, uint32_t lane, int sub) {
+                                                  int cta, int num_ctas, uint32_t w, uint32_t lane,
+                                                  int sub) {
   constexpr int NB = Cfg::BN / 32;  // B-row groups of this tile (<= 8)
-  const uint32_t q = warp & 3u;
-  uint32_t gcount = 0;  // groups of 4 K blocks so far, in step with the MMA role
-  int tcount = 0;       // tiles so far, against the producer's count of tiles whose A rows are there
   const int ntiles = Policy::num_tiles(p);
   const int nkb = g.num_k_blocks;
-  const uint32_t t0 = tmem_base + ((q * 32u) << 16) + Cfg::SF_BASE;
+  uint32_t gcount = 0;  // groups so far, in step with the MMA role
+  int tcount = 0;       // tiles so far, against the producer's count of tiles whose A rows are there
   constexpr uint32_t kOne = 0x7f7f7f7fu;  // exponent 127 = 1.0, for rows outside the operands
+  uint4* const dst = reinterpret_cast<uint4*>(sf_smem + w * Cfg::SF_GROUP_BYTES + lane * 16u);
   for (int tile = cta; tile < ntiles; tile += num_ctas) {
     int m_blk, n_blk;
     Policy::tile_coord(p, tile, &m_blk, &n_blk);
-    // this CTA's 128 rows of the tile; all BN columns of B
     // A tile whose A rows come from another rank: its scale words arrive with the rows.  The
     // producer waits for them before its first load of the tile and then counts the tile in
     // `a_ready_tiles`; this warp follows that count.
@@ -569,59 +585,41 @@ __device__ __forceinline__ void gemm_scale_writer(const P& p, const GemmShape& g
       ++tcount;
     }
     long long pitch_a = 0;
+    // this CTA's 128 rows of the tile; all BN columns of B
     const uint32_t* pa = tile_a_sf<Policy>(p, g, m_blk, &pitch_a) + sub * Cfg::CTA_M;
     const int a_rows_left = g.M - m_blk * Cfg::BM - sub * Cfg::CTA_M;
     const int b_row0 = Policy::b_row(p, m_blk, n_blk);
     const int b_rows_left = g.N - n_blk * Cfg::BN;
-    auto load_group = [&](int kb, uint32_t (&wa)[4], uint32_t (&wb)[NB]) {
+    for (int kg = 0; kg < nkb; kg += 4, ++gcount) {
+      if ((gcount & 3u) != w) continue;
+      uint32_t wa[4], wb[8];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int r = c * 32 + static_cast<int>(lane);
         // L2-coherent load: the words of gathered rows were written by a peer during this launch
-        wa[c] = (kb < nkb && r < a_rows_left) ? __ldcg(pa + (kb >> 2) * pitch_a + r) : kOne;
+        wa[c] = r < a_rows_left ? __ldcg(pa + (kg >> 2) * pitch_a + r) : kOne;
       }
 #pragma unroll
-      for (int c = 0; c < NB; ++c) {
+      for (int c = 0; c < 8; ++c) {
         const int r = c * 32 + static_cast<int>(lane);
-        wb[c] = (kb < nkb && r < b_rows_left)
-                    ? __ldg(g.sfb + static_cast<long long>(kb >> 2) * g.sfb_rows + b_row0 + r)
+        wb[c] = (c < NB && r < b_rows_left)
+                    ? __ldg(g.sfb + static_cast<long long>(kg >> 2) * g.sfb_rows + b_row0 + r)
                     : kOne;
       }
-    };
-    uint32_t wa[4], wb[NB], na[4], nb[NB];
-    load_group(0, wa, wb);
-    for (int kg = 0; kg < nkb; kg += 4) {
-      load_group(kg + 4, na, nb);  // in flight while this group is written
-      const uint32_t grp = gcount & 1u;
-      if (!mbar_wait_traced(&ctl->sf_empty[grp], ((gcount >> 1) & 1u) ^ 1u, &ctl->abort_flag,
-                            status, 0x500 + grp, false, nullptr))
+      if (!mbar_wait_traced(&ctl->sf_empty[w], ((gcount >> 2) & 1u) ^ 1u, &ctl->abort_flag, status,
+                            0x500 + w, false, nullptr))
         return;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t ra[4], rb[8];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) ra[c] = ((wa[c] >> (8 * j)) & 0xffu) * 0x01010101u;
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          rb[c] = c < NB ? ((wb[c < NB ? c : 0] >> (8 * j)) & 0xffu) * 0x01010101u : kOne;
-        const uint32_t t = t0 + (grp * 4u + j) * Cfg::SF_STRIDE;
-        tmem_st_32x4(t, ra);
-        tmem_st_32x8(t + 4u, rb);
-      }
-      tmem_wait_st();
-      tc_fence_before_sync();
+      dst[0] = make_uint4(wa[0], wa[1], wa[2], wa[3]);
+      dst[32] = make_uint4(wb[0], wb[1], wb[2], wb[3]);
+      dst[64] = make_uint4(wb[4], wb[5], wb[6], wb[7]);
+      fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
         if (Cfg::PAIR == 2 && sub != 0)
-          mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->sf_full[grp]), 0));
+          mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->sf_full[w]), 0));
         else
-          mbar_arrive(&ctl->sf_full[grp]);
+          mbar_arrive(&ctl->sf_full[w]);
       }
-      ++gcount;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) wa[c] = na[c];
-#pragma unroll
-      for (int c = 0; c < NB; ++c) wb[c] = nb[c];
     }
   }
 }
@@ -1233,8 +1231,8 @@ __device__ __forceinline__ uint32_t gemm_setup(GemmCtl<Cfg::STAGES>* ctl, uint32
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&ctl->sf_full[i], 4 * Cfg::PAIR);  // one arrival per scale warp (of the pair)
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&ctl->sf_full[i], Cfg::PAIR);   // one arrival per CTA
       mbar_init(&ctl->sf_empty[i], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -1343,15 +1341,16 @@ __device__ __forceinline__ void gemm_cta_main(const P& p, const GemmShape& g, ui
   } else if (warp == 1) {
     if constexpr (Cfg::MX) {
       if (sub == 0)
-        gemm_mma_mx<Cfg, Policy>(p, g, ring, &ctl, status, worker, num_workers, tmem_base);
+        gemm_mma_mx<Cfg, Policy>(p, g, ring, epi + Cfg::EPI_BYTES, &ctl, status, worker, num_workers,
+                                 tmem_base);
     } else {
       if (sub == 0)
         gemm_mma<Cfg, Policy>(p, g, ring, &ctl, status, worker, num_workers, tmem_base);
     }
   } else if (Cfg::MX && warp >= Cfg::SCALE_WARP0) {
     if constexpr (Cfg::MX)
-      gemm_scale_writer<Cfg, Policy>(p, g, &ctl, status, worker, num_workers, tmem_base, warp,
-                                     lane, sub);
+      gemm_scale_stager<Cfg, Policy>(p, g, epi + Cfg::EPI_BYTES, &ctl, status, worker, num_workers,
+                                     warp - Cfg::SCALE_WARP0, lane, sub);
   } else if (warp < 2 + Cfg::EPI_WARPS) {
     gemm_epilogue<Cfg, Policy>(p, g, epi, &ctl, status, worker, num_workers, tmem_base, warp,
                                lane, sub);

@@ -162,19 +162,21 @@ __device__ __forceinline__ void mma_mxf8_ss_pair(uint32_t d_tmem, uint64_t a_des
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
-// 32 lanes x 4 / 8 columns stores (registers -> TMEM), thread t writes lane (base + t).
-__device__ __forceinline__ void tmem_st_32x4(uint32_t taddr, const uint32_t (&r)[4]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr),
-               "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
-               : "memory");
+// Shared memory -> TMEM copy of scale factors: 512 contiguous bytes, lane i's 16 at 16 i, become four
+// columns of 32 lanes, repeated in all four lane quadrants - the layout block_scale operands are read
+// in.  Asynchronous, issued by the MMA thread: tcgen05.mma issued afterwards by the same thread sees it.
+// The pair form copies in both CTAs, each from its own shared memory.
+__device__ __forceinline__ uint64_t make_sf_copy_desc(uint32_t smem_addr) {
+  return static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4)   // start address
+         | (static_cast<uint64_t>(128 >> 4) << 32)            // stride between groups of 8 lanes
+         | (static_cast<uint64_t>(1) << 46);                  // descriptor version; no swizzle
 }
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-      : "memory");
+__device__ __forceinline__ void tmem_copy_sf(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
 }
-
+__device__ __forceinline__ void tmem_copy_sf_pair(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
 // ------------------------------------------------- CTA pairs (cta_group::2)
 // A pair is the two CTAs of a cluster of 2.  Both CTAs run the allocation and
 // the free (same warp index, same shared-memory word), the even CTA issues the
