@@ -21,7 +21,15 @@
 //     which otherwise is as busy as the tensor pipe;
 //   * CTAs draw tickets: the first `num_comm` tickets copy the list of 2-D pieces
 //     (peer -> local, 16-byte loads and stores), bumping each piece's counter when done; the
-//     others take (query tile pair, head, batch) items, heaviest first.
+//     others take (query tile pair, head, batch) items, heaviest first.  A launch without
+//     communication CTAs is persistent: one CTA per SM walks its share of the items, and the next
+//     item's Q, keys and first scores overlap this one's last products and its epilogue (with one
+//     CTA per item, launch, tensor-memory allocation and the pipeline's fill and drain cost 8 to 15 us
+//     an item: 16384 tokens, 32 / 8 heads, causal 2231 us then, 2064 now; 1000 queries over 7000 keys
+//     130, 122; 2 x 3000 tokens, 16 / 4 heads 109, 99).
+// What bounds the inner loop (3500 cycles for 128 keys x 256 rows against 2048 on the tensor cores): the
+// MMA warp's issue, 32 MMAs at about 75 cycles, and behind it a tile's chain scores -> softmax (1700) ->
+// P -> product -> next scores; the exponentials alone are not (without them: the same time).
 // No CTA waits for another GPU inside this kernel: remote data is pulled, and the cross-GPU
 // barriers that say "shards are published" / "shards may be overwritten" bracket the launch.
 //
@@ -41,7 +49,7 @@
 namespace cb {
 
 struct CpCtl {
-  uint64_t q_full;
+  uint64_t q_full, q_empty;
   uint64_t k_full[CP_KST], k_empty[CP_KST];
   uint64_t v_full[CP_VST], v_empty[CP_VST];
   uint64_t s_full[2], p_full[2], pv_done[2];  // per query tile
@@ -84,6 +92,13 @@ __device__ __forceinline__ float cp_max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
+}
+
+// Scores from the `visible`-th on become -inf.  One compare per element against a constant: with the
+// two conditions of the mask written out per element a masked block took 6.5 us instead of 1.
+__device__ __forceinline__ void cp_mask_tail(uint32_t (&s)[128], int visible) {
+#pragma unroll
+  for (int i = 0; i < 128; ++i) s[i] = i < visible ? s[i] : 0xff800000u;
 }
 
 // One block of the online softmax: the 128 masked scores of this thread's row in `s` become the
@@ -265,6 +280,43 @@ __device__ __forceinline__ void cp_reg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+// One attention item: a pair of query tiles of one head and batch.  Pairs run from the end of a query
+// segment to its start (under a causal mask the late rows are the long items).
+struct CpItem {
+  int qs_i, pair, head, batch;
+  int q_first, q_last;   // positions of the pair's first row and last valid row
+  int nblk;              // key blocks it visits
+  __device__ __forceinline__ bool decode(const FaCpParams& p, int item) {
+    const int per_pair = p.heads * p.B;
+    int gp = item / per_pair;
+    const int rem = item - gp * per_pair;
+    head = rem % p.heads;
+    batch = rem / p.heads;
+    for (qs_i = 0; qs_i < p.nqseg; ++qs_i) {
+      const int np = (p.qseg[qs_i].nrows + 2 * CP_BM - 1) / (2 * CP_BM);
+      if (gp < np) {
+        pair = np - 1 - gp;
+        q_first = p.qseg[qs_i].qpos0 + pair * 2 * CP_BM;
+        int rows = p.qseg[qs_i].nrows - pair * 2 * CP_BM;
+        if (rows > 2 * CP_BM) rows = 2 * CP_BM;
+        q_last = q_first + rows - 1;
+        nblk = CpBlockIter::total(p, q_last);
+        return true;
+      }
+      gp -= np;
+    }
+    return false;
+  }
+  // The i-th item of a CTA.  With tickets a CTA has one.  A launch without them is persistent: one CTA
+  // per SM walks the list, heaviest items first, forwards in even rounds and backwards in odd
+  // ones, which evens out what the CTAs get.
+  __device__ __forceinline__ bool at(const FaCpParams& p, int ticket, int i) {
+    if (p.sched != nullptr) return i == 0 && decode(p, ticket - p.num_comm);
+    const int g = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
+    return decode(p, i * g + ((i & 1) != 0 ? g - 1 - c : c));
+  }
+};
+
 // kPoly: every kPoly-th pair of keys takes its exponential from the FMA pipe (0: none).
 template <int kPoly>
 __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_constant__ FaCpParams p) {
@@ -285,41 +337,16 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
     __syncthreads();
     ticket = ctl.ticket;
   }
-  bool attend = false;
-  int qs_i = 0, pair = 0, head = 0, batch = 0;
+  CpItem first;
   if (ticket < p.num_comm) {
     cp_comm_cta(p, ticket);
-  } else {
-    // item -> (query segment, tile pair inside it, head, batch); pairs run from the end of a
-    // segment to its start (under a causal mask the late rows are the long items)
-    int item = ticket - p.num_comm;
-    const int per_pair = p.heads * p.B;
-    int gp = item / per_pair;
-    const int rem = item - gp * per_pair;
-    head = rem % p.heads;
-    batch = rem / p.heads;
-    for (qs_i = 0; qs_i < p.nqseg; ++qs_i) {
-      const int np = (p.qseg[qs_i].nrows + 2 * CP_BM - 1) / (2 * CP_BM);
-      if (gp < np) {
-        pair = np - 1 - gp;
-        attend = true;
-        break;
-      }
-      gp -= np;
-    }
-  }
-
-  if (attend) {
-    const CpQSeg qs = p.qseg[qs_i];
-    const int q_first = qs.qpos0 + pair * 2 * CP_BM;          // position of row 0 of tile 0
-    int rows_here = qs.nrows - pair * 2 * CP_BM;              // valid query rows of this pair
-    if (rows_here > 2 * CP_BM) rows_here = 2 * CP_BM;
-    const int q_last = q_first + rows_here - 1;
-    const int nblk = CpBlockIter::total(p, q_last);
-    const int kv_head = head / p.kv_group;
-
+  } else if (first.at(p, ticket, 0)) {
+    // Every role walks the CTA's items with a copy of its own; block counts run through, so that
+    // barriers, rings and tensor memory carry over and the next item's Q, keys and scores overlap
+    // this one's last products and epilogue.
     if (threadIdx.x == 0) {
       mbar_init(&ctl.q_full, 1);
+      mbar_init(&ctl.q_empty, 1);
       for (int i = 0; i < CP_KST; ++i) {
         mbar_init(&ctl.k_full[i], 1);
         mbar_init(&ctl.k_empty[i], 1);
@@ -351,82 +378,97 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
     if (warp < 4) {
     cp_reg_dec<72>();
     if (warp == 0) {
-      if (lane == 0 && nblk > 0) {
+      if (lane == 0) {
         // ---------------------------------------------------------------- producer
-        const CUtensorMap* tmq = qs.map < 0 ? &p.tm_q_local : p.tm_q_arr + qs.map;
-        mbar_arrive_expect_tx(&ctl.q_full, 2 * CP_TILE);
-        const int qrow = batch * p.q_bstride + qs.row0 + pair * 2 * CP_BM;
-        for (int t = 0; t < 2; ++t) {
-          tma_load_3d(sQ + t * CP_TILE, tmq, 0, p.q_head0 + head, qrow + t * CP_BM, &ctl.q_full);
-          tma_load_3d(sQ + t * CP_TILE + CP_SUB, tmq, 64, p.q_head0 + head, qrow + t * CP_BM,
-                      &ctl.q_full);
-        }
-        CpBlockIter ik, iv;
-        ik.start(p, q_last);
-        iv.start(p, q_last);
-        int jk = 0, jv = 0, ready_seg = -1;
+        CpItem w;
         bool ok = true;
-        uint32_t idle = 0;
-        uint64_t t0 = 0;
-        while (ok && (jk < nblk || jv < nblk)) {
-          bool progress = false;
-          if (jk < nblk) {
-            const int s = jk % CP_KST, use = jk / CP_KST;
-            if (use == 0 || mbar_try_wait(&ctl.k_empty[s], (use - 1) & 1)) {
-              // First block of a segment that is still being pulled: wait for its counter.
-              // K and V of a segment arrive under the same counter.
-              if (ik.seg != ready_seg) {
-                const CpSeg& g = p.seg[ik.seg];
-                if (g.flag >= 0) {
-                  if (!wait_flag_ge_gpu(p.flags + g.flag, p.flag_target, p.timeout_ns, p.status,
-                                        40, static_cast<uint32_t>(ik.seg))) {
-                    ctl.abort_flag = 1;
-                    ok = false;
-                    break;
+        int g0 = 0, nq = 0;   // blocks and items before this item
+        for (int i = 0; ok && w.at(p, ticket, i); ++i) {
+          if (w.nblk == 0) continue;
+          const CpQSeg& qs = p.qseg[w.qs_i];
+          const int kv_head = w.head / p.kv_group;
+          if (nq > 0 && !mbar_wait(&ctl.q_empty, (nq - 1) & 1, &ctl.abort_flag, p.status, 0xE01))
+            break;
+          ++nq;
+          const CUtensorMap* tmq = qs.map < 0 ? &p.tm_q_local : p.tm_q_arr + qs.map;
+          mbar_arrive_expect_tx(&ctl.q_full, 2 * CP_TILE);
+          const int qrow = w.batch * p.q_bstride + qs.row0 + w.pair * 2 * CP_BM;
+          for (int t = 0; t < 2; ++t) {
+            tma_load_3d(sQ + t * CP_TILE, tmq, 0, p.q_head0 + w.head, qrow + t * CP_BM, &ctl.q_full);
+            tma_load_3d(sQ + t * CP_TILE + CP_SUB, tmq, 64, p.q_head0 + w.head, qrow + t * CP_BM,
+                        &ctl.q_full);
+          }
+          CpBlockIter ik, iv;
+          ik.start(p, w.q_last);
+          iv.start(p, w.q_last);
+          int jk = 0, jv = 0, ready_seg = -1;
+          uint32_t idle = 0;
+          uint64_t t0 = 0;
+          while (ok && (jk < w.nblk || jv < w.nblk)) {
+            bool progress = false;
+            if (jk < w.nblk) {
+              const int s = (g0 + jk) % CP_KST, use = (g0 + jk) / CP_KST;
+              if (use == 0 || mbar_try_wait(&ctl.k_empty[s], (use - 1) & 1)) {
+                // First block of a segment that is still being pulled: wait for its counter.
+                // K and V of a segment arrive under the same counter.
+                if (ik.seg != ready_seg) {
+                  const CpSeg& g = p.seg[ik.seg];
+                  if (g.flag >= 0) {
+                    if (!wait_flag_ge_gpu(p.flags + g.flag, p.flag_target, p.timeout_ns, p.status,
+                                          40, static_cast<uint32_t>(ik.seg))) {
+                      ctl.abort_flag = 1;
+                      ok = false;
+                      break;
+                    }
+                    fence_proxy_async();  // the rows were written with ordinary stores
                   }
-                  fence_proxy_async();  // the rows were written with ordinary stores
+                  ready_seg = ik.seg;
                 }
-                ready_seg = ik.seg;
+                const int krow = w.batch * p.kv_bstride + p.seg[ik.seg].row0 + ik.i * CP_BN;
+                mbar_arrive_expect_tx(&ctl.k_full[s], CP_TILE);
+                tma_load_3d(sK + s * CP_TILE, &p.tm_k, 0, kv_head, krow, &ctl.k_full[s]);
+                tma_load_3d(sK + s * CP_TILE + CP_SUB, &p.tm_k, 64, kv_head, krow, &ctl.k_full[s]);
+                ++jk;
+                ik.next(p, w.q_last);
+                progress = true;
               }
-              const int krow = batch * p.kv_bstride + p.seg[ik.seg].row0 + ik.i * CP_BN;
-              mbar_arrive_expect_tx(&ctl.k_full[s], CP_TILE);
-              tma_load_3d(sK + s * CP_TILE, &p.tm_k, 0, kv_head, krow, &ctl.k_full[s]);
-              tma_load_3d(sK + s * CP_TILE + CP_SUB, &p.tm_k, 64, kv_head, krow, &ctl.k_full[s]);
-              ++jk;
-              ik.next(p, q_last);
-              progress = true;
+            }
+            if (jv < w.nblk && jv < jk) {
+              const int s = (g0 + jv) % CP_VST, use = (g0 + jv) / CP_VST;
+              if (use == 0 || mbar_try_wait(&ctl.v_empty[s], (use - 1) & 1)) {
+                const int vrow = w.batch * p.kv_bstride + p.seg[iv.seg].row0 + iv.i * CP_BN;
+                mbar_arrive_expect_tx(&ctl.v_full[s], CP_TILE);
+                tma_load_3d(sV + s * CP_TILE, &p.tm_v, 0, kv_head, vrow, &ctl.v_full[s]);
+                tma_load_3d(sV + s * CP_TILE + CP_SUB, &p.tm_v, 64, kv_head, vrow, &ctl.v_full[s]);
+                ++jv;
+                iv.next(p, w.q_last);
+                progress = true;
+              }
+            }
+            if (progress) {
+              idle = 0;
+              continue;
+            }
+            if ((++idle & 255u) == 0u) {
+              if (*reinterpret_cast<volatile int*>(&ctl.abort_flag) != 0) {
+                ok = false;
+                break;
+              }
+              const uint64_t now = globaltimer_ns();
+              if (t0 == 0 || idle == 256u) t0 = now;
+              if (now - t0 > CB_MBAR_TIMEOUT_NS) {
+                ctl.abort_flag = 1;
+                report_status(p.status, CB_TIMEOUT_MBARRIER, 0, 0xE00);
+                ok = false;
+                break;
+              }
             }
           }
-          if (jv < nblk && jv < jk) {
-            const int s = jv % CP_VST, use = jv / CP_VST;
-            if (use == 0 || mbar_try_wait(&ctl.v_empty[s], (use - 1) & 1)) {
-              const int vrow = batch * p.kv_bstride + p.seg[iv.seg].row0 + iv.i * CP_BN;
-              mbar_arrive_expect_tx(&ctl.v_full[s], CP_TILE);
-              tma_load_3d(sV + s * CP_TILE, &p.tm_v, 0, kv_head, vrow, &ctl.v_full[s]);
-              tma_load_3d(sV + s * CP_TILE + CP_SUB, &p.tm_v, 64, kv_head, vrow, &ctl.v_full[s]);
-              ++jv;
-              iv.next(p, q_last);
-              progress = true;
-            }
-          }
-          if (progress) {
-            idle = 0;
-            continue;
-          }
-          if ((++idle & 255u) == 0u) {
-            if (*reinterpret_cast<volatile int*>(&ctl.abort_flag) != 0) break;
-            const uint64_t now = globaltimer_ns();
-            if (t0 == 0 || idle == 256u) t0 = now;
-            if (now - t0 > CB_MBAR_TIMEOUT_NS) {
-              ctl.abort_flag = 1;
-              report_status(p.status, CB_TIMEOUT_MBARRIER, 0, 0xE00);
-              break;
-            }
-          }
+          g0 += w.nblk;
         }
       }
     } else if (warp == 1) {
-      if (nblk > 0) {
+      {
         // --------------------------------------------------------------------- MMA
         // The whole warp walks the schedule and waits; one elected lane issues.
         constexpr uint32_t idesc_s = make_idesc(128, 128, 1u);
@@ -437,20 +479,23 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
         constexpr uint64_t kTileStep = static_cast<uint64_t>(CP_TILE >> 4);
         constexpr uint64_t kSubStep = static_cast<uint64_t>(CP_SUB >> 4);
         auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t detail) -> bool {
-          const bool w = mbar_wait(bar, parity, &ctl.abort_flag, p.status, detail);
-          return __all_sync(0xffffffffu, w ? 1 : 0) != 0;
+          return mbar_wait_warp(bar, parity, &ctl.abort_flag, p.status, detail);
         };
-        bool ok = wait_all(&ctl.q_full, 0, 0xE10);
+        // A broadcast value is warp-uniform to the compiler: it can live in a uniform register, where
+        // the operands of an MMA have to be.
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        bool ok = true;
+        int g0 = 0, nq = 0;   // blocks and items before this item
         auto issue_qk = [&](int t, int j) -> bool {
-          const int s = j % CP_KST;
-          if (!wait_all(&ctl.k_full[s], (j / CP_KST) & 1, 0xE11)) return false;
+          const int g = g0 + j, s = g % CP_KST;
+          if (!wait_all(&ctl.k_full[s], (g / CP_KST) & 1, 0xE11)) return false;
           tc_fence_after_sync();
           if (elect_one()) {
             const uint64_t qa = q_desc0 + t * kTileStep, ka = k_desc0 + s * kTileStep;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
               const uint64_t off = (kk >> 2) * kSubStep + 2u * (kk & 3);
-              mma_bf16_ss(tmem + 256u * t, qa + off, ka + off, idesc_s, kk > 0 ? 1u : 0u);
+              mma_bf16_ss(tmem_u + 256u * t, qa + off, ka + off, idesc_s, kk > 0 ? 1u : 0u);
             }
             mma_commit(&ctl.s_full[t]);
           }
@@ -458,36 +503,50 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           return true;
         };
         auto issue_pv = [&](int t, int j) -> bool {
-          const int s = j % CP_VST;
-          if (!wait_all(&ctl.p_full[t], j & 1, 0xE20 + t)) return false;
-          if (!wait_all(&ctl.v_full[s], (j / CP_VST) & 1, 0xE22)) return false;
+          // The first product of an item overwrites the O of the last one, which the softmax warps
+          // have read before they hand over the item's first block.
+          const int g = g0 + j, s = g % CP_VST;
+          if (!wait_all(&ctl.p_full[t], g & 1, 0xE20 + t)) return false;
+          if (!wait_all(&ctl.v_full[s], (g / CP_VST) & 1, 0xE22)) return false;
           tc_fence_after_sync();
           if (elect_one()) {
             const uint64_t va = v_desc0 + s * kTileStep;
-            const uint32_t d = tmem + 256u * t + 128u;
+            const uint32_t d = tmem_u + 256u * t + 128u;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-              mma_bf16_ts(d, tmem + 256u * t + 8u * kk, va + kk * (2048u >> 4), idesc_pv,
+              mma_bf16_ts(d, tmem_u + 256u * t + 8u * kk, va + kk * (2048u >> 4), idesc_pv,
                           (j > 0 || kk > 0) ? 1u : 0u);
             mma_commit(&ctl.pv_done[t]);
           }
           __syncwarp();
           return true;
         };
-        for (int t = 0; ok && t < 2; ++t) ok = issue_qk(t, 0);
-        if (ok && elect_one()) mma_commit(&ctl.k_empty[0]);
-        __syncwarp();
-        for (int j = 0; ok && j < nblk; ++j) {
-          for (int t = 0; ok && t < 2; ++t) {
-            ok = issue_pv(t, j);
-            if (ok && j + 1 < nblk) ok = issue_qk(t, j + 1);
-          }
-          if (!ok) break;
-          if (elect_one()) {
-            mma_commit(&ctl.v_empty[j % CP_VST]);
-            if (j + 1 < nblk) mma_commit(&ctl.k_empty[(j + 1) % CP_KST]);
+        CpItem w;
+        for (int i = 0; ok && w.at(p, ticket, i); ++i) {
+          const int nblk = __shfl_sync(0xffffffffu, w.nblk, 0);
+          if (nblk == 0) continue;
+          ok = wait_all(&ctl.q_full, nq & 1, 0xE10);
+          ++nq;
+          for (int t = 0; ok && t < 2; ++t) ok = issue_qk(t, 0);
+          if (ok && elect_one()) {
+            mma_commit(&ctl.k_empty[g0 % CP_KST]);
+            if (nblk == 1) mma_commit(&ctl.q_empty);
           }
           __syncwarp();
+          for (int j = 0; ok && j < nblk; ++j) {
+            for (int t = 0; ok && t < 2; ++t) {
+              ok = issue_pv(t, j);
+              if (ok && j + 1 < nblk) ok = issue_qk(t, j + 1);
+            }
+            if (!ok) break;
+            if (elect_one()) {
+              mma_commit(&ctl.v_empty[(g0 + j) % CP_VST]);
+              if (j + 1 < nblk) mma_commit(&ctl.k_empty[(g0 + j + 1) % CP_KST]);
+              if (j + 2 == nblk) mma_commit(&ctl.q_empty);   // the item's last scores
+            }
+            __syncwarp();
+          }
+          g0 += nblk;
         }
       }
     }
@@ -500,85 +559,88 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
       const uint32_t lane_addr = (q * 32u) << 16;
       const uint32_t tS = tmem + 256u * t + lane_addr;
       const uint32_t tO = tS + 128u;
-      const int row_in_seg = pair * 2 * CP_BM + t * CP_BM + static_cast<int>(r);
-      const int tile_first = q_first + t * CP_BM;     // position of row 0 of this tile
-      const int q_pos = tile_first + static_cast<int>(r);
-      float m_ref = -INFINITY, l = 0.f;
+      CpItem w;
       bool ok = true;
-      CpBlockIter it;
-      it.start(p, q_last);
-      for (int j = 0; ok && j < nblk; ++j) {
-        if (!mbar_wait(&ctl.s_full[t], j & 1, &ctl.abort_flag, p.status, 0xE30 + t)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after_sync();
-        uint32_t s[128];
-        tmem_ld_32x32_at(tS, &s[0]);
-        tmem_ld_32x32_at(tS + 32u, &s[32]);
-        tmem_ld_32x32_at(tS + 64u, &s[64]);
-        tmem_ld_32x32_at(tS + 96u, &s[96]);
-        tmem_wait_ld();
-
-        const CpSeg& g = p.seg[it.seg];
-        const int key0 = g.kpos0 + it.i * CP_BN;
-        const int kv_left = g.nkeys - it.i * CP_BN;
-        const bool need_mask = kv_left < CP_BN || (p.causal && key0 + CP_BN - 1 > tile_first);
-        it.next(p, q_last);
-        if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 128; ++i)
-            if (!(i < kv_left && (!p.causal || key0 + i <= q_pos))) s[i] = 0xff800000u;  // -inf
-        }
-        cp_online_softmax<kPoly>(s, tO, p.scale_log2, need_mask, j > 0, m_ref, l);
-        // P_t(j): row r = lane r, keys 2c and 2c+1 in column c.
-        tmem_st_32x32_at(tS, &s[0]);
-        tmem_st_32x32_at(tS + 32u, &s[32]);
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl.p_full[t]);
-      }
-      // ------------------------------------------------------------------ epilogue
-      if (ok && nblk > 0)
-        ok = mbar_wait(&ctl.pv_done[t], (nblk - 1) & 1, &ctl.abort_flag, p.status, 0xE34 + t);
-      // Tile-uniform condition: the tensor-memory loads below are warp-collective; rows past
-      // the end of the segment are only kept from being stored.
-      if (ok && pair * 2 * CP_BM + t * CP_BM < qs.nrows) {
-        const bool row_ok = row_in_seg < qs.nrows;
-        tc_fence_after_sync();
-        const float inv = l > 0.f ? 1.f / l : 0.f;
-        const int orow = qs.row0 + row_in_seg;
-        __nv_bfloat16* dst =
-            p.o[qs.out] + ((static_cast<size_t>(batch) * p.o_rows[qs.out] + orow) * p.o_heads +
-                           p.o_head0 + head) * CP_D;
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t o[32];
-          if (nblk > 0) {
-            tmem_ld_32x32(tO + c * 32u, o);
-            tmem_wait_ld();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = 0u;
+      int g0 = 0;   // blocks before this item
+      for (int i = 0; ok && w.at(p, ticket, i); ++i) {
+        const CpQSeg& qs = p.qseg[w.qs_i];
+        const int row_in_seg = w.pair * 2 * CP_BM + t * CP_BM + static_cast<int>(r);
+        const int tile_first = w.q_first + t * CP_BM;     // position of row 0 of this tile
+        const int q_pos = tile_first + static_cast<int>(r);
+        float m_ref = -INFINITY, l = 0.f;
+        CpBlockIter it;
+        it.start(p, w.q_last);
+        for (int j = 0; ok && j < w.nblk; ++j) {
+          if (!mbar_wait(&ctl.s_full[t], (g0 + j) & 1, &ctl.abort_flag, p.status, 0xE30 + t)) {
+            ok = false;
+            break;
           }
-          if (row_ok) {
+          tc_fence_after_sync();
+          uint32_t s[128];
+          tmem_ld_32x32_at(tS, &s[0]);
+          tmem_ld_32x32_at(tS + 32u, &s[32]);
+          tmem_ld_32x32_at(tS + 64u, &s[64]);
+          tmem_ld_32x32_at(tS + 96u, &s[96]);
+          tmem_wait_ld();
+
+          const CpSeg& g = p.seg[it.seg];
+          const int key0 = g.kpos0 + it.i * CP_BN;
+          const int kv_left = g.nkeys - it.i * CP_BN;
+          const bool need_mask = kv_left < CP_BN || (p.causal && key0 + CP_BN - 1 > tile_first);
+          it.next(p, w.q_last);
+          if (need_mask) cp_mask_tail(s, p.causal ? min(kv_left, q_pos - key0 + 1) : kv_left);
+          cp_online_softmax<kPoly>(s, tO, p.scale_log2, need_mask, j > 0, m_ref, l);
+          // P_t(j): row r = lane r, keys 2c and 2c+1 in column c.
+          tmem_st_32x32_at(tS, &s[0]);
+          tmem_st_32x32_at(tS + 32u, &s[32]);
+          tmem_wait_st();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.p_full[t]);
+        }
+        // ------------------------------------------------------------------ epilogue
+        if (ok && w.nblk > 0)
+          ok = mbar_wait(&ctl.pv_done[t], (g0 + w.nblk - 1) & 1, &ctl.abort_flag, p.status, 0xE34 + t);
+        // Tile-uniform condition: the tensor-memory loads below are warp-collective; rows past
+        // the end of the segment are only kept from being stored.
+        if (ok && w.pair * 2 * CP_BM + t * CP_BM < qs.nrows) {
+          const bool row_ok = row_in_seg < qs.nrows;
+          tc_fence_after_sync();
+          const float inv = l > 0.f ? 1.f / l : 0.f;
+          const int orow = qs.row0 + row_in_seg;
+          __nv_bfloat16* dst =
+              p.o[qs.out] + ((static_cast<size_t>(w.batch) * p.o_rows[qs.out] + orow) * p.o_heads +
+                             p.o_head0 + w.head) * CP_D;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            if (w.nblk > 0) {
+              tmem_ld_32x32(tO + c * 32u, o);
+              tmem_wait_ld();
+            } else {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 v;
-              __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&v);
+              for (int i = 0; i < 32; ++i) o[i] = 0u;
+            }
+            if (row_ok) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                hh[k] = __floats2bfloat162_rn(__uint_as_float(o[i + 2 * k]) * inv,
-                                              __uint_as_float(o[i + 2 * k + 1]) * inv);
-              *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
+              for (int i = 0; i < 32; i += 8) {
+                uint4 v;
+                __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  hh[k] = __floats2bfloat162_rn(__uint_as_float(o[i + 2 * k]) * inv,
+                                                __uint_as_float(o[i + 2 * k + 1]) * inv);
+                *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
+              }
             }
           }
+          if (row_ok && p.lse[qs.out] != nullptr)
+            p.lse[qs.out][(static_cast<size_t>(w.batch) * p.o_heads + p.o_head0 + w.head) *
+                              p.o_rows[qs.out] + orow] =
+                l > 0.f ? (m_ref * 0.6931471805599453f + logf(l)) : -INFINITY;
         }
-        if (row_ok && p.lse[qs.out] != nullptr)
-          p.lse[qs.out][(static_cast<size_t>(batch) * p.o_heads + p.o_head0 + head) *
-                            p.o_rows[qs.out] + orow] =
-              l > 0.f ? (m_ref * 0.6931471805599453f + logf(l)) : -INFINITY;
+        tc_fence_before_sync();   // O has been read: the hand-over of the next item's first block says so
+        g0 += w.nblk;
       }
     }
     __syncwarp();

@@ -241,8 +241,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
       constexpr uint64_t kTileStep = static_cast<uint64_t>(CP_TILE >> 4);
       constexpr uint64_t kSubStep = static_cast<uint64_t>(CP_SUB >> 4);
       auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t detail) -> bool {
-        const bool w = mbar_wait(bar, parity, &ctl.abort_flag, p.status, detail);
-        return __all_sync(0xffffffffu, w ? 1 : 0) != 0;
+        return mbar_wait_warp(bar, parity, &ctl.abort_flag, p.status, detail);
       };
       int g0 = 0;                 // blocks before this segment
       uint32_t pv_count[2] = {0u, 0u};
@@ -336,11 +335,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
         const int key0 = pl.kv_offset + kb;
         const int kv_left = pl.Skv - kb;
         const bool need_mask = kv_left < CP_BN || (pl.causal && key0 + CP_BN - 1 > tile_first);
-        if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 128; ++i)
-            if (!(i < kv_left && (!pl.causal || key0 + i <= q_pos))) s[i] = 0xff800000u;  // -inf
-        }
+        if (need_mask) cp_mask_tail(s, pl.causal ? min(kv_left, q_pos - key0 + 1) : kv_left);
         cp_online_softmax<0>(s, tO, p.scale_log2, need_mask, j > 1, m_ref, l);
         tmem_st_32x32_at(tS, &s[0]);
         tmem_st_32x32_at(tS + 32u, &s[32]);
@@ -604,11 +599,11 @@ static int split_sms() {
 // kPairBlock for a key block of its 256 rows and is as long as its longest item or its share of all
 // of them; the split kernel takes SP_BLOCK_US for a unit of its 128 rows, plus the merge.
 // Measured, split / pair (B, Sq, Skv, Hq, Hkv): (1, 64, 64, 4, 4) 7.6 / 9.0 us, (1, 300, 300, 4, 1)
-// 11 / 14, (1, 500, 4596, 8, 2) 23 / 81, (1, 8192, 8192, 4, 4) 94 / 138; near the line
-// (2, 1000, 1000, 8, 8) 26 / 27, (1, 2000, 2777, 16, 4) 57 / 55, (1, 1000, 7000, 32, 8) 125 / 122; beyond
-// it (2, 2000, 2000, 32, 8) 131 / 105.
+// 11 / 14, (1, 500, 4596, 8, 2) 23 / 81, (1, 8192, 8192, 4, 4) 90 / 127; near the line
+// (1, 1280, 1280, 16, 8) 33 / 30, (1, 2000, 2777, 16, 4) 54 / 51, (1, 1000, 7000, 32, 8) 118 / 112;
+// beyond it (2, 2000, 2000, 32, 8) 125 / 88.
 static bool split_wins(const SplitPlan& pl, int sms) {
-  constexpr float kPairBlock = 2.2f, kPairStart = 7.f, kStart = 6.f;
+  constexpr float kPairBlock = 2.0f, kPairStart = 7.f, kStart = 6.f;
   const float pair_tiles = static_cast<float>((pl.Sq + 2 * CP_BM - 1) / (2 * CP_BM));
   float blocks = 0.f;
   for (int i = 0; i < pl.nqt; ++i) blocks += static_cast<float>(pl.nblk[i]);

@@ -182,7 +182,8 @@ int cb_ring_attn(const CbRingAttnDesc* dp, void* stream) {
   p.flags = static_cast<uint32_t*>(d.flags);
   // every counter gets one increment per communication CTA for each of its 2 B pieces (K and V)
   p.flag_target = (d.calls + 1u) * static_cast<uint32_t>(2 * d.B * p.num_comm);
-  p.sched = static_cast<uint32_t*>(d.sched);
+  // tickets only where communication CTAs must be the first to run
+  p.sched = p.num_comm > 0 ? static_cast<uint32_t*>(d.sched) : nullptr;
   p.status = static_cast<uint32_t*>(d.status);
   p.timeout_ns = d.timeout_ns;
   if (d.write_plan && !copies.empty()) {

@@ -139,33 +139,17 @@ struct GemmShape {
   unsigned long long* trace = nullptr;
 };
 
-// Warp-collective mbar_wait: every lane of a converged warp calls it and all of them get the
-// same answer (a lane that saw the barrier flip at the last moment must not go on alone to a
-// `.sync.aligned` instruction or an election while its neighbours give up).  The usual case is one
-// try and one vote; the loop with its time limit is the slow path.  With tracing on (a lane may
-// trace while its neighbours do not, so nothing collective depends on it), the waiting time is
-// added to `*acc_cycles`.
+// mbar_wait_warp whose waiting time is added to `*acc_cycles` with tracing on (a lane may trace while
+// its neighbours do not, so nothing collective depends on it).
 __device__ __forceinline__ bool mbar_wait_traced(uint64_t* bar, uint32_t parity,
                                                  volatile int* abort_flag, uint32_t* status,
                                                  uint32_t detail, bool tracing,
                                                  long long* acc_cycles) {
   // The whole call is timed: a try_wait may itself block for a while before it answers.
   const long long t0 = tracing ? clock64() : 0;
-  bool ok = __all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) != 0;
-  if (!ok)
-    ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, detail) ? 1 : 0) != 0;
+  const bool ok = mbar_wait_warp(bar, parity, abort_flag, status, detail);
   if (tracing) *acc_cycles += clock64() - t0;
   return ok;
-}
-
-// Two barriers that an issuing warp needs together: one vote when both are ready at the first try.
-__device__ __forceinline__ bool mbar_wait_both(uint64_t* bar0, uint32_t parity0, uint32_t detail0,
-                                               uint64_t* bar1, uint32_t parity1, uint32_t detail1,
-                                               volatile int* abort_flag, uint32_t* status) {
-  const bool r0 = mbar_try_wait(bar0, parity0), r1 = mbar_try_wait(bar1, parity1);
-  if (__all_sync(0xffffffffu, (r0 && r1) ? 1 : 0) != 0) return true;
-  return mbar_wait_traced(bar0, parity0, abort_flag, status, detail0, false, nullptr) &&
-         mbar_wait_traced(bar1, parity1, abort_flag, status, detail1, false, nullptr);
 }
 
 // Grouped rasterisation: consecutive tiles share a panel of up to `group` row

@@ -77,4 +77,25 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// Warp-collective form: every lane of a converged warp calls it and all of them get the same answer
+// (a lane that saw the barrier flip at the last moment must not go on alone to a `.sync.aligned`
+// instruction or an election while its neighbours give up).  The usual case is one try and one
+// vote; the loop with its limits is the slow path.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
+                                               volatile int* abort_flag, uint32_t* status,
+                                               uint32_t detail) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) != 0) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, detail) ? 1 : 0) != 0;
+}
+
+// Two barriers that a warp needs together: one vote when both are ready at the first try.
+__device__ __forceinline__ bool mbar_wait_both(uint64_t* bar0, uint32_t parity0, uint32_t detail0,
+                                               uint64_t* bar1, uint32_t parity1, uint32_t detail1,
+                                               volatile int* abort_flag, uint32_t* status) {
+  const bool r0 = mbar_try_wait(bar0, parity0), r1 = mbar_try_wait(bar1, parity1);
+  if (__all_sync(0xffffffffu, (r0 && r1) ? 1 : 0) != 0) return true;
+  return mbar_wait_warp(bar0, parity0, abort_flag, status, detail0) &&
+         mbar_wait_warp(bar1, parity1, abort_flag, status, detail1);
+}
+
 }  // namespace cb

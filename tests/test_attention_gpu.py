@@ -197,3 +197,30 @@ def test_split_and_pair_kernels_agree_on_the_public_call(native_lib):
                            0, 1, C.c_float(0.1), N.ptr(o), C.c_longlong(16), C.c_void_p(0),
                            N.stream_ptr())
     assert rc != 0 and "workspace" in N.last_error()
+
+
+@pytest.mark.parametrize("causal,kv_offset", [(False, 0), (True, 0), (True, 400)])
+def test_persistent_tile_pairs(native_lib, causal, kv_offset):
+    """More tile pairs than SMs, so a CTA walks several of different lengths: ragged rows and keys, and
+    with kv_offset whole pairs that see no key (zero rows, lse -inf) between ones that do.
+    Bounds as for the split-key kernel."""
+    import ctypes as C
+    import math
+
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.cp import reference_attention
+
+    B, Sq, Skv, Hq, Hkv = 2, 700, 300, 64, 4
+    q, k, v = _qkv(B, Sq, Skv, Hq, Hkv, 41)
+    o, lse = torch.empty_like(q), torch.empty(B, Hq, Sq, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    rc = N.load().cb_attn_fwd4(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(o), N.ptr(lse), B, Sq, Skv, Hq, Hkv,
+                               0, kv_offset, int(causal), C.c_float(1.0 / math.sqrt(128)),
+                               N.ptr(status), N.stream_ptr())
+    assert rc == 0, N.last_error()
+    ro, rl = reference_attention(q, k, v, causal=causal, kv_offset=kv_offset)
+    assert int(status.abs().sum()) == 0
+    assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
+    seen = rl > float("-inf")
+    assert torch.equal(lse > float("-inf"), seen)
+    assert (lse - rl)[seen].abs().max() < 1e-4
