@@ -104,12 +104,14 @@ __device__ __forceinline__ void cp_mask_tail(uint32_t (&s)[128], int visible) {
 // One block of the online softmax: the 128 masked scores of this thread's row in `s` become the
 // bf16 probabilities s[0..63]; m_ref (log2 units) and l are the running reference maximum and sum.
 // The accumulator in tensor memory at `tO` is rescaled when the maximum has grown by more than
-// CP_RESCALE_THRESHOLD in any row of the warp (`rescale_o`: it holds something already).
+// CP_RESCALE_THRESHOLD in any row of the warp that `votes` (`rescale_o`: it holds something already).
+// A row that was not loaded must not vote: its scores come from whatever was in shared memory, and when
+// the other rows are rescaled decides how they are rounded.
 // kPoly: see fa_cp_kernel.  Warp-collective.
 template <int kPoly>
 __device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t tO, float scale_log2,
-                                                  bool need_mask, bool rescale_o, float& m_ref,
-                                                  float& l) {
+                                                  bool need_mask, bool rescale_o, bool votes,
+                                                  float& m_ref, float& l) {
   float mx8[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
@@ -122,8 +124,8 @@ __device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t t
       cp_max3(fmaxf(cp_max3(mx8[0], mx8[1], mx8[2]), cp_max3(mx8[3], mx8[4], mx8[5])),
               mx8[6], mx8[7]);
   const float mx_s = mx_all * scale_log2;
-  const bool grow =
-      mx_s > m_ref + CP_RESCALE_THRESHOLD || (m_ref == -INFINITY && mx_s > -INFINITY);
+  const bool grow = votes && (mx_s > m_ref + CP_RESCALE_THRESHOLD ||
+                              (m_ref == -INFINITY && mx_s > -INFINITY));
   const bool any_grow = __any_sync(0xffffffffu, grow);
   if (any_grow) {
     const float m_new = fmaxf(m_ref, mx_s);
@@ -589,7 +591,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           const bool need_mask = kv_left < CP_BN || (p.causal && key0 + CP_BN - 1 > tile_first);
           it.next(p, w.q_last);
           if (need_mask) cp_mask_tail(s, p.causal ? min(kv_left, q_pos - key0 + 1) : kv_left);
-          cp_online_softmax<kPoly>(s, tO, p.scale_log2, need_mask, j > 0, m_ref, l);
+          cp_online_softmax<kPoly>(s, tO, p.scale_log2, need_mask, j > 0, true, m_ref, l);
           // P_t(j): row r = lane r, keys 2c and 2c+1 in column c.
           tmem_st_32x32_at(tS, &s[0]);
           tmem_st_32x32_at(tS + 32u, &s[32]);

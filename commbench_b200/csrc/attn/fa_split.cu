@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
         const int kv_left = pl.Skv - kb;
         const bool need_mask = kv_left < CP_BN || (pl.causal && key0 + CP_BN - 1 > tile_first);
         if (need_mask) cp_mask_tail(s, pl.causal ? min(kv_left, q_pos - key0 + 1) : kv_left);
-        cp_online_softmax<0>(s, tO, p.scale_log2, need_mask, j > 1, m_ref, l);
+        cp_online_softmax<0>(s, tO, p.scale_log2, need_mask, j > 1, r < tile_rows, m_ref, l);
         tmem_st_32x32_at(tS, &s[0]);
         tmem_st_32x32_at(tS + 32u, &s[32]);
         tmem_wait_st();

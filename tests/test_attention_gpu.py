@@ -224,3 +224,22 @@ def test_persistent_tile_pairs(native_lib, causal, kv_offset):
     seen = rl > float("-inf")
     assert torch.equal(lse > float("-inf"), seen)
     assert (lse - rl)[seen].abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 2000, 1, 1), (4, 1, 3000, 16, 4), (2, 4, 5000, 32, 8),
+                                   (2, 5, 700, 6, 2)])
+def test_split_key_attention_repeats_its_bits(native_lib, shape):
+    """Tiles with fewer than 128 rows: what other kernels leave in shared memory where rows are missing
+    must not show in the result."""
+    from commbench_b200.ops.cp import flash_attention
+
+    B, Sq, Skv, Hq, Hkv = shape
+    q, k, v = _qkv(B, Sq, Skv, Hq, Hkv, 23)
+    # a full tile of queries with large scores, of another size each time
+    others = [_qkv(8, 128, 2048, 8, 8, 29 + i) for i in range(4)]
+    ref = flash_attention(q, k, v, q_offset=Skv - Sq)
+    for i in range(12):
+        qn, kn, vn = others[i % 4]
+        flash_attention(qn * float(1 + i), kn, vn, causal=False)
+        o, lse = flash_attention(q, k, v, q_offset=Skv - Sq)
+        assert torch.equal(o, ref[0]) and torch.equal(lse, ref[1]), i
