@@ -36,15 +36,13 @@ def _split_attention(q, k, v, out, lse, causal, q_offset, kv_offset, sc, status_
     nbytes = lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, q_offset, kv_offset, int(causal))
     if nbytes < 0:
         return False
-    ws = 0
+    ws = None
     if nbytes > 0:
-        buf = q.new_empty((nbytes,), dtype=torch.uint8)
-        if stream is not None:
-            buf.record_stream(stream)
-        ws = buf.data_ptr()
+        ws = N.new_empty(q, (nbytes,), torch.uint8, stream, handed_out=False)
     rc = lib.cb_attn_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                            lse.data_ptr() if lse is not None else 0, B, Sq, Skv, Hq, Hkv, q_offset,
-                           kv_offset, int(causal), sc, ws, nbytes, status_ptr, N.raw_stream(stream))
+                           kv_offset, int(causal), sc, ws.data_ptr() if ws is not None else 0, nbytes,
+                           status_ptr, N.raw_stream(stream))
     if rc != 0:
         raise CommError(f"attention launch failed: {N.last_error()}")
     return True
@@ -73,9 +71,9 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: 
     if v.shape != k.shape or k.shape[0] != B:
         raise CommError("k and v must have the same shape and q's batch size")
     if out is None:
-        out = torch.empty_like(q)
+        out = N.new_empty(q, q.shape, stream=stream)
     if lse is None:
-        lse = q.new_empty((B, Hq, Sq), dtype=torch.float32)
+        lse = N.new_empty(q, (B, Hq, Sq), torch.float32, stream)
     sc = scale if scale is not None else 1.0 / math.sqrt(D)
     if impl is None:
         impl = get_config().attn_impl
@@ -145,6 +143,13 @@ class _UlyssesDesc(C.Structure):
     ]
 
 
+def _tensors(x):
+    """The CUDA tensors of nested lists and tuples."""
+    if isinstance(x, (list, tuple)):
+        return [t for y in x for t in _tensors(y)]
+    return [x] if isinstance(x, torch.Tensor) and x.is_cuda else []
+
+
 class _CpBase:
     """State shared by the two context-parallel attention ops: symmetric buffers seen the same
     way for real ranks and for virtual ranks on one GPU, the local counters of the kernel and
@@ -181,6 +186,21 @@ class _CpBase:
 
     def _status_ptr(self, i):
         return self.ctx.comms[i].status if self.emu else self.ctx.comm.status
+
+    def _run(self, stream, inputs, fn, *args):
+        """``fn(*args)`` with ``stream`` (None: as it is) as the current stream, so that a call's input
+        copies, barriers, allocations and launches are ordered among themselves; inputs and results
+        are recorded on both streams."""
+        if stream is None:
+            return fn(*args)
+        caller = torch.cuda.current_stream(self.ctx.device)
+        for t in _tensors(inputs):
+            t.record_stream(stream)
+        with torch.cuda.stream(stream):
+            res = fn(*args)
+        for t in _tensors(res):
+            t.record_stream(caller)
+        return res
 
     def _barrier(self):
         # Real ranks: a cross-GPU barrier kernel on the stream.  Virtual ranks run one after
@@ -232,7 +252,7 @@ class RingAttention(_CpBase):
     def v_local(self, i: int = 0) -> torch.Tensor:
         return self._v_own[i]
 
-    def _launch(self, i, r, q, o, lse, causal, scale, stream):
+    def _launch(self, i, r, q, o, lse, causal, scale):
         d = _RingDesc()
         d.rank, d.world, d.B, d.s_local, d.hq, d.hkv = r, self.W, self.B, self.Sl, self.Hq, self.Hkv
         d.causal, d.zigzag, d.num_comm, d.scale = int(causal), int(self.zigzag), self.num_comm, scale
@@ -243,14 +263,19 @@ class RingAttention(_CpBase):
         d.calls = self.calls
         d.write_plan = int(self._plan_key != (bool(causal),))
         d.status, d.timeout_ns = self._status_ptr(i), self.ctx.timeout_ns
-        if self.lib.cb_ring_attn(C.byref(d), N.stream_ptr(stream)) != 0:
+        if self.lib.cb_ring_attn(C.byref(d), N.stream_ptr()) != 0:
             raise CommError(f"ring attention failed: {N.last_error()}")
 
     @traced("cb200.ring_attention")
     def forward(self, q, k, v, causal: bool = True, out=None, want_lse: bool = True,
                 scale: float | None = None, stream=None):
         """``q`` [B, S_local, Hq, 128], ``k`` / ``v`` [B, S_local, Hkv, 128] bf16 (lists with one
-        entry per virtual rank under an ``EmuContext``).  Returns ``(o, lse)``."""
+        entry per virtual rank under an ``EmuContext``).  Returns ``(o, lse)``.
+
+        With ``stream`` the whole call runs there, the copy of ``k`` / ``v`` into their slot included."""
+        return self._run(stream, (q, k, v), self._forward, q, k, v, causal, out, want_lse, scale)
+
+    def _forward(self, q, k, v, causal, out, want_lse, scale):
         qs, ks, vs = (q, k, v) if self.emu else ([q], [k], [v])
         sc = scale if scale is not None else 1.0 / math.sqrt(128)
         outs, lses = [], []
@@ -277,8 +302,8 @@ class RingAttention(_CpBase):
             lse = qi.new_empty((self.B, self.Hq, self.Sl), dtype=torch.float32) if want_lse else None
             # one rank: a plain local attention over its own slot
             if self.W > 1 or not _split_attention(qi, self._k_own[i], self._v_own[i], o, lse,
-                                                  causal, 0, 0, sc, self._status_ptr(i), stream):
-                self._launch(i, r, qi, o, lse, causal, sc, stream)
+                                                  causal, 0, 0, sc, self._status_ptr(i), None):
+                self._launch(i, r, qi, o, lse, causal, sc)
             outs.append(o)
             lses.append(lse)
         self._barrier()                       # nobody overwrites a shard that is still being read
@@ -332,7 +357,7 @@ class UlyssesAttention(_CpBase):
         if not self.emu:
             ctx.host_barrier()
 
-    def _launch(self, i, r, causal, scale, stream):
+    def _launch(self, i, r, causal, scale):
         d = _UlyssesDesc()
         d.rank, d.world, d.B, d.s_local, d.hq, d.hkv = r, self.W, self.B, self.Sl, self.Hq, self.Hkv
         d.causal, d.num_comm, d.pieces, d.scale = int(causal), self.num_comm, self.pieces, scale
@@ -348,14 +373,19 @@ class UlyssesAttention(_CpBase):
         d.calls = self.calls
         d.write_plan = int(self._plan_key is None)
         d.status, d.timeout_ns = self._status_ptr(i), self.ctx.timeout_ns
-        if self.lib.cb_ulysses_attn(C.byref(d), N.stream_ptr(stream)) != 0:
+        if self.lib.cb_ulysses_attn(C.byref(d), N.stream_ptr()) != 0:
             raise CommError(f"Ulysses attention failed: {N.last_error()}")
 
     @traced("cb200.ulysses_attention")
     def forward(self, q=None, k=None, v=None, causal: bool = True, scale: float | None = None,
                 stream=None):
         """Inputs that are not the op's own symmetric buffers are copied in; ``None`` means
-        "already there".  Returns this rank's ``o_buf`` (valid until the next call)."""
+        "already there".  Returns this rank's ``o_buf`` (valid until the next call).
+
+        With ``stream`` the whole call runs there, the input copies included."""
+        return self._run(stream, (q, k, v), self._forward, q, k, v, causal, scale)
+
+    def _forward(self, q, k, v, causal, scale):
         sc = scale if scale is not None else 1.0 / math.sqrt(128)
         for name, src, bufs in (("q", q, self.q_buf), ("k", k, self.k_buf), ("v", v, self.v_buf)):
             if src is None:
@@ -366,7 +396,7 @@ class UlyssesAttention(_CpBase):
                     bufs[i].copy_(srcs[i])
         self._barrier()                       # inputs of every rank are in place
         for i, r in enumerate(self._ranks()):
-            self._launch(i, r, causal, sc, stream)
+            self._launch(i, r, causal, sc)
         self._barrier()                       # every owner has all its output rows
         self._plan_key = True
         self.calls += 1

@@ -243,3 +243,57 @@ def test_split_key_attention_repeats_its_bits(native_lib, shape):
         flash_attention(qn * float(1 + i), kn, vn, causal=False)
         o, lse = flash_attention(q, k, v, q_offset=Skv - Sq)
         assert torch.equal(o, ref[0]) and torch.equal(lse, ref[1]), i
+
+
+@pytest.mark.parametrize("given", [True, False])
+def test_call_on_a_side_stream_leaves_blocks_of_the_current_stream_alone(native_lib, given):
+    """A block that the current stream has freed but still has a copy queued from is not handed to a
+    call that runs on another stream, neither as its workspace nor as a result made inside."""
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.cp import flash_attention
+
+    B, Skv, Hq, Hkv = 4, 3000, 16, 4
+    q, k, v = _qkv(B, 1, Skv, Hq, Hkv, 19)
+    ref_o, ref_l = flash_attention(q, k, v, q_offset=Skv - 1)
+    sizes = [N.load().cb_attn_split_bytes(B, 1, Skv, Hq, Hkv, Skv - 1, 0, 1), ref_o.numel() * 2,
+             ref_l.numel() * 4]
+    assert min(sizes) > 0
+    out, lse = (torch.empty_like(ref_o), torch.empty_like(ref_l)) if given else (None, None)
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        blocks = [torch.full((n,), 0x5a, dtype=torch.uint8, device="cuda") for n in sizes]
+        kept = [torch.empty_like(b) for b in blocks]
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)                 # about 10 ms: the copies stay queued behind it
+        for a, b in zip(kept, blocks):
+            a.copy_(b)
+        del a, b, blocks
+        o, l = flash_attention(q, k, v, q_offset=Skv - 1, out=out, lse=lse, stream=side)
+        torch.cuda.synchronize()
+        assert all(bool((x == 0x5a).all()) for x in kept)
+        assert torch.equal(o, ref_o) and torch.equal(l, ref_l)
+
+
+@pytest.mark.parametrize("op", ["ring", "ulysses"])
+def test_context_parallel_call_runs_wholly_on_its_stream(native_lib, op):
+    """Inputs outside the op's own buffers, with the current stream busy: copies and launch follow
+    each other on the given stream and read what that stream was given to wait for."""
+    from commbench_b200.ops.cp import RingAttention, UlyssesAttention, reference_attention
+    from commbench_b200.runtime.context import CommContext
+
+    ctx = CommContext(heap_bytes=64 << 20)
+    attn = (RingAttention if op == "ring" else UlyssesAttention)(ctx, 1, 512, 4, 1)
+    side = torch.cuda.Stream()
+    for seed in (5, 6):
+        q, k, v = _qkv(1, 512, 512, 4, 1, seed)
+        ro, _ = reference_attention(q, k, v)
+        side.wait_stream(torch.cuda.current_stream())
+        torch.cuda._sleep(20_000_000)
+        o = attn.forward(q, k, v, stream=side)
+        o = o[0] if op == "ring" else o
+        side.synchronize()                            # the current stream is still asleep
+        with torch.cuda.stream(side):
+            assert torch.allclose(o.float(), ro, atol=2e-2, rtol=2e-2)
+        torch.cuda.synchronize()
+    ctx.check_status()
+    ctx.close()
