@@ -293,3 +293,34 @@ def test_role_trace_runs_with_one_tracing_lane(native_lib, bn):
     r = gemm_role_trace(a, b, bn)
     assert r["mma_cycles"] > 0
     assert all(0.0 <= v <= 1.0 for k, v in r.items() if k != "mma_cycles"), r
+
+
+@pytest.mark.parametrize("path", ["bf16", "mx", "blockscaled"])
+def test_gemm_on_a_side_stream_leaves_blocks_of_the_current_stream_alone(native_lib, path):
+    """A result made inside a call that is given a stream does not take a block that the current stream
+    has freed but still has a copy queued from."""
+    from commbench_b200.ops.gemm import (gemm, gemm_fp8_blockscaled, gemm_fp8_mx, quantize_blockscaled,
+                                         quantize_blockscaled_pow2)
+
+    a = torch.randn(512, 1024, device="cuda").bfloat16()
+    b = torch.randn(2048, 1024, device="cuda").bfloat16()
+    if path == "bf16":
+        run = lambda **kw: gemm(a, b, **kw)
+    elif path == "mx":
+        (aq, _, asf), (bq, _, bsf) = quantize_blockscaled_pow2(a, 1), quantize_blockscaled_pow2(b, 128)
+        run = lambda **kw: gemm_fp8_mx(aq, asf, bq, bsf, **kw)
+    else:
+        (aq, as_), (bq, bs) = quantize_blockscaled(a, 1), quantize_blockscaled(b, 128)
+        run = lambda **kw: gemm_fp8_blockscaled(aq, as_, bq, bs, **kw)
+    ref = run()
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        block = torch.full((ref.numel() * 2,), 0x5a, dtype=torch.uint8, device="cuda")
+        kept = torch.empty_like(block)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)                 # about 10 ms: the copy stays queued behind it
+        kept.copy_(block)
+        del block
+        out = run(stream=side)
+        torch.cuda.synchronize()
+        assert bool((kept == 0x5a).all()) and torch.equal(out, ref)
