@@ -47,8 +47,8 @@ struct MoeSendArgs {
 
 // Token-major dispatch: a warp loads up to 1024 columns of a token ONCE, quantises them ONCE
 // (per-128-channel absmax -> scale -> e4m3) and writes them to every row that the token's K
-// selections have; all slices of a token belong to one CTA, which releases once at the end and then
-// bumps the arrival counter of every expert it wrote rows for.
+// selections have; all slices of a token belong to one CTA, which at its end bumps the arrival counter
+// of every expert it wrote rows for.
 //
 // Rows for another rank go there as fp8 plus scales.  Rows for an expert of THIS rank never take
 // the fp8 detour through memory: the quantised values, expanded to bf16 exactly as the receive
@@ -171,13 +171,12 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
-  // One release of everything this CTA wrote, then the counters.
-  __syncthreads();
-  if (threadIdx.x == 0) fence_acq_rel_sys();
+  // Every counter update is a release of its own: it covers what the whole CTA wrote before the
+  // barrier, but only for the thread that makes it - a fence of another thread would not.
   __syncthreads();
   for (int e = threadIdx.x; e < a.E; e += blockDim.x)
     if (sent[e] > 0)
-      red_relaxed_sys_add(a.arrived[e / El] + e % El, static_cast<uint32_t>(sent[e]));
+      red_release_sys_add(a.arrived[e / El] + e % El, static_cast<uint32_t>(sent[e]));
 }
 
 struct MoeRecvArgs {

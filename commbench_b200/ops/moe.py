@@ -264,7 +264,7 @@ class MoELayer:
             a.recv_meta, a.arrived = _P8(*self.recv_meta.ptrs), _P8(*self.arrived.ptrs)
             a.rank, a.world, a.T, a.K, a.H, a.E, a.max_rows = st.r, W, T, K, H, E, self.max_rows
             a.status, a.per_token = self._status(st), int(self.per_token)
-            # four CTAs per SM at most: each releases its rows and bumps the counters once
+            # four CTAs per SM at most: each bumps the counters once, when its rows are written
             N.check(lib.cb_moe_dispatch_send(C.byref(a), 4 * self.sms, sp), "cb_moe_dispatch_send")
         self._mark("dispatch_send")
         # 5. receive: wait per expert, dequantise other ranks' rows to bf16, mark padding rows

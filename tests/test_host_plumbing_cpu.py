@@ -251,3 +251,16 @@ def test_dispatch_rows_per_pair_and_per_token():
     pair, tok = dispatch_rows(big, 256, 8, False), dispatch_rows(big, 256, 8, True)
     assert sum(pair) == 512 * 8 and all(t <= p for t, p in zip(tok, pair))
     assert 0.55 < sum(tok) / sum(pair) < 0.75        # 8 * (1 - (7/8)^8) / 8 = 0.66 expected
+
+
+def test_dispatch_counter_updates_are_releases_of_their_own():
+    """The arrival counters of the expert dispatch are bumped by many threads of a CTA.  A release is the
+    fence and the update of ONE thread, so a relaxed update would not publish the rows; on one GPU no
+    run can tell, so the source is looked at."""
+    import re
+
+    csrc = os.path.join(os.path.dirname(HERE), "commbench_b200", "csrc", "moe", "moe_dispatch.cu")
+    with open(csrc) as f:
+        code = re.sub(r"//[^\n]*", "", f.read())
+    updates = re.findall(r"\b(\w+)\(a\.arrived\[", code)
+    assert updates and set(updates) == {"red_release_sys_add"}
