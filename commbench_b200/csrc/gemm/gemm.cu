@@ -162,7 +162,10 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
   if (tiles * Cfg::PAIR < ctas) ctas = tiles * Cfg::PAIR;
   ctas -= ctas % Cfg::PAIR;
-  if (ctas < Cfg::PAIR) return 0;
+  if (ctas < Cfg::PAIR) {
+    set_last_error("gemm: a tile of a CTA pair needs a limit of at least two CTAs");
+    return -1;
+  }
   cudaError_t e = launch_gemm_kernel(gemm_plain_kernel<Cfg>, ctas, Cfg::THREADS, Cfg::SMEM_BYTES,
                                      st, Cfg::PAIR, false, p);
   if (e != cudaSuccess) {
@@ -229,11 +232,12 @@ static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
   return best;
 }
 
-// Tile of the persistent kernels for a caller that limits the CTAs: pairs on 256 x 256 tiles when
-// there are plenty of them, narrower tiles for skinny problems.
-static int persistent_tile(int M, int N) {
+// Tile of the persistent kernels for a caller that limits the CTAs to `max_ctas`: pairs on 256 x 256
+// tiles when there are plenty of them (and the limit admits a pair), narrower tiles for skinny
+// problems.
+static int persistent_tile(int M, int N, int max_ctas) {
   const long long m_blocks = (M + 127) / 128;
-  if (static_cast<long long>((M + 255) / 256) * ((N + 255) / 256) * 2 >= sm_count()) return 512;
+  if (max_ctas >= 2 && static_cast<long long>((M + 255) / 256) * ((N + 255) / 256) * 2 >= sm_count()) return 512;
   if (m_blocks * ((N + 255) / 256) >= sm_count()) return 256;
   if (m_blocks * ((N + 127) / 128) >= sm_count()) return 128;
   return 64;
@@ -324,7 +328,7 @@ int cb_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, flo
     const GemmChoice g = choose_gemm(M, N, 2ll * K, sm_count());
     if (g.split > 0 && max_ctas <= 0)
       return run_small_bn<false>(a, b, c, M, N, K, alpha, g.bn, g.split, s, st);
-    bn = g.split > 0 ? persistent_tile(M, N) : g.bn;
+    bn = g.split > 0 || max_ctas == 1 ? persistent_tile(M, N, max_ctas) : g.bn;
   }
   switch (bn) {
     case 512:
@@ -393,7 +397,7 @@ int cb_gemm_fp8(const void* a, const void* b, void* c, int M, int N, int K, floa
     const GemmChoice g = choose_gemm(M, N, K, sm_count());
     if (g.split > 0 && max_ctas <= 0)
       return run_small_bn<true>(a, b, c, M, N, K, alpha, g.bn, g.split, s, st);
-    bn = g.split > 0 ? persistent_tile(M, N) : g.bn;
+    bn = g.split > 0 || max_ctas == 1 ? persistent_tile(M, N, max_ctas) : g.bn;
   }
   switch (bn) {
     case 512:

@@ -324,3 +324,29 @@ def test_gemm_on_a_side_stream_leaves_blocks_of_the_current_stream_alone(native_
         out = run(stream=side)
         torch.cuda.synchronize()
         assert bool((kept == 0x5a).all()) and torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("max_ctas", [1, 2, 3])
+def test_gemm_with_a_limit_of_few_ctas(native_lib, max_ctas, fp8):
+    """A limit below a CTA pair: a shape for which the size rule picks pairs runs on single CTAs, and an
+    explicit pair tile is refused instead of leaving the result unwritten.  bf16 rounding, 2-norm
+    3e-3."""
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.gemm import GemmError, gemm
+
+    M, Nn, K = 3000, 2568, 1040
+    assert N.load().cb_gemm_choice(M, Nn, K, int(fp8)) == 512
+    g = torch.Generator(device="cuda").manual_seed(17)
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    b = torch.randn(Nn, K, device="cuda", generator=g).bfloat16()
+    if fp8:
+        a, b = a.to(torch.float8_e4m3fn), b.to(torch.float8_e4m3fn)
+    ref = _ref(a, b)
+    for bn in (0, 256, 128, 64) + ((512,) if max_ctas > 1 else ()):
+        out = torch.full((M, Nn), float("nan"), device="cuda", dtype=torch.bfloat16)
+        gemm(a, b, out=out, bn=bn, max_ctas=max_ctas)
+        assert (out.float() - ref).norm() <= 3e-3 * ref.norm(), bn
+    if max_ctas == 1:
+        with pytest.raises(GemmError, match="pair"):
+            gemm(a, b, bn=512, max_ctas=1)
