@@ -20,7 +20,9 @@
 //     tensor-memory lane is readable from both warp-groups, only (max, sum) goes through shared memory;
 //   * a segment that is a whole item writes its output rows; one that is cut leaves its unnormalised
 //     fp32 O and (max, sum), which a second kernel, launched as a programmatic dependent, merges
-//     per row in the order of the keys.  At most two segments of a CTA are cut.
+//     per row in the order of the keys.  At most two segments of a CTA are cut - the one it takes over
+//     from the CTA before and the one it hands on - so the workspace is two tiles per CTA, 20 MB
+//     at most, whatever the batch.
 // Measured, tile-pair kernel -> this: 16 sequences x 1 query over 6001 keys, 32 / 8 heads: 398 ->
 // 69 us (5.7 TB/s of 6.6); 32 x 16384 keys, 64 / 8 heads: 3783 -> 325 us (6.6 TB/s); 1 x 16384 keys,
 // 8 / 8 heads: 259 -> 20 us.
@@ -50,7 +52,7 @@ struct SplitPlan {
   int item_cost;             // units an item counts beside its key blocks
   int per;                   // units per CTA
   int ctas;
-  int max_parts;             // CTAs that an item's blocks may be spread over
+  int max_parts;             // CTAs that an item's blocks may be spread over, at most
   int merge;                 // some row is not finished by the first kernel
   int q_offset, kv_offset, causal;
   int nblk[SP_MAX_QT];       // visible key blocks of a tile
@@ -61,8 +63,8 @@ struct FaSplitParams {
   CUtensorMap tm_q, tm_k, tm_v;   // {128, heads, rows, batch}
   SplitPlan pl;
   float scale_log2;
-  float* part_o;                  // [item][part][tile row][128] unnormalised
-  float2* part_ml;                // [item][part][tile row] {max (log2 units), sum}
+  float* part_o;                  // [CTA][taken over / handed on][tile row][128] unnormalised
+  float2* part_ml;                // [CTA][taken over / handed on][tile row] {max (log2 units), sum}
   __nv_bfloat16* o;               // [B, Sq, Hq, 128]
   float* lse;                     // [B, Hq, Sq] or null
   uint32_t* status;
@@ -106,21 +108,20 @@ struct SplitWalk {
   int pos, end;   // flat units: this segment's first, the range's end
   int qt, bh;     // current item: query tile, batch * Hkv + key/value head
   int k0, n;      // its blocks k0 .. k0 + n - 1 belong to this segment
-  int part;       // which of the item's parts this segment is
 
   __device__ __forceinline__ bool start(const SplitPlan& pl, int cta) {
     const int total = pl.first[pl.nqt] * pl.B * pl.Hkv;
     pos = cta * pl.per;
     end = pos + pl.per < total ? pos + pl.per : total;
     qt = 0;
-    return locate(pl, cta);
+    return locate(pl);
   }
   __device__ __forceinline__ bool next(const SplitPlan& pl) {
     pos += n;
-    return locate(pl, blockIdx.x);
+    return locate(pl);
   }
   // Moves `pos` to the next key block of the range.
-  __device__ __forceinline__ bool locate(const SplitPlan& pl, int cta) {
+  __device__ __forceinline__ bool locate(const SplitPlan& pl) {
     const int items = pl.B * pl.Hkv;
     while (pos < end) {
       while (pos >= pl.first[qt + 1] * items) ++qt;
@@ -132,14 +133,17 @@ struct SplitWalk {
       k0 = skip > 0 ? 0 : -skip;
       n = pl.nblk[qt] - k0;
       if (n > end - pos) n = end - pos;
-      if (n > 0) {
-        part = cta - (pos - k0) / pl.per;
-        return true;
-      }
+      if (n > 0) return true;
     }
     return false;
   }
 };
+
+// Slot of a cut segment of a CTA: the one that begins with its item's first block is handed on, the other
+// was taken over.
+__device__ __forceinline__ uint32_t split_slot(uint32_t cta, bool begins_item) {
+  return 2u * cta + (begins_item ? 1u : 0u);
+}
 
 __global__ void __launch_bounds__(CP_THREADS, 1)
     fa_split_kernel(const __grid_constant__ FaSplitParams p) {
@@ -375,8 +379,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
       const bool row_ok = r < tile_rows && srow < pl.Sq;
       const bool whole = w.n == pl.nblk[w.qt];
       const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
-      const size_t part =
-          (static_cast<size_t>(w.qt * pl.B * pl.Hkv + w.bh) * pl.max_parts + w.part) * tile_rows + r;
+      const size_t part = static_cast<size_t>(split_slot(blockIdx.x, w.k0 == 0)) * tile_rows + r;
 #pragma unroll 1
       for (int c = 2 * t; c < 2 * t + 2; ++c) {
         uint32_t o0[32], o1[32];
@@ -454,11 +457,11 @@ __global__ void __launch_bounds__(SP_MERGE_THREADS, 6)
   const uint32_t items = pl.B * pl.Hkv, item = b * pl.Hkv + kvh;
   const uint32_t n = pl.nblk[qt];
   const uint32_t start = pl.first[qt] * items + item * (n + pl.item_cost) + pl.item_cost;
-  const int parts = n == 0 ? 0 : static_cast<int>((start + n - 1) / per - start / per + 1);
+  const uint32_t cta0 = start / per;   // its part i is CTA cta0 + i's
+  const int parts = n == 0 ? 0 : static_cast<int>((start + n - 1) / per - cta0 + 1);
   if (parts == 1) return;           // the row is final
-  const size_t row0 = static_cast<size_t>(qt * items + item) * pl.max_parts * tile_rows + r;
-  const float2* ml = p.part_ml + row0;
-  const float4* po = reinterpret_cast<const float4*>(p.part_o + row0 * CP_D) + lane;
+  const float2* ml = p.part_ml + r;
+  const float4* po = reinterpret_cast<const float4*>(p.part_o + static_cast<size_t>(r) * CP_D) + lane;
 
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float m = -INFINITY, l = 0.f;
@@ -473,8 +476,9 @@ __global__ void __launch_bounds__(SP_MERGE_THREADS, 6)
     for (int u = 0; u < 8; ++u) {
       x[u] = make_float2(-INFINITY, 0.f);
       if (base + u < i1) {
-        x[u] = ml[static_cast<size_t>(base + u) * tile_rows];
-        v[u] = po[static_cast<size_t>(base + u) * tile_rows * (CP_D / 4)];
+        const uint32_t row = split_slot(cta0 + base + u, base + u == 0) * tile_rows;
+        x[u] = ml[row];
+        v[u] = po[row * (CP_D / 4)];
       }
     }
     float m_new = m;
@@ -617,7 +621,7 @@ static bool split_wins(const SplitPlan& pl, int sms) {
 
 // Rows of partial results, and the bytes they take (none when no item is cut).
 static size_t split_rows(const SplitPlan& pl) {
-  return static_cast<size_t>(pl.nqt) * pl.B * pl.Hkv * pl.max_parts * pl.qrows * pl.group;
+  return 2ull * pl.ctas * pl.qrows * pl.group;
 }
 static long long split_bytes(const SplitPlan& pl) {
   return pl.merge ? static_cast<long long>(split_rows(pl) * (CP_D * sizeof(float) + sizeof(float2)))

@@ -297,3 +297,30 @@ def test_context_parallel_call_runs_wholly_on_its_stream(native_lib, op):
         torch.cuda.synchronize()
     ctx.check_status()
     ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(4, 1, 3000, 16, 4), (60, 16, 1501, 128, 8), (2, 130, 1500, 8, 2)])
+def test_split_key_workspace_is_two_tiles_per_cta(native_lib, shape):
+    """The bytes asked for are enough - nothing behind them is written, the result is right (bounds as
+    above) - and do not grow with the batch."""
+    import math
+
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.cp import reference_attention
+
+    B, Sq, Skv, Hq, Hkv = shape
+    q, k, v = _qkv(B, Sq, Skv, Hq, Hkv, 3)
+    lib = N.load()
+    nbytes = lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, Skv - Sq, 0, 1)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 0 < nbytes <= 2 * sms * 128 * 520
+    ws = torch.full((nbytes + 4096,), 0xff, dtype=torch.uint8, device="cuda")
+    o, lse = torch.empty_like(q), torch.empty(B, Hq, Sq, device="cuda")
+    rc = lib.cb_attn_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, Sq,
+                           Skv, Hq, Hkv, Skv - Sq, 0, 1, 1.0 / math.sqrt(128), ws.data_ptr(), nbytes,
+                           0, N.raw_stream())
+    assert rc == 0, N.last_error()
+    assert bool((ws[nbytes:] == 0xff).all())
+    ro, rl = reference_attention(q, k, v, q_offset=Skv - Sq)
+    assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
+    assert (lse - rl).abs().max() < 1e-4

@@ -264,3 +264,12 @@ def test_dispatch_counter_updates_are_releases_of_their_own():
         code = re.sub(r"//[^\n]*", "", f.read())
     updates = re.findall(r"\b(\w+)\(a\.arrived\[", code)
     assert updates and set(updates) == {"red_release_sys_add"}
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 16384, 8, 8), (512, 16, 1100, 128, 8), (512, 16, 3001, 128, 8),
+                                   (2048, 1, 3001, 64, 8), (1, 500, 4596, 8, 2)])
+def test_split_attention_workspace_does_not_grow_with_the_batch(native_lib, shape):
+    """Two cut tiles per CTA of at most 148, 128 rows of 130 fp32 words each."""
+    B, Sq, Skv, Hq, Hkv = shape
+    nbytes = native_lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, Skv - Sq, 0, 1)
+    assert 0 <= nbytes <= 2 * 148 * 128 * 520
