@@ -37,13 +37,6 @@ static int cp_launch_t(const FaCpParams& p, int grid, cudaStream_t st) {
 
 int cp_launch(const FaCpParams& p, int grid, cudaStream_t st) {
   if (grid < 1) return 0;
-  if (p.sched == nullptr) {   // persistent: one CTA per SM
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        sms > 0 && grid > sms)
-      grid = sms;
-  }
   switch (g_cp_poly) {
     case 2: return cp_launch_t<2>(p, grid, st);
     case 3: return cp_launch_t<3>(p, grid, st);

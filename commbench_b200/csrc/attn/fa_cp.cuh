@@ -22,11 +22,12 @@
 //   * CTAs draw tickets: the first `num_comm` tickets copy the list of 2-D pieces
 //     (peer -> local, 16-byte loads and stores), bumping each piece's counter when done; the
 //     others take (query tile pair, head, batch) items, heaviest first.  A launch without
-//     communication CTAs is persistent: one CTA per SM walks its share of the items, and the next
-//     item's Q, keys and first scores overlap this one's last products and its epilogue (with one
-//     CTA per item, launch, tensor-memory allocation and the pipeline's fill and drain cost 8 to 15 us
-//     an item: 16384 tokens, 32 / 8 heads, causal 2231 us then, 2064 now; 1000 queries over 7000 keys
-//     130, 122; 2 x 3000 tokens, 16 / 4 heads 109, 99).
+//     communication CTAs is persistent: a CTA goes on with the items of CTAs that have not been
+//     launched yet, and the next item's Q, keys and first scores overlap this one's last products and
+//     its epilogue (with one CTA per item, launch, tensor-memory allocation and the pipeline's fill
+//     and drain cost 8 to 15 us an item: 16384 tokens, 32 / 8 heads, causal 2231 us, 2036 so).
+//     Items go to whatever SM is free: with two SMs held by a kernel of another stream the same call
+//     takes 5 % more (16: 17 %), where a fixed share of the items per CTA took twice as long.
 // What bounds the inner loop (3500 cycles for 128 keys x 256 rows against 2048 on the tensor cores): the
 // MMA warp's issue, 32 MMAs at about 75 cycles, and behind it a tile's chain scores -> softmax (1700) ->
 // P -> product -> next scores; the exponentials alone are not (without them: the same time).
@@ -42,6 +43,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include "../prim/clc.cuh"
 #include "../prim/tcgen05.cuh"
 #include "../prim/tma.cuh"
 #include "fa_cp_types.h"
@@ -53,6 +55,8 @@ struct CpCtl {
   uint64_t k_full[CP_KST], k_empty[CP_KST];
   uint64_t v_full[CP_VST], v_empty[CP_VST];
   uint64_t s_full[2], p_full[2], pv_done[2];  // per query tile
+  uint64_t item_full, item_empty;             // the answer to the CTA's request for its next item
+  uint4 item_answer;
   uint32_t tmem_base;
   int abort_flag;
   int ticket;
@@ -309,15 +313,46 @@ struct CpItem {
     }
     return false;
   }
-  // The i-th item of a CTA.  With tickets a CTA has one.  A launch without them is persistent: one CTA
-  // per SM walks the list, heaviest items first, forwards in even rounds and backwards in odd
-  // ones, which evens out what the CTAs get.
-  __device__ __forceinline__ bool at(const FaCpParams& p, int ticket, int i) {
-    if (p.sched != nullptr) return i == 0 && decode(p, ticket - p.num_comm);
-    const int g = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
-    return decode(p, i * g + ((i & 1) != 0 ? g - 1 - c : c));
+};
+
+// The items of a CTA, for one role.  The first is that of its ticket or block index.  With tickets there
+// is no other; without, the CTA goes on with items of CTAs that have not been launched (prim/clc.cuh):
+// cp_fetch_items asks for one ahead, and every role reads the answer and says so.
+struct CpWalk {
+  CpItem item;
+  int n = 0;   // items taken
+  // The next item, or false at the end (or on an abort).  Called by one thread, or with kWarp by all lanes
+  // of a converged warp.
+  template <bool kWarp>
+  __device__ __forceinline__ bool next(const FaCpParams& p, CpCtl& ctl, int ticket) {
+    if (n++ == 0) return item.decode(p, ticket - p.num_comm);
+    if (p.sched != nullptr) return false;
+    if constexpr (kWarp) {
+      if (!mbar_wait_warp(&ctl.item_full, n & 1, &ctl.abort_flag, p.status, 0xE40)) return false;
+    } else {
+      if (!mbar_wait(&ctl.item_full, n & 1, &ctl.abort_flag, p.status, 0xE40)) return false;
+    }
+    const int block = clc_cancelled_block(&ctl.item_answer);
+    if constexpr (kWarp) __syncwarp();
+    if (!kWarp || (threadIdx.x & 31u) == 0u) mbar_arrive(&ctl.item_empty);
+    return block >= 0 && item.decode(p, block);
   }
 };
+// Roles that walk the items: producer, MMA warp, eight softmax warps.
+static constexpr int CP_ITEM_READERS = 10;
+
+// One thread: keeps one item ahead of the CTA's roles.  A request is made when all of them have started on
+// the item before, so a CTA holds one item in reserve, and ends with the first that found none.
+__device__ __forceinline__ void cp_fetch_items(const FaCpParams& p, CpCtl& ctl) {
+  for (uint32_t i = 0;; ++i) {
+    if (i > 0 && !mbar_wait(&ctl.item_empty, (i - 1) & 1, &ctl.abort_flag, p.status, 0xE41)) return;
+    fence_proxy_async_smem();   // the last answer was read with ordinary loads
+    mbar_arrive_expect_tx(&ctl.item_full, 16);
+    clc_try_cancel(&ctl.item_answer, &ctl.item_full);
+    if (!mbar_wait(&ctl.item_full, i & 1, &ctl.abort_flag, p.status, 0xE42)) return;
+    if (clc_cancelled_block(&ctl.item_answer) < 0) return;
+  }
+}
 
 // kPoly: every kPoly-th pair of keys takes its exponential from the FMA pipe (0: none).
 template <int kPoly>
@@ -342,13 +377,15 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
   CpItem first;
   if (ticket < p.num_comm) {
     cp_comm_cta(p, ticket);
-  } else if (first.at(p, ticket, 0)) {
+  } else if (first.decode(p, ticket - p.num_comm)) {
     // Every role walks the CTA's items with a copy of its own; block counts run through, so that
     // barriers, rings and tensor memory carry over and the next item's Q, keys and scores overlap
     // this one's last products and epilogue.
     if (threadIdx.x == 0) {
       mbar_init(&ctl.q_full, 1);
       mbar_init(&ctl.q_empty, 1);
+      mbar_init(&ctl.item_full, 1);
+      mbar_init(&ctl.item_empty, CP_ITEM_READERS);
       for (int i = 0; i < CP_KST; ++i) {
         mbar_init(&ctl.k_full[i], 1);
         mbar_init(&ctl.k_empty[i], 1);
@@ -382,10 +419,11 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
     if (warp == 0) {
       if (lane == 0) {
         // ---------------------------------------------------------------- producer
-        CpItem w;
+        CpWalk walk;
+        const CpItem& w = walk.item;
         bool ok = true;
         int g0 = 0, nq = 0;   // blocks and items before this item
-        for (int i = 0; ok && w.at(p, ticket, i); ++i) {
+        while (ok && walk.next<false>(p, ctl, ticket)) {
           if (w.nblk == 0) continue;
           const CpQSeg& qs = p.qseg[w.qs_i];
           const int kv_head = w.head / p.kv_group;
@@ -523,9 +561,9 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           __syncwarp();
           return true;
         };
-        CpItem w;
-        for (int i = 0; ok && w.at(p, ticket, i); ++i) {
-          const int nblk = __shfl_sync(0xffffffffu, w.nblk, 0);
+        CpWalk walk;
+        while (ok && walk.next<true>(p, ctl, ticket)) {
+          const int nblk = __shfl_sync(0xffffffffu, walk.item.nblk, 0);
           if (nblk == 0) continue;
           ok = wait_all(&ctl.q_full, nq & 1, 0xE10);
           ++nq;
@@ -551,6 +589,8 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           g0 += nblk;
         }
       }
+    } else if (warp == 2) {
+      if (lane == 0 && p.sched == nullptr) cp_fetch_items(p, ctl);
     }
     } else {
       cp_reg_inc<216>();
@@ -561,10 +601,11 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
       const uint32_t lane_addr = (q * 32u) << 16;
       const uint32_t tS = tmem + 256u * t + lane_addr;
       const uint32_t tO = tS + 128u;
-      CpItem w;
+      CpWalk walk;
+      const CpItem& w = walk.item;
       bool ok = true;
       int g0 = 0;   // blocks before this item
-      for (int i = 0; ok && w.at(p, ticket, i); ++i) {
+      while (ok && walk.next<true>(p, ctl, ticket)) {
         const CpQSeg& qs = p.qseg[w.qs_i];
         const int row_in_seg = w.pair * 2 * CP_BM + t * CP_BM + static_cast<int>(r);
         const int tile_first = w.q_first + t * CP_BM;     // position of row 0 of this tile

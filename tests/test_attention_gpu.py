@@ -324,3 +324,39 @@ def test_split_key_workspace_is_two_tiles_per_cta(native_lib, shape):
     ro, rl = reference_attention(q, k, v, q_offset=Skv - Sq)
     assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
     assert (lse - rl).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("kv_offset", [0, 900])
+def test_tile_pairs_beside_a_kernel_that_holds_sms(native_lib, kv_offset):
+    """More tile pairs than SMs while a GEMM on another stream holds some of these: the same bits as
+    without it.  With kv_offset some pairs see no key."""
+    import math
+
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.gemm import gemm
+
+    B, S, Hq, Hkv = 2, 2000, 32, 8
+    q, k, v = _qkv(B, S, S, Hq, Hkv, 47)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    a = torch.randn(4096, 4096, device="cuda").bfloat16()
+    side = torch.cuda.Stream()
+
+    def run():
+        o, lse = torch.empty_like(q), torch.empty(B, Hq, S, device="cuda")
+        rc = N.load().cb_attn_fwd4(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
+                                   B, S, S, Hq, Hkv, 0, kv_offset, 1, 1.0 / math.sqrt(128),
+                                   status.data_ptr(), N.raw_stream())
+        assert rc == 0, N.last_error()
+        return o, lse
+
+    ref = run()
+    c = torch.empty(4096, 4096, dtype=torch.bfloat16, device="cuda")
+    for n in (1, 8, 100):
+        torch.cuda.synchronize()
+        gemm(a, a, out=c, bn=256, max_ctas=n, stream=side)
+        torch.cuda._sleep(100_000)                    # the GEMM is there first
+        for _ in range(3):
+            o, lse = run()
+            assert torch.equal(o, ref[0]) and torch.equal(lse, ref[1])
+    torch.cuda.synchronize()
+    assert int(status.abs().sum()) == 0
