@@ -317,42 +317,39 @@ struct CpItem {
 
 // The items of a CTA, for one role.  The first is that of its ticket or block index.  With tickets there
 // is no other; without, the CTA goes on with items of CTAs that have not been launched (prim/clc.cuh):
-// cp_fetch_items asks for one ahead, and every role reads the answer and says so.
+// the producer asks for one when it has issued all loads of the item before, and every role reads the
+// answer and says so.  Asking earlier would hand the short items at the end of the list to whoever started
+// first, not to whoever is free first: 2 x 3272 tokens, 8 / 2 heads, 208 items took 77 us so, 60 now.
 struct CpWalk {
   CpItem item;
   int n = 0;   // items taken
-  // The next item, or false at the end (or on an abort).  Called by one thread, or with kWarp by all lanes
-  // of a converged warp.
-  template <bool kWarp>
+  // For a warp other than the producer's, all lanes converged: the next item, or false at the end (or on
+  // an abort).
   __device__ __forceinline__ bool next(const FaCpParams& p, CpCtl& ctl, int ticket) {
     if (n++ == 0) return item.decode(p, ticket - p.num_comm);
     if (p.sched != nullptr) return false;
-    if constexpr (kWarp) {
-      if (!mbar_wait_warp(&ctl.item_full, n & 1, &ctl.abort_flag, p.status, 0xE40)) return false;
-    } else {
-      if (!mbar_wait(&ctl.item_full, n & 1, &ctl.abort_flag, p.status, 0xE40)) return false;
-    }
+    if (!mbar_wait_warp(&ctl.item_full, n & 1, &ctl.abort_flag, p.status, 0xE40)) return false;
     const int block = clc_cancelled_block(&ctl.item_answer);
-    if constexpr (kWarp) __syncwarp();
-    if (!kWarp || (threadIdx.x & 31u) == 0u) mbar_arrive(&ctl.item_empty);
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0u) mbar_arrive(&ctl.item_empty);
     return block >= 0 && item.decode(p, block);
   }
-};
-// Roles that walk the items: producer, MMA warp, eight softmax warps.
-static constexpr int CP_ITEM_READERS = 10;
-
-// One thread: keeps one item ahead of the CTA's roles.  A request is made when all of them have started on
-// the item before, so a CTA holds one item in reserve, and ends with the first that found none.
-__device__ __forceinline__ void cp_fetch_items(const FaCpParams& p, CpCtl& ctl) {
-  for (uint32_t i = 0;; ++i) {
-    if (i > 0 && !mbar_wait(&ctl.item_empty, (i - 1) & 1, &ctl.abort_flag, p.status, 0xE41)) return;
+  // For the producer thread.
+  __device__ __forceinline__ bool request(const FaCpParams& p, CpCtl& ctl, int ticket) {
+    if (n++ == 0) return item.decode(p, ticket - p.num_comm);
+    if (p.sched != nullptr) return false;
+    if (n > 2 && !mbar_wait(&ctl.item_empty, (n - 1) & 1, &ctl.abort_flag, p.status, 0xE41))
+      return false;
     fence_proxy_async_smem();   // the last answer was read with ordinary loads
     mbar_arrive_expect_tx(&ctl.item_full, 16);
     clc_try_cancel(&ctl.item_answer, &ctl.item_full);
-    if (!mbar_wait(&ctl.item_full, i & 1, &ctl.abort_flag, p.status, 0xE42)) return;
-    if (clc_cancelled_block(&ctl.item_answer) < 0) return;
+    if (!mbar_wait(&ctl.item_full, n & 1, &ctl.abort_flag, p.status, 0xE42)) return false;
+    const int block = clc_cancelled_block(&ctl.item_answer);
+    return block >= 0 && item.decode(p, block);
   }
-}
+};
+// Warps that read an answer: MMA and eight of the softmax.
+static constexpr int CP_ITEM_READERS = 9;
 
 // kPoly: every kPoly-th pair of keys takes its exponential from the FMA pipe (0: none).
 template <int kPoly>
@@ -423,7 +420,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
         const CpItem& w = walk.item;
         bool ok = true;
         int g0 = 0, nq = 0;   // blocks and items before this item
-        while (ok && walk.next<false>(p, ctl, ticket)) {
+        while (ok && walk.request(p, ctl, ticket)) {
           if (w.nblk == 0) continue;
           const CpQSeg& qs = p.qseg[w.qs_i];
           const int kv_head = w.head / p.kv_group;
@@ -562,7 +559,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           return true;
         };
         CpWalk walk;
-        while (ok && walk.next<true>(p, ctl, ticket)) {
+        while (ok && walk.next(p, ctl, ticket)) {
           const int nblk = __shfl_sync(0xffffffffu, walk.item.nblk, 0);
           if (nblk == 0) continue;
           ok = wait_all(&ctl.q_full, nq & 1, 0xE10);
@@ -589,8 +586,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           g0 += nblk;
         }
       }
-    } else if (warp == 2) {
-      if (lane == 0 && p.sched == nullptr) cp_fetch_items(p, ctl);
     }
     } else {
       cp_reg_inc<216>();
@@ -605,7 +600,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
       const CpItem& w = walk.item;
       bool ok = true;
       int g0 = 0;   // blocks before this item
-      while (ok && walk.next<true>(p, ctl, ticket)) {
+      while (ok && walk.next(p, ctl, ticket)) {
         const CpQSeg& qs = p.qseg[w.qs_i];
         const int row_in_seg = w.pair * 2 * CP_BM + t * CP_BM + static_cast<int>(r);
         const int tile_first = w.q_first + t * CP_BM;     // position of row 0 of this tile
