@@ -163,15 +163,13 @@ def raw_stream(stream=None) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
-def new_empty(like, shape, dtype=None, stream=None, handed_out: bool = True):
-    """``like.new_empty`` for memory that a call running on ``stream`` (None: the current stream) writes.
+def new_empty_on(stream, like, shape, dtype=None, handed_out: bool = True):
+    """``like.new_empty`` for memory that a call running on ``stream`` writes.
 
     It comes from the pool of the stream that writes it: a block of the current stream's pool may have
     been freed with work of that stream still queued on it, and nothing orders ``stream`` behind that
     work.  For a result (``handed_out``), the current stream, where the caller goes on with it, is
     recorded as a second user, so that the block is not reused before that stream is done either."""
-    if stream is None:
-        return like.new_empty(shape, dtype=dtype)
     import torch
 
     with torch.cuda.stream(stream):

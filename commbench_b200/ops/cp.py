@@ -36,13 +36,14 @@ def _split_attention(q, k, v, out, lse, causal, q_offset, kv_offset, sc, status_
     nbytes = lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, q_offset, kv_offset, int(causal))
     if nbytes < 0:
         return False
-    ws = None
+    ws = 0
     if nbytes > 0:
-        ws = N.new_empty(q, (nbytes,), torch.uint8, stream, handed_out=False)
+        buf = q.new_empty((nbytes,), dtype=torch.uint8) if stream is None else \
+            N.new_empty_on(stream, q, (nbytes,), torch.uint8, handed_out=False)
+        ws = buf.data_ptr()
     rc = lib.cb_attn_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                            lse.data_ptr() if lse is not None else 0, B, Sq, Skv, Hq, Hkv, q_offset,
-                           kv_offset, int(causal), sc, ws.data_ptr() if ws is not None else 0, nbytes,
-                           status_ptr, N.raw_stream(stream))
+                           kv_offset, int(causal), sc, ws, nbytes, status_ptr, N.raw_stream(stream))
     if rc != 0:
         raise CommError(f"attention launch failed: {N.last_error()}")
     return True
@@ -71,9 +72,10 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: 
     if v.shape != k.shape or k.shape[0] != B:
         raise CommError("k and v must have the same shape and q's batch size")
     if out is None:
-        out = N.new_empty(q, q.shape, stream=stream)
+        out = torch.empty_like(q) if stream is None else N.new_empty_on(stream, q, q.shape)
     if lse is None:
-        lse = N.new_empty(q, (B, Hq, Sq), torch.float32, stream)
+        lse = q.new_empty((B, Hq, Sq), dtype=torch.float32) if stream is None else \
+            N.new_empty_on(stream, q, (B, Hq, Sq), torch.float32)
     sc = scale if scale is not None else 1.0 / math.sqrt(D)
     if impl is None:
         impl = get_config().attn_impl
@@ -188,11 +190,9 @@ class _CpBase:
         return self.ctx.comms[i].status if self.emu else self.ctx.comm.status
 
     def _run(self, stream, inputs, fn, *args):
-        """``fn(*args)`` with ``stream`` (None: as it is) as the current stream, so that a call's input
-        copies, barriers, allocations and launches are ordered among themselves; inputs and results
-        are recorded on both streams."""
-        if stream is None:
-            return fn(*args)
+        """``fn(*args)`` with ``stream`` as the current stream, so that a call's input copies, barriers,
+        allocations and launches are ordered among themselves; inputs and results are recorded on
+        both streams."""
         caller = torch.cuda.current_stream(self.ctx.device)
         for t in _tensors(inputs):
             t.record_stream(stream)
@@ -273,6 +273,8 @@ class RingAttention(_CpBase):
         entry per virtual rank under an ``EmuContext``).  Returns ``(o, lse)``.
 
         With ``stream`` the whole call runs there, the copy of ``k`` / ``v`` into their slot included."""
+        if stream is None:
+            return self._forward(q, k, v, causal, out, want_lse, scale)
         return self._run(stream, (q, k, v), self._forward, q, k, v, causal, out, want_lse, scale)
 
     def _forward(self, q, k, v, causal, out, want_lse, scale):
@@ -383,6 +385,8 @@ class UlyssesAttention(_CpBase):
         "already there".  Returns this rank's ``o_buf`` (valid until the next call).
 
         With ``stream`` the whole call runs there, the input copies included."""
+        if stream is None:
+            return self._forward(q, k, v, causal, scale)
         return self._run(stream, (q, k, v), self._forward, q, k, v, causal, scale)
 
     def _forward(self, q, k, v, causal, scale):

@@ -35,7 +35,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, alph
     if K != K2:
         raise GemmError(f"inner dimensions differ: {K} vs {K2}")
     if out is None:
-        out = N.new_empty(a, (M, Nn), torch.bfloat16, stream)
+        out = a.new_empty((M, Nn), dtype=torch.bfloat16) if stream is None else \
+            N.new_empty_on(stream, a, (M, Nn), torch.bfloat16)
     else:
         _check(out, "out")
         if out.dtype != torch.bfloat16 or tuple(out.shape) != (M, Nn):
@@ -150,7 +151,8 @@ def gemm_fp8_mx(a_q, a_sf, b_q, b_sf, out=None, alpha: float = 1.0, pair: bool =
         if not (t.dtype == torch.int32 and t.is_contiguous() and tuple(t.shape) == (kg, rows)):
             raise GemmError(f"{name} must be a contiguous int32 tensor [{kg}, {rows}]")
     if out is None:
-        out = N.new_empty(a_q, (M, Nn), torch.bfloat16, stream)
+        out = a_q.new_empty((M, Nn), dtype=torch.bfloat16) if stream is None else \
+            N.new_empty_on(stream, a_q, (M, Nn), torch.bfloat16)
     else:
         _check(out, "out")
     # pair: a CTA pair per 256 x 192 tile (default, fastest); otherwise one CTA per 128 x 192
@@ -196,7 +198,8 @@ def gemm_fp8_blockscaled(a_q, a_s, b_q, b_s, out=None, alpha: float = 1.0, pair:
             and b_s.dtype == torch.float32):
         raise GemmError("scales must be contiguous fp32 tensors")
     if out is None:
-        out = N.new_empty(a_q, (M, Nn), torch.bfloat16, stream)
+        out = a_q.new_empty((M, Nn), dtype=torch.bfloat16) if stream is None else \
+            N.new_empty_on(stream, a_q, (M, Nn), torch.bfloat16)
     else:
         _check(out, "out")
     rc = lib.cb_gemm_fp8_blockscaled(a_q.data_ptr(), a_s.data_ptr(), b_q.data_ptr(), b_s.data_ptr(),
