@@ -3,9 +3,8 @@
 // shards that are already there, and carries the running (max, sum, O) of a query tile across
 // ALL shards in registers / tensor memory - no partial results, no merge launches.
 //
-// The attention math is the kernel of fa_fwd4.cu (two 128-row query tiles per CTA, a softmax
-// warp-group per tile, S / P / O in tensor memory, K ring of 3 and V ring of 2).  What is
-// generalised here:
+// Two 128-row query tiles per CTA, a softmax warp-group per tile, S / P / O in tensor memory, K ring
+// of 3 and V ring of 2:
 //   * keys and values are a list of SEGMENTS of one local buffer (row range, global position of
 //     the first key, optional "ready" counter).  Ring attention lists the shards in ring
 //     order - own shard first, then rank-1, rank-2, ... - Ulysses lists the sequence in order;
@@ -16,7 +15,7 @@
 //     TMA loads and whose O rows are stored straight into their owners' output tensors;
 //   * registers are moved from the four utility warps (producer, MMA issuer, two idle) to
 //     the eight softmax warps with setmaxnreg (72 / 216 per thread), which keeps a 128-column row
-//     of scores in registers without spills, and every `kPoly`-th pair of exponentials is
+//     of scores in registers (three of them spilled), and every `kPoly`-th pair of exponentials is
 //     computed on the FMA pipe (a cubic after a round-to-nearest split) instead of the SFU,
 //     which otherwise is as busy as the tensor pipe;
 //   * CTAs draw tickets: the first `num_comm` tickets copy the list of 2-D pieces
@@ -25,9 +24,9 @@
 //     communication CTAs is persistent: a CTA goes on with the items of CTAs that have not been
 //     launched yet, and the next item's Q, keys and first scores overlap this one's last products and
 //     its epilogue (with one CTA per item, launch, tensor-memory allocation and the pipeline's fill
-//     and drain cost 8 to 15 us an item: 16384 tokens, 32 / 8 heads, causal 2231 us, 2036 so).
+//     and drain cost 8 to 15 us an item: 16384 tokens, 32 / 8 heads, causal 2231 us, 2040 so).
 //     Items go to whatever SM is free: with two SMs held by a kernel of another stream the same call
-//     takes 5 % more (16: 17 %), where a fixed share of the items per CTA took twice as long.
+//     takes 5 % more (16: 16 %), where a fixed share of the items per CTA took twice as long.
 // What bounds the inner loop (3500 cycles for 128 keys x 256 rows against 2048 on the tensor cores): the
 // MMA warp's issue, 32 MMAs at about 75 cycles, and behind it a tile's chain scores -> softmax (1700) ->
 // P -> product -> next scores; the exponentials alone are not (without them: the same time).

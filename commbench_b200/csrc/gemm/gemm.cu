@@ -181,8 +181,10 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
 // 256-wide tiles 0.16 / 0.22 / 0.34 (0.18 / 0.30 / 0.50 where rows do not start on 128-byte lines, since
 // every box row then touches two); all CTAs together draw at most 17 TB/s out of L2 (11), weights
 // arrive at 6 TB/s from memory, and a persistent tile takes 2.5 us however short its K loop
-// (its epilogue).  Over 105 random shapes (M 1-8192, N 512-16384, K 512-8192, bf16 and fp8) the choice
-// is within 1.5 % of the best of all variants on (geometric) average.
+// (its epilogue).  Over 105 random shapes (M 1-8192, N 512-16384, K 512-8192, bf16 and fp8), called in
+// a row, the choice takes 3.5 % more than the best of all variants on (geometric) average and over 10 %
+// more for 17 of them; the worst is 593 x 3696 x 1200, where it picks pairs (14.5 us) and 128-wide tiles
+// of the small kernel take 9.0.
 struct GemmChoice {
   int bn;      // persistent: 64 ... 512 as in cb_gemm_bf16; small kernel: its tile width
   int split;   // 0: persistent kernel; else the small kernel's K splits

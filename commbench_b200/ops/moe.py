@@ -148,8 +148,8 @@ class MoELayer:
         straight to its final position in the destination's per-expert buffer; ``"per_token"``
         sends a token once per destination RANK and lets the receive kernel expand it to the
         rows of that rank's experts (fewer NVLink bytes when a token selects several experts of
-        one rank: about a third at top-8 over 8 ranks; the receive then waits for all of a
-        rank's rows instead of expert by expert)."""
+        one rank: about a third at top-8 over 8 ranks).  In neither form is an expert's input there
+        early: a dispatch CTA holds rows of all experts and counts them in at its end."""
         self.ctx, self.lib = ctx, ctx.lib
         from ..config import get_config
 
@@ -226,8 +226,9 @@ class MoELayer:
         ``bias0`` / ``bias1``: optional [T, H] bf16 tensors added in the combine reduction (a
         shared expert's output, a residual).  Returns y [T, H] bf16 (list in emulation).
 
-        The small kernels of the layer (slots, plan, dispatch, receive, combine reduction) are chained with programmatic dependent launch: each may be scheduled while
-        its predecessor still runs and waits on the device for it."""
+        The small kernels of the layer (slots, plan, dispatch, receive, combine reduction) are chained
+        with programmatic dependent launch: each may be scheduled while its predecessor still runs
+        and waits on the device for it."""
         lib, W, E, K, T, H, I = self.lib, self.W, self.E, self.K, self.T, self.H, self.I
         if not self.emu:
             xs, topk_idx, topk_w = [xs], [topk_idx], [topk_w]

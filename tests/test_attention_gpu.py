@@ -178,9 +178,11 @@ def test_split_key_attention_matches_reference(native_lib, shape, causal):
 
 
 def test_split_and_pair_kernels_agree_on_the_public_call(native_lib):
-    """The size rule sends decode to the split kernel and a full prefill to the tile-pair kernel;
-    a workspace that is too small is refused."""
+    """The size rule sends decode to the split kernel and a full prefill to the tile-pair kernel; both
+    give the same on one call (each within 1e-2 of the largest value of fp32, lse within 1e-4); a
+    workspace that is too small is refused."""
     import ctypes as C
+    import math
 
     from commbench_b200 import _native as N
     from commbench_b200.ops.cp import flash_attention, reference_attention
@@ -193,6 +195,12 @@ def test_split_and_pair_kernels_agree_on_the_public_call(native_lib):
     ro, rl = reference_attention(q, k, v, causal=True, q_offset=2999)
     assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
     assert (lse - rl).abs().max() < 1e-4
+    o4, lse4 = torch.empty_like(o), torch.empty_like(lse)
+    rc = lib.cb_attn_fwd4(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(o4), N.ptr(lse4), 4, 1, 3000, 16, 4, 2999,
+                          0, 1, 1.0 / math.sqrt(128), 0, N.stream_ptr())
+    assert rc == 0, N.last_error()
+    assert (o.float() - o4.float()).abs().max() <= 2e-2 * ro.abs().max()
+    assert (lse - lse4).abs().max() < 2e-4
     rc = lib.cb_attn_split(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(o), N.ptr(lse), 4, 1, 3000, 16, 4, 2999,
                            0, 1, C.c_float(0.1), N.ptr(o), C.c_longlong(16), C.c_void_p(0),
                            N.stream_ptr())
@@ -360,3 +368,48 @@ def test_tile_pairs_beside_a_kernel_that_holds_sms(native_lib, kv_offset):
             assert torch.equal(o, ref[0]) and torch.equal(lse, ref[1])
     torch.cuda.synchronize()
     assert int(status.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("s,hq,hkv,split", [(512, 4, 1, True), (2304, 32, 8, False)])
+def test_ring_on_one_real_rank_takes_either_kernel(native_lib, s, hq, hkv, split):
+    """One rank of a real context: few query tiles go to the split-key kernel, more tile pairs than SMs
+    to the tile-pair kernel, persistent since there is nothing to pull.  Both masks in turn on one object;
+    bounds as for the two kernels."""
+    from commbench_b200 import _native as N
+    from commbench_b200.ops.cp import RingAttention, reference_attention
+    from commbench_b200.runtime.context import CommContext
+
+    assert (N.load().cb_attn_split_bytes(1, s, s, hq, hkv, 0, 0, 1) >= 0) == split
+    ctx = CommContext(heap_bytes=64 << 20)
+    ring = RingAttention(ctx, 1, s, hq, hkv)
+    q, k, v = _qkv(1, s, s, hq, hkv, 61)
+    for causal in (True, True, False, True):
+        o, lse = ring.forward(q, k, v, causal=causal)
+        o2, none = ring.forward(q, ring.k_local(), ring.v_local(), causal=causal, want_lse=False)
+        ro, rl = reference_attention(q, k, v, causal=causal)
+        assert (o.float() - ro).abs().max() <= 1e-2 * ro.abs().max()
+        assert (lse - rl).abs().max() < 1e-4
+        assert none is None and torch.equal(o, o2)
+    ctx.check_status()
+    ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(4, 1, 3000, 16, 4), (1, 1100, 1100, 32, 8)])
+def test_attention_in_a_cuda_graph(native_lib, shape):
+    """Split-key kernel, its merge and the workspace made inside the call, and the tile-pair kernel with
+    more items than SMs, captured and replayed on new inputs: the bits of the plain call."""
+    from commbench_b200.ops.cp import flash_attention
+
+    B, Sq, Skv, Hq, Hkv = shape
+    q, k, v = _qkv(B, Sq, Skv, Hq, Hkv, 71)
+    flash_attention(q, k, v, q_offset=Skv - Sq)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o, lse = flash_attention(q, k, v, q_offset=Skv - Sq)
+    for seed in range(3):
+        for t, x in zip((q, k, v), _qkv(B, Sq, Skv, Hq, Hkv, seed)):
+            t.copy_(x)
+        graph.replay()
+        ro, rl = flash_attention(q, k, v, q_offset=Skv - Sq)
+        assert torch.equal(o, ro) and torch.equal(lse, rl)

@@ -133,3 +133,26 @@ def test_moe_dispatch_edges(native_lib, T, H, K, world, dispatch):
         ref = reference_moe(xs[r], idxs[r], wr, w1_all, w2_all, I)
         err = (ys[r].float() - ref).abs().max().item()
         assert err / (ref.abs().max().item() + 1e-6) < 3e-2, (r, err)
+
+
+@pytest.mark.parametrize("dispatch", ["per_pair", "per_token"])
+def test_moe_layer_on_one_real_rank(native_lib, dispatch):
+    """A context of one real rank takes its own counts as the count matrix (no gather, one launch less).
+    3e-2 of the largest value, as in the layer test above."""
+    from commbench_b200.ops.moe import MoELayer, reference_moe, router_topk
+    from commbench_b200.runtime.context import CommContext
+
+    T, H, I, E, K = 96, 512, 256, 8, 2
+    ctx = CommContext(heap_bytes=64 << 20)
+    layer = MoELayer(ctx, T, H, I, E, K, dispatch=dispatch)
+    assert layer.launches_per_call == 7
+    w1, w2 = layer.weights()
+    for seed in range(3):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+        idx, w = router_topk(torch.randn(T, E, device="cuda", generator=g), K)
+        y = layer.forward(x, idx, w)
+        ref = reference_moe(x, idx, w, w1, w2, I)
+        assert (y.float() - ref).abs().max() <= 3e-2 * ref.abs().max()
+    ctx.check_status()
+    ctx.close()
