@@ -160,10 +160,10 @@ def raw_stream(stream=None) -> int:
         return stream.cuda_stream
     import torch
 
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)     # private: may go in another torch
-    if raw is None:
+    try:
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    except AttributeError:               # private: may be missing in another torch
         return torch.cuda.current_stream().cuda_stream
-    return raw(torch.cuda.current_device())
 
 
 def new_empty_on(stream, like, shape, dtype=None, handed_out: bool = True):

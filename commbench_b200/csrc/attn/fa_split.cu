@@ -28,6 +28,8 @@
 // (6.6 TB/s); 1 x 16384 keys, 8 / 8 heads: 259 -> 20 us.
 //
 // Every mbarrier wait is bounded (see mbarrier.cuh).
+#include <math.h>
+
 #include <string>
 
 #include "../gemm/launch.h"
@@ -41,9 +43,20 @@ namespace cb {
 static constexpr int SP_MAX_QT = 64;                                 // query tiles per batch and head
 static constexpr int SP_ITEM_COST = 3;
 static constexpr int SP_MERGE_THREADS = 128;
-// Microseconds of a unit, and of the merge: 2 on the device, the rest the workspace and the second
-// launch of a call that is bound by its launches.
-static constexpr float SP_BLOCK_US = 1.5f, SP_MERGE_US = 5.f;
+// Microseconds of a unit, of the merge and of a launch's start and end on the device.
+static constexpr float SP_BLOCK_US = 1.5f, SP_MERGE_US = 5.f, SP_START_US = 6.f;
+
+// What a call takes when calls follow each other: on the device, but no less than on the host, where a
+// cut costs a workspace and a second launch (measured through flash_attention, 16.5 and 21.5 us).  Calls that
+// are both bound by the host are told apart by the device.
+struct CallTime {
+  float device;
+  bool merge;
+  bool better_than(const CallTime& o) const {
+    const float a = fmaxf(device, merge ? 21.f : 16.5f), b = fmaxf(o.device, o.merge ? 21.f : 16.5f);
+    return a < b || (a == b && device < o.device);
+  }
+};
 
 struct SplitPlan {
   int B, Sq, Skv, Hq, Hkv, group;
@@ -574,7 +587,8 @@ static bool split_plan(SplitPlan& pl, int B, int Sq, int Skv, int Hq, int Hkv, i
   if (pl.nqt == 1) {
     // Whole items per CTA when that costs less than the merge.
     const long long whole = (items + sms - 1) / sms * pl.nblk[0];
-    if (SP_BLOCK_US * static_cast<float>(whole) < SP_BLOCK_US * static_cast<float>(pl.per) + SP_MERGE_US)
+    const CallTime uncut = {SP_START_US + SP_BLOCK_US * static_cast<float>(whole), false};
+    if (uncut.better_than({SP_START_US + SP_BLOCK_US * static_cast<float>(pl.per) + SP_MERGE_US, true}))
       pl.per = static_cast<int>(whole);
   }
   pl.ctas = static_cast<int>((total + pl.per - 1) / pl.per);
@@ -602,12 +616,12 @@ static int split_sms() {
 // Which kernel takes a call, from a model of both in microseconds.  The tile-pair kernel takes
 // kPairBlock for a key block of its 256 rows and is as long as its longest item or its share of all
 // of them; the split kernel takes SP_BLOCK_US for a unit of its 128 rows, plus the merge.
-// Measured, split / pair (B, Sq, Skv, Hq, Hkv): (1, 64, 64, 4, 4) 7.6 / 9.0 us, (1, 300, 300, 4, 1)
-// 11 / 14, (1, 500, 4596, 8, 2) 23 / 81, (1, 8192, 8192, 4, 4) 90 / 127; near the line
-// (1, 1280, 1280, 16, 8) 33 / 30, (1, 2000, 2777, 16, 4) 54 / 51, (1, 1000, 7000, 32, 8) 118 / 112;
+// Measured on the device, split / pair (B, Sq, Skv, Hq, Hkv): (1, 64, 64, 4, 4) 7.6 / 9.0 us,
+// (1, 300, 300, 4, 1) 11 / 14 (with a merge, so a call takes 21.5 / 16.5), (1, 500, 4596, 8, 2)
+// 23 / 81, (1, 8192, 8192, 4, 4) 90 / 127; near the line (1, 1280, 1280, 16, 8) 33 / 30, (1, 2000, 2777, 16, 4) 54 / 51, (1, 1000, 7000, 32, 8) 118 / 112;
 // beyond it (2, 2000, 2000, 32, 8) 125 / 88.
 static bool split_wins(const SplitPlan& pl, int sms) {
-  constexpr float kPairBlock = 2.0f, kPairStart = 7.f, kStart = 6.f;
+  constexpr float kPairBlock = 2.0f, kPairStart = 7.f;
   const float pair_tiles = static_cast<float>((pl.Sq + 2 * CP_BM - 1) / (2 * CP_BM));
   float blocks = 0.f;
   for (int i = 0; i < pl.nqt; ++i) blocks += static_cast<float>(pl.nblk[i]);
@@ -615,8 +629,11 @@ static bool split_wins(const SplitPlan& pl, int sms) {
   const float share = avg * pair_tiles * static_cast<float>(pl.Hq) * static_cast<float>(pl.B) /
                       static_cast<float>(sms);
   const float longest = static_cast<float>(pl.nblk[pl.nqt - 1]);
-  const float pair = kPairStart + kPairBlock * (share > longest ? share : longest);
-  return kStart + (pl.merge ? SP_MERGE_US : 0.f) + SP_BLOCK_US * static_cast<float>(pl.per) < pair;
+  const CallTime pair = {kPairStart + kPairBlock * (share > longest ? share : longest), false};
+  const CallTime split = {SP_START_US + (pl.merge ? SP_MERGE_US : 0.f) +
+                              SP_BLOCK_US * static_cast<float>(pl.per),
+                          pl.merge != 0};
+  return split.better_than(pair);
 }
 
 // Rows of partial results, and the bytes they take (none when no item is cut).

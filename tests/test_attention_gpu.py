@@ -370,7 +370,7 @@ def test_tile_pairs_beside_a_kernel_that_holds_sms(native_lib, kv_offset):
     assert int(status.abs().sum()) == 0
 
 
-@pytest.mark.parametrize("s,hq,hkv,split", [(512, 4, 1, True), (2304, 32, 8, False)])
+@pytest.mark.parametrize("s,hq,hkv,split", [(1024, 4, 1, True), (2304, 32, 8, False)])
 def test_ring_on_one_real_rank_takes_either_kernel(native_lib, s, hq, hkv, split):
     """One rank of a real context: few query tiles go to the split-key kernel, more tile pairs than SMs
     to the tile-pair kernel, persistent since there is nothing to pull.  Both masks in turn on one object;

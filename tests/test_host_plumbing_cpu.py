@@ -273,3 +273,13 @@ def test_split_attention_workspace_does_not_grow_with_the_batch(native_lib, shap
     B, Sq, Skv, Hq, Hkv = shape
     nbytes = native_lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, Skv - Sq, 0, 1)
     assert 0 <= nbytes <= 2 * 148 * 128 * 520
+
+
+@pytest.mark.parametrize("shape,cut", [((1, 300, 300, 4, 1), None), ((2, 1, 700, 8, 1), False),
+                                       ((1, 1, 16384, 8, 8), True), ((1, 64, 64, 4, 4), False)])
+def test_attention_is_not_cut_where_the_host_bounds_the_call(native_lib, shape, cut):
+    """A cut costs a workspace and a second launch on the host: a call of about that length is left to the
+    tile-pair kernel (None) or to whole items."""
+    B, Sq, Skv, Hq, Hkv = shape
+    nbytes = native_lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, Skv - Sq, 0, 1)
+    assert (nbytes == -1) if cut is None else (nbytes > 0) == cut and nbytes >= 0
