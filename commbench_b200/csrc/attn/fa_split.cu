@@ -618,8 +618,9 @@ static int split_sms() {
 // of them; the split kernel takes SP_BLOCK_US for a unit of its 128 rows, plus the merge.
 // Measured on the device, split / pair (B, Sq, Skv, Hq, Hkv): (1, 64, 64, 4, 4) 7.6 / 9.0 us,
 // (1, 300, 300, 4, 1) 11 / 14 (with a merge, so a call takes 21.5 / 16.5), (1, 500, 4596, 8, 2)
-// 23 / 81, (1, 8192, 8192, 4, 4) 90 / 127; near the line (1, 1280, 1280, 16, 8) 33 / 30, (1, 2000, 2777, 16, 4) 54 / 51, (1, 1000, 7000, 32, 8) 118 / 112;
-// beyond it (2, 2000, 2000, 32, 8) 125 / 88.
+// 23 / 81, (1, 8192, 8192, 4, 4) 90 / 127; near the line (1, 1280, 1280, 16, 8) 33 / 30,
+// (1, 2000, 2777, 16, 4) 54 / 51, (1, 1000, 7000, 32, 8) 118 / 112; beyond it (2, 2000, 2000, 32, 8)
+// 125 / 88.
 static bool split_wins(const SplitPlan& pl, int sms) {
   constexpr float kPairBlock = 2.0f, kPairStart = 7.f;
   const float pair_tiles = static_cast<float>((pl.Sq + 2 * CP_BM - 1) / (2 * CP_BM));
