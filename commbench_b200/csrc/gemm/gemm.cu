@@ -63,6 +63,7 @@ int make_tmap_2d(CUtensorMap* out, const void* base, TmapDtype dt, unsigned long
 
 struct PlainParams {
   CUtensorMap tm_a, tm_b, tm_c;
+  CUtensorMap tm_c_half;   // 32-column boxes, for tile widths that are no multiple of 64
   GemmShape g;
   uint32_t* status;
   int raster_group;
@@ -86,6 +87,10 @@ struct PlainPolicy {
   __device__ static void store_box(const P& p, int m_blk, int n_blk, int row, int col,
                                    const void* smem_box) {
     tma_store_2d(&p.tm_c, smem_box, n_blk * Cfg::BN + col, m_blk * Cfg::BM + row);
+  }
+  __device__ static void store_half_box(const P& p, int m_blk, int n_blk, int row, int col,
+                                        const void* smem_box) {
+    tma_store_2d(&p.tm_c_half, smem_box, n_blk * Cfg::BN + col, m_blk * Cfg::BM + row);
   }
   __device__ static void tile_done(const P&, int, int, int) {}
 };
@@ -124,6 +129,10 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
   if (make_tmap_2d(&p.tm_c, c, TMAP_BF16, N, M, (unsigned long long)N * 2, Cfg::EPI_COLS, 32,
                    true))
     return -1;
+  if constexpr (Cfg::BN % Cfg::EPI_COLS != 0) {
+    if (make_tmap_2d(&p.tm_c_half, c, TMAP_BF16, N, M, (unsigned long long)N * 2, 32, 32, false))
+      return -1;
+  }
   p.g.M = M;
   p.g.N = N;
   p.g.K = K;
@@ -178,6 +187,19 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
   return 0;
 }
 
+// A narrower tile of a CTA pair is worth it where it fills the last wave: 8192 x 3584 x 8192 is 448 tiles of
+// 256 x 256 on 74 pairs, 7 waves for 6.05, and 512 of 256 x 224, 6.92.  All pairs together are bound by what
+// they draw out of L2, so a tile's time falls by less than its width; the cost below puts the line between 256
+// and 224 (192 and 224 with hardware block scales) where it was measured, 256 / 224 wide in us: the shape
+// above bf16 339 / 328, fp8 169 / 164 (192 / 224 with block scales: 185 / 173); 3000 x 8192 x 3584 124 / 119,
+// 67 / 65; 4096 x 7168 x 2048 with block scales 57 / 53; the other way 8192 x 8192 x 4096 353 / 361, 185 / 190,
+// 2048 x 4096 x 4096 with block scales 36 / 40.
+// Calls in a row, under the power cap: the shape above fp8 199.6 -> 191.5 us, with block scales 213.8 -> 202.
+static float pair_tile_cost(int bn) { return static_cast<float>(bn + 512); }
+static long long pair_waves(long long m256, int N, int bn, int sms) {
+  return (m256 * ((N + bn - 1) / bn) + sms / 2 - 1) / (sms / 2);
+}
+
 // Which kernel and tile a GEMM runs on, by a model of its time in microseconds.  kbytes: bytes of one
 // K row (K x element size).  Per-128-byte-K-block times of a CTA that nothing else holds up, measured on
 // one m-block: persistent pairs on 256 x 256 tiles 0.30, single CTAs 0.36, the small kernel's 64 / 128 /
@@ -205,14 +227,20 @@ static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
       best = {bn, split};
     }
   };
-  {  // persistent kernels: pairs on 256 x 256, single CTAs on 128 x 256
-    const long long pairs = m256 * ((N + 255) / 256), singles = m128 * ((N + 255) / 256);
-    const long long pw = (pairs + sms / 2 - 1) / (sms / 2), sw = (singles + sms - 1) / sms;
-    const float pair_ctas = 2.f * static_cast<float>(pairs < sms / 2 ? pairs : sms / 2);
+  {  // persistent kernels: pairs on 256 x 256 and 256 x 224, single CTAs on 128 x 256
+    // (224 from 32 K blocks on: in short loops the epilogue counts, which gains nothing)
+    for (int bn = 256; bn >= (nkb >= 32.f ? 224 : 256); bn -= 32) {
+      const long long pairs = m256 * ((N + bn - 1) / bn);
+      const float pair_ctas = 2.f * static_cast<float>(pairs < sms / 2 ? pairs : sms / 2);
+      const float cta_bytes = static_cast<float>(128 + bn / 2) * 128.f;   // per CTA and K block
+      const float pair_kb =
+          fmaxf(0.30f * pair_tile_cost(bn) / pair_tile_cost(256), pair_ctas * cta_bytes / l2_rate);
+      const float waves = static_cast<float>(pair_waves(m256, N, bn, sms));
+      offer(2 * bn, 0, 7.f + fmaxf(waves * fmaxf(nkb * pair_kb, 2.5f), hbm_us));
+    }
+    const long long singles = m128 * ((N + 255) / 256), sw = (singles + sms - 1) / sms;
     const float single_ctas = static_cast<float>(singles < sms ? singles : sms);
-    const float pair_kb = fmaxf(0.30f, pair_ctas * 32768.f / l2_rate);
     const float single_kb = fmaxf(0.36f, single_ctas * 49152.f / l2_rate);
-    offer(512, 0, 7.f + fmaxf(static_cast<float>(pw) * fmaxf(nkb * pair_kb, 2.5f), hbm_us));
     offer(256, 0, 6.5f + fmaxf(static_cast<float>(sw) * fmaxf(nkb * single_kb, 2.5f), hbm_us));
   }
   const int a_rows = M < 128 ? (M + 7) / 8 * 8 : 128;
@@ -319,7 +347,8 @@ extern "C" {
 
 // bf16: A [M,K], B [N,K], C [M,N], all row-major and 16-byte aligned; K % 8 == 0, N % 8 == 0.
 // `bn` picks the tile: 256, 128 or 64 = one CTA per 128 x bn tile; 512 = a CTA pair per
-// 256 x 256 tile, 384 = a pair per 256 x 128 tile; 0 = choose from the shape.
+// 256 x 256 tile, 448 = a pair per 256 x 224 tile, 384 = a pair per 256 x 128 tile; 0 = choose
+// from the shape.
 // `status` may be null.  Returns 0 or -1 (cb_last_error()).
 int cb_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, float alpha, int bn,
                  int max_ctas, void* status, void* stream) {
@@ -338,6 +367,8 @@ int cb_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, flo
   switch (bn) {
     case 512:
       return launch_plain<GemmCfg<256, 6, false, 2>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
+    case 448:
+      return launch_plain<GemmCfg<224, 6, false, 2>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
     case 384:
       return launch_plain<GemmCfg<128, 8, false, 2>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
     case 256:
@@ -347,7 +378,7 @@ int cb_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, flo
     case 64:
       return launch_plain<GemmCfg<64, 8, false>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
     default:
-      set_last_error("cb_gemm_bf16: bn must be 0, 64, 128, 256, 384 or 512");
+      set_last_error("cb_gemm_bf16: bn must be 0, 64, 128, 256, 384, 448 or 512");
       return -1;
   }
 }
@@ -407,6 +438,8 @@ int cb_gemm_fp8(const void* a, const void* b, void* c, int M, int N, int K, floa
   switch (bn) {
     case 512:
       return launch_plain<GemmCfg<256, 6, true, 2>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
+    case 448:
+      return launch_plain<GemmCfg<224, 6, true, 2>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
     case 256:
       return launch_plain<GemmCfg<256, 4, true>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
     case 128:
@@ -414,7 +447,7 @@ int cb_gemm_fp8(const void* a, const void* b, void* c, int M, int N, int K, floa
     case 64:
       return launch_plain<GemmCfg<64, 8, true>>(a, b, c, M, N, K, alpha, s, max_ctas, st);
     default:
-      set_last_error("cb_gemm_fp8: bn must be 0, 64, 128, 256 or 512");
+      set_last_error("cb_gemm_fp8: bn must be 0, 64, 128, 256, 448 or 512");
       return -1;
   }
 }
@@ -474,6 +507,14 @@ int cb_gemm_fp8_mx_traced(const void* a, const void* sfa, const void* b, const v
         a, b, c, M, N, K, alpha, static_cast<uint32_t*>(status), max_ctas,
         static_cast<cudaStream_t>(stream), static_cast<unsigned long long*>(trace), nullptr,
         nullptr, static_cast<const uint32_t*>(sfa), static_cast<const uint32_t*>(sfb));
+  const int sms = max_ctas > 1 && max_ctas < sm_count() ? max_ctas : sm_count();
+  const long long m256 = (M + 255) / 256;
+  if (static_cast<float>(pair_waves(m256, N, 224, sms)) * pair_tile_cost(224) <
+      static_cast<float>(pair_waves(m256, N, 192, sms)) * pair_tile_cost(192))
+    return launch_plain<GemmCfg<224, 6, true, 2, false, true>>(
+        a, b, c, M, N, K, alpha, static_cast<uint32_t*>(status), max_ctas,
+        static_cast<cudaStream_t>(stream), static_cast<unsigned long long*>(trace), nullptr, nullptr,
+        static_cast<const uint32_t*>(sfa), static_cast<const uint32_t*>(sfb));
   return launch_plain<GemmCfg<192, 6, true, 2, false, true>>(
       a, b, c, M, N, K, alpha, static_cast<uint32_t*>(status), max_ctas,
       static_cast<cudaStream_t>(stream), static_cast<unsigned long long*>(trace), nullptr, nullptr,

@@ -55,7 +55,7 @@
 // packed words serve as they are, every step of K block j selecting byte j.  Four scale warps fetch
 // the words of the next groups of four K blocks and lay them out in shared memory; the MMA thread
 // copies a group into its scale-factor columns (tcgen05.cp) once, before its first MMA.  Tiles are
-// 192 columns wide so that two accumulators and the scale columns fit in the 512 columns.
+// 192 or 224 columns wide, so that two accumulators and the scale columns fit in the 512 columns.
 //
 // No load in this file is a cluster-multicast load.  Every wait is bounded: on a
 // time-out the CTA raises its abort word (and its partner's), every role leaves
@@ -97,7 +97,7 @@ struct GemmCfg {
   static constexpr int SF_GROUP_BYTES = MX_ ? 3 * 512 : 0;   // A rows, B rows 0..127, B rows 128..255
   static constexpr int SF_BYTES = SF_GROUPS * SF_GROUP_BYTES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + SF_BYTES + 1024;
-  static constexpr int TMEM_COLS = MX_ ? 512 : 2 * BN;
+  static constexpr int TMEM_COLS = MX_ || BN > 128 ? 512 : 2 * BN;
   // Warp roles.  Plain: producer, MMA, 4 epilogue warps, signal warp.  Block-scaled: a
   // utility warp-group (producer, MMA, signal, one idle warp) that gives registers away and
   // two epilogue warp-groups that take them (setmaxnreg works on whole warp-groups).
@@ -105,13 +105,13 @@ struct GemmCfg {
   static constexpr int SIGNAL_WARP = BS_ ? 2 : 6;
   static constexpr int SCALE_WARP0 = 8;       // MX: warps 8..11 stage scale factors
   static constexpr int THREADS = (BS_ || MX_) ? 384 : 224;
-  static_assert(!MX_ || (FP8_ && !BS_ && BN_ <= 192 &&
-                         2 * BN_ + 4 * SF_STRIDE <= 512),
+  static_assert(!MX_ || (FP8_ && !BS_ && 2 * BN_ + 4 * SF_STRIDE <= 512),
                 "hardware block scales: fp8, accumulators + scale slots within 512 TMEM columns");
   static_assert(!BS_ || (FP8_ && BN_ == 256 && PAIR_ == 1),
                 "block scales: fp8 operands, 256-column tiles, one CTA per tile");
   static_assert(PAIR_ == 1 || PAIR_ == 2, "one CTA or a pair per tile");
-  static_assert(BN % 64 == 0 && BN >= 64 && BN <= 256, "BN in {64,128,192,256}");
+  static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "BN in {64,96,...,256}");
+  static_assert(B_BYTES % 1024 == 0, "ring slots start on swizzle atoms");
   static_assert((TMEM_COLS & (TMEM_COLS - 1)) == 0 && TMEM_COLS >= 32 && TMEM_COLS <= 512,
                 "TMEM columns must be a power of two");
   static_assert(SMEM_BYTES <= 232448, "over the 227 KB shared-memory limit");
@@ -194,6 +194,8 @@ struct GemmCtl {
 //   void store_box(const P&, int m_blk, int n_blk, int row_in_tile, int col_in_tile,
 //                  const void* smem_box)       issued by one lane; must issue exactly one
 //                                              bulk-group worth of stores (commit is done here)
+//   store_half_box                             the same for the last 32 columns of a tile whose width is
+//                                              no multiple of 64 (unswizzled 32 x 64 B box)
 //   void direct_targets(const P&, int m_blk, int n_blk, DirectTargets*)
 //   int  b_row(const P&, int m_blk, int n_blk)  row coordinate of the B tile in map_b
 //   direct policies also: kSignalPerTile (signal warp raises a flag per tile) and
@@ -645,6 +647,22 @@ __device__ __forceinline__ void epi_write_row_swizzled(uint8_t* buf, uint32_t la
   }
 }
 
+// fp32 accumulator row (32 columns) -> bf16 in a plain [32 rows][64 B] buffer.
+__device__ __forceinline__ void epi_write_row_32(uint8_t* buf, uint32_t lane, const uint32_t (&r)[32],
+                                                 float alpha) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[c * 8 + j * 2]) * alpha,
+                                               __uint_as_float(r[c * 8 + j * 2 + 1]) * alpha);
+      w[j] = *reinterpret_cast<uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(buf + lane * 64u + c * 16u) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 // Where a "direct" policy wants a finished tile: up to 8 destinations (peer or
 // local global memory) that all receive the same data with plain 16-byte stores.
 struct DirectTargets {
@@ -961,7 +979,10 @@ __device__ __forceinline__ void gemm_epilogue_tma(const P& p, const GemmShape& g
       return;
     tc_fence_after_sync();
     constexpr bool kGated = policy_gated<Policy>();
-    constexpr int kBoxes = Cfg::BN / Cfg::EPI_COLS / (kGated ? 2 : 1);  // store boxes per tile
+    constexpr int kBoxes =                                              // store boxes per tile
+        (Cfg::BN + Cfg::EPI_COLS - 1) / Cfg::EPI_COLS / (kGated ? 2 : 1);
+    constexpr bool kHalfBox = Cfg::BN % Cfg::EPI_COLS != 0;             // the last one 32 columns wide
+    static_assert(!kGated || Cfg::BN % (2 * Cfg::EPI_COLS) == 0, "whole boxes of gate and up columns");
 #pragma unroll 1
     for (int c = 0; c < kBoxes; ++c) {
       const uint32_t taddr = tmem_base + ((q * 32u) << 16) + acc * Cfg::BN + c * Cfg::EPI_COLS;
@@ -978,7 +999,7 @@ __device__ __forceinline__ void gemm_epilogue_tma(const P& p, const GemmShape& g
         epi_gate_32(r1, up, g.alpha);
       } else {
         tmem_ld_32x32(taddr, r0);
-        tmem_ld_32x32(taddr + 32u, r1);
+        if (!kHalfBox || c < kBoxes - 1) tmem_ld_32x32(taddr + 32u, r1);
         tmem_wait_ld();
       }
       if (c == kBoxes - 1) {
@@ -991,12 +1012,22 @@ __device__ __forceinline__ void gemm_epilogue_tma(const P& p, const GemmShape& g
       if (lane == 0) bulk_wait_read<1>();
       __syncwarp();
       uint8_t* b = bufs + buf * Cfg::EPI_BUF_BYTES;
-      epi_write_row_swizzled(b, lane, r0, r1, kGated ? 1.0f : g.alpha);
+      if constexpr (kHalfBox) {
+        if (c == kBoxes - 1) epi_write_row_32(b, lane, r0, g.alpha);
+        else epi_write_row_swizzled(b, lane, r0, r1, g.alpha);
+      } else {
+        epi_write_row_swizzled(b, lane, r0, r1, kGated ? 1.0f : g.alpha);
+      }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        Policy::store_box(p, m_blk, n_blk, sub * Cfg::CTA_M + static_cast<int>(q * 32u),
-                          c * Cfg::EPI_COLS, b);
+        const int row = sub * Cfg::CTA_M + static_cast<int>(q * 32u);
+        if constexpr (kHalfBox) {
+          if (c == kBoxes - 1) Policy::store_half_box(p, m_blk, n_blk, row, c * Cfg::EPI_COLS, b);
+          else Policy::store_box(p, m_blk, n_blk, row, c * Cfg::EPI_COLS, b);
+        } else {
+          Policy::store_box(p, m_blk, n_blk, row, c * Cfg::EPI_COLS, b);
+        }
         bulk_commit();
       }
       buf ^= 1u;

@@ -155,7 +155,7 @@ def gemm_fp8_mx(a_q, a_sf, b_q, b_sf, out=None, alpha: float = 1.0, pair: bool =
             N.new_empty_on(stream, a_q, (M, Nn), torch.bfloat16)
     else:
         _check(out, "out")
-    # pair: a CTA pair per 256 x 192 tile (default, fastest); otherwise one CTA per 128 x 192
+    # pair: a CTA pair per 256 x 192 or 256 x 224 tile (default, fastest); otherwise one CTA per 128 x 192
     rc = lib.cb_gemm_fp8_mx(a_q.data_ptr(), a_sf.data_ptr(), b_q.data_ptr(), b_sf.data_ptr(),
                             out.data_ptr(), M, Nn, K, alpha, 0 if pair else -1, status_ptr,
                             N.raw_stream(stream))

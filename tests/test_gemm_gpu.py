@@ -373,3 +373,42 @@ def test_split_k_gemm_in_a_cuda_graph(native_lib, m):
         x.copy_(torch.randn(m, 2048, device="cuda", generator=torch.Generator("cuda").manual_seed(seed)))
         graph.replay()
         assert torch.equal(y, gemm(gemm(x, w1), w2))
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("shape", [(1, 8, 64), (256, 224, 128), (257, 216, 192), (300, 232, 320),
+                                   (513, 904, 512), (700, 1112, 1040)])
+def test_gemm_pair_tiles_224_wide_exact_on_small_ints(native_lib, shape, fp8):
+    """256 x 224 tiles: three store boxes of 64 columns and one of 32 per row group; widths that end in
+    each of them, row counts around the tile height."""
+    from commbench_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randint(-3, 4, (M, K), device="cuda", generator=g).float()
+    b = torch.randint(-3, 4, (N, K), device="cuda", generator=g).float()
+    dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
+    guard = torch.full((M + 2, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = guard[1:M + 1]
+    gemm(a.to(dt), b.to(dt), out=out, bn=448)
+    # |sums| < 9 * 1040 are exact in fp32; the result is their rounding to bf16
+    assert torch.equal(out.float(), _ref(a, b).bfloat16().float())
+    assert bool((guard[0] == 7).all()) and bool((guard[M + 1] == 7).all())
+
+
+@pytest.mark.parametrize("n", [3584, 3568, 3544, 3400])
+def test_fp8_gemm_with_hardware_block_scales_224_wide(native_lib, n):
+    """Shapes at which 256 x 224 tiles take fewer waves than 256 x 192, the last column tile whole,
+    ending inside its half box, inside a whole box, and nearly empty."""
+    from commbench_b200.ops.gemm import gemm_fp8_mx, quantize_blockscaled_pow2
+
+    M, K = 8100, 640
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.randn(M, K, device="cuda", generator=g) * (1.0 + (torch.arange(M, device="cuda") % 7))[:, None]
+    b = torch.randn(n, K, device="cuda", generator=g) * 0.02 * (1 + torch.arange(n, device="cuda") // 128)[:, None]
+    aq, as_, asf = quantize_blockscaled_pow2(a.bfloat16().contiguous(), 1)
+    bq, bs, bsf = quantize_blockscaled_pow2(b.bfloat16().contiguous(), 128)
+    out = gemm_fp8_mx(aq, asf, bq, bsf)
+    _check(out, _bs_reference(aq, as_, bq, bs), 1e-2)
+    # the same K order on one CTA per 128 x 192 tile: the same bits
+    assert torch.equal(out, gemm_fp8_mx(aq, asf, bq, bsf, pair=False))
