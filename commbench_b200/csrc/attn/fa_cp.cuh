@@ -15,7 +15,7 @@
 //     TMA loads and whose O rows are stored straight into their owners' output tensors;
 //   * registers are moved from the four utility warps (producer, MMA issuer, two idle) to
 //     the eight softmax warps with setmaxnreg (72 / 216 per thread), which keeps a 128-column row
-//     of scores in registers (three of them spilled), and every `kPoly`-th pair of exponentials is
+//     of scores in registers, and every `kPoly`-th pair of exponentials is
 //     computed on the FMA pipe (a cubic after a round-to-nearest split) instead of the SFU,
 //     which otherwise is as busy as the tensor pipe;
 //   * CTAs draw tickets: the first `num_comm` tickets copy the list of 2-D pieces
@@ -27,9 +27,16 @@
 //     and drain cost 8 to 15 us an item: 16384 tokens, 32 / 8 heads, causal 2231 us, 2040 so).
 //     Items go to whatever SM is free: with two SMs held by a kernel of another stream the same call
 //     takes 5 % more (16: 16 %), where a fixed share of the items per CTA took twice as long.
-// What bounds the inner loop (3500 cycles for 128 keys x 256 rows against 2048 on the tensor cores): the
-// MMA warp's issue, 32 MMAs at about 75 cycles, and behind it a tile's chain scores -> softmax (1700) ->
-// P -> product -> next scores; the exponentials alone are not (without them: the same time).
+//   * P is handed over in two halves of 64 keys: the product with the first runs while the exponentials of
+//     the second are taken.  16384 tokens, 32 / 8 heads, causal: 1790 -> 1705 us in a burst (1965 MHz), 2050 ->
+//     1965 us when such calls follow each other (1.6 GHz under the power cap).
+// What bounds the inner loop (3400 cycles for 128 keys x 256 rows against 2048 on the tensor cores): the MMA
+// warp, which is issuing for 3000 of them - 60 cycles for a product's MMA, about 115 for one of the scores,
+// whose two operands both come from shared memory, beside the 64 KB that arrive per block - and behind it a
+// tile's chain scores -> softmax (1700) -> P -> product -> next scores; without the exponentials 1670 us.
+// Slower: CTA pairs, which halve the shared-memory traffic of K and V (1807 us: a pair's MMAs start too late
+// after each hand-over), three quarters of P first (1757), the loads of the scores in halves beside the
+// maximum, asking for K and V before P (1700 to 1720).
 // No CTA waits for another GPU inside this kernel: remote data is pulled, and the cross-GPU
 // barriers that say "shards are published" / "shards may be overwritten" bracket the launch.
 //
@@ -53,7 +60,7 @@ struct CpCtl {
   uint64_t q_full, q_empty;
   uint64_t k_full[CP_KST], k_empty[CP_KST];
   uint64_t v_full[CP_VST], v_empty[CP_VST];
-  uint64_t s_full[2], p_full[2], pv_done[2];  // per query tile
+  uint64_t s_full[2], p_first[2], p_rest[2], pv_done[2];  // per query tile
   uint64_t item_full, item_empty;             // the answer to the CTA's request for its next item
   uint4 item_answer;
   uint32_t tmem_base;
@@ -104,18 +111,9 @@ __device__ __forceinline__ void cp_mask_tail(uint32_t (&s)[128], int visible) {
   for (int i = 0; i < 128; ++i) s[i] = i < visible ? s[i] : 0xff800000u;
 }
 
-// One block of the online softmax: the 128 masked scores of this thread's row in `s` become the
-// bf16 probabilities s[0..63]; m_ref (log2 units) and l are the running reference maximum and sum.
-// The accumulator in tensor memory at `tO` is rescaled when the maximum has grown by more than
-// CP_RESCALE_THRESHOLD in any row of the warp that `votes` (`rescale_o`: it holds something already).
-// A row that was not loaded must not vote: its scores come from whatever was in shared memory, and when
-// the other rows are rescaled decides how they are rounded.
-// kPoly: see fa_cp_kernel.  Warp-collective.
-template <int kPoly>
-__device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t tO, float scale_log2,
-                                                  bool need_mask, bool rescale_o, bool votes,
-                                                  float& m_ref, float& l) {
-  float mx8[8];
+// The online softmax of one block, in the order of use.  cp_row_max: the maximum of the 128 masked scores of
+// this thread's row, as eight partial ones.
+__device__ __forceinline__ void cp_row_max(const uint32_t (&s)[128], float (&mx8)[8]) {
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     mx8[i] = fmaxf(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]));
@@ -123,6 +121,15 @@ __device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t t
   for (int i = 16; i < 128; i += 2)
     mx8[(i >> 1) & 7] =
         cp_max3(mx8[(i >> 1) & 7], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+}
+
+// Running reference maximum m_ref (log2 units) and sum l of the row.  The accumulator in tensor memory at
+// `tO` is rescaled when the maximum has grown by more than CP_RESCALE_THRESHOLD in any row of the warp that
+// `votes` (`rescale_o`: it holds something already).
+// A row that was not loaded must not vote: its scores come from whatever was in shared memory, and when
+// the other rows are rescaled decides how they are rounded.  Warp-collective.
+__device__ __forceinline__ void cp_update_max(const float (&mx8)[8], uint32_t tO, float scale_log2,
+                                              bool rescale_o, bool votes, float& m_ref, float& l) {
   const float mx_all =
       cp_max3(fmaxf(cp_max3(mx8[0], mx8[1], mx8[2]), cp_max3(mx8[3], mx8[4], mx8[5])),
               mx8[6], mx8[7]);
@@ -148,13 +155,19 @@ __device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t t
       }
     }
   }
+}
+
+// The scores FROM ... TO-1 become bf16 probabilities, two to a word, in s[FROM / 2 ... TO / 2 - 1], their sums
+// are added to sum4.  kPoly: see fa_cp_kernel.
+template <int kPoly, int FROM, int TO>
+__device__ __forceinline__ void cp_probabilities(uint32_t (&s)[128], float scale_log2, float m_ref,
+                                                 bool need_mask, uint64_t (&sum4)[4]) {
   const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
   const uint64_t scale2 = cp_pack(scale_log2, scale_log2), negm2 = cp_pack(-m_use, -m_use);
-  uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
   // The bf16 pairs go back into s[0..63]: element i is only written after s[2i], s[2i+1]
   // have been consumed.
 #pragma unroll
-  for (int i = 0; i < 128; i += 2) {
+  for (int i = FROM; i < TO; i += 2) {
     const uint64_t y = cp_fma2(cp_pack_u(s[i], s[i + 1]), scale2, negm2);
     float p0, p1;
     if (kPoly > 0 && !need_mask && ((i >> 1) % (kPoly > 0 ? kPoly : 1)) == kPoly - 1) {
@@ -181,10 +194,23 @@ __device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t t
     __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
     s[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
   }
-  {
-    const uint64_t a = cp_add2(cp_add2(sum4[0], sum4[1]), cp_add2(sum4[2], sum4[3]));
-    l += __uint_as_float(static_cast<uint32_t>(a)) + __uint_as_float(static_cast<uint32_t>(a >> 32));
-  }
+}
+__device__ __forceinline__ void cp_add_sums(const uint64_t (&sum4)[4], float& l) {
+  const uint64_t a = cp_add2(cp_add2(sum4[0], sum4[1]), cp_add2(sum4[2], sum4[3]));
+  l += __uint_as_float(static_cast<uint32_t>(a)) + __uint_as_float(static_cast<uint32_t>(a >> 32));
+}
+
+// All of it on a row that is complete.  Warp-collective.
+template <int kPoly>
+__device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t tO, float scale_log2,
+                                                  bool need_mask, bool rescale_o, bool votes,
+                                                  float& m_ref, float& l) {
+  float mx8[8];
+  cp_row_max(s, mx8);
+  cp_update_max(mx8, tO, scale_log2, rescale_o, votes, m_ref, l);
+  uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
+  cp_probabilities<kPoly, 0, 128>(s, scale_log2, m_ref, need_mask, sum4);
+  cp_add_sums(sum4, l);
 }
 
 // Walks the key blocks that a query tile pair attends to, segment by segment.  Every role of a
@@ -392,7 +418,8 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
       }
       for (int i = 0; i < 2; ++i) {
         mbar_init(&ctl.s_full[i], 1);
-        mbar_init(&ctl.p_full[i], 4);
+        mbar_init(&ctl.p_first[i], 4);
+        mbar_init(&ctl.p_rest[i], 4);
         mbar_init(&ctl.pv_done[i], 1);
       }
       ctl.abort_flag = 0;
@@ -542,16 +569,26 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
           // The first product of an item overwrites the O of the last one, which the softmax warps
           // have read before they hand over the item's first block.
           const int g = g0 + j, s = g % CP_VST;
-          if (!wait_all(&ctl.p_full[t], g & 1, 0xE20 + t)) return false;
-          if (!wait_all(&ctl.v_full[s], (g / CP_VST) & 1, 0xE22)) return false;
+          if (!wait_all(&ctl.p_first[t], g & 1, 0xE20 + 2 * t)) return false;
+          if (!wait_all(&ctl.v_full[s], (g / CP_VST) & 1, 0xE24)) return false;
           tc_fence_after_sync();
           if (elect_one()) {
             const uint64_t va = v_desc0 + s * kTileStep;
             const uint32_t d = tmem_u + 256u * t + 128u;
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
+            for (int kk = 0; kk < 4; ++kk)
               mma_bf16_ts(d, tmem_u + 256u * t + 8u * kk, va + kk * (2048u >> 4), idesc_pv,
                           (j > 0 || kk > 0) ? 1u : 0u);
+          }
+          __syncwarp();
+          if (!wait_all(&ctl.p_rest[t], g & 1, 0xE21 + 2 * t)) return false;
+          tc_fence_after_sync();
+          if (elect_one()) {
+            const uint64_t va = v_desc0 + s * kTileStep;
+            const uint32_t d = tmem_u + 256u * t + 128u;
+#pragma unroll
+            for (int kk = 4; kk < 8; ++kk)
+              mma_bf16_ts(d, tmem_u + 256u * t + 8u * kk, va + kk * (2048u >> 4), idesc_pv, 1u);
             mma_commit(&ctl.pv_done[t]);
           }
           __syncwarp();
@@ -613,27 +650,37 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
             break;
           }
           tc_fence_after_sync();
+          const CpSeg& g = p.seg[it.seg];
+          const int key0 = g.kpos0 + it.i * CP_BN;
+          const int kv_left = g.nkeys - it.i * CP_BN;
+          const bool need_mask = kv_left < CP_BN || (p.causal && key0 + CP_BN - 1 > tile_first);
+          it.next(p, w.q_last);
           uint32_t s[128];
           tmem_ld_32x32_at(tS, &s[0]);
           tmem_ld_32x32_at(tS + 32u, &s[32]);
           tmem_ld_32x32_at(tS + 64u, &s[64]);
           tmem_ld_32x32_at(tS + 96u, &s[96]);
           tmem_wait_ld();
-
-          const CpSeg& g = p.seg[it.seg];
-          const int key0 = g.kpos0 + it.i * CP_BN;
-          const int kv_left = g.nkeys - it.i * CP_BN;
-          const bool need_mask = kv_left < CP_BN || (p.causal && key0 + CP_BN - 1 > tile_first);
-          it.next(p, w.q_last);
           if (need_mask) cp_mask_tail(s, p.causal ? min(kv_left, q_pos - key0 + 1) : kv_left);
-          cp_online_softmax<kPoly>(s, tO, p.scale_log2, need_mask, j > 0, true, m_ref, l);
-          // P_t(j): row r = lane r, keys 2c and 2c+1 in column c.
+          float mx8[8];
+          cp_row_max(s, mx8);
+          cp_update_max(mx8, tO, p.scale_log2, j > 0, true, m_ref, l);
+          // P_t(j): row r = lane r, keys 2c and 2c+1 in column c.  The product with the first 64 keys runs
+          // while the others' exponentials are taken.
+          uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
+          cp_probabilities<kPoly, 0, 64>(s, p.scale_log2, m_ref, need_mask, sum4);
           tmem_st_32x32_at(tS, &s[0]);
+          tmem_wait_st();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.p_first[t]);
+          cp_probabilities<kPoly, 64, 128>(s, p.scale_log2, m_ref, need_mask, sum4);
           tmem_st_32x32_at(tS + 32u, &s[32]);
           tmem_wait_st();
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl.p_full[t]);
+          if (lane == 0) mbar_arrive(&ctl.p_rest[t]);
+          cp_add_sums(sum4, l);
         }
         // ------------------------------------------------------------------ epilogue
         if (ok && w.nblk > 0)
