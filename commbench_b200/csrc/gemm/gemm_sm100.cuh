@@ -66,6 +66,7 @@
 #include <cuda_bf16.h>
 
 #include "../prim/cluster.cuh"
+#include "../prim/pdl.cuh"
 #include "../prim/tcgen05.cuh"
 #include "../prim/tma.cuh"
 
@@ -204,6 +205,20 @@ struct GemmCtl {
 //                                              were issued (one lane); quadrant = 4 * (CTA of
 //                                              the pair) + epilogue warp, or 4 * CTA from the
 //                                              signal warp of a direct policy
+//   optional: int a_rows32(const P&, int m_blk), const CUtensorMap* map_a32(const P&)   (one CTA per tile) the
+//                                              tile has rows in its first 32 a_rows32 only, which are
+//                                              loaded in boxes of 32; the others are whatever the ring holds
+//   optional: static constexpr bool kPdl       launched with programmatic dependent launch: after set-up,
+//                                              wait for the kernels before
+template <class Policy>
+__host__ __device__ constexpr bool policy_pdl() {
+  if constexpr (requires { Policy::kPdl; }) {
+    return Policy::kPdl;
+  } else {
+    return false;
+  }
+}
+
 // Producer and MMA roles are executed by a whole, converged warp: every lane follows the loop
 // and the waits, one elected lane issues the TMA loads / MMAs / commits.  Measured on B200
 // with back-to-back MMAs of 32 pipe cycles each: 43-49 cycles per instruction issued this way
@@ -241,6 +256,9 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
     }
     const CUtensorMap* ma = Policy::map_a(p, m_blk);
     const CUtensorMap* mb = Policy::map_b(p);
+    constexpr bool kRagged = Cfg::PAIR == 1 && requires { Policy::a_rows32(p, m_blk); };
+    [[maybe_unused]] int a32 = 4;
+    if constexpr (kRagged) a32 = Policy::a_rows32(p, m_blk);
     const int arow = Policy::a_row(p, m_blk) + sub * Cfg::CTA_M;
     const int brow = Policy::b_row(p, m_blk, n_blk) + sub * Cfg::B_ROWS;
     for (int kb = 0; kb < g.num_k_blocks; ++kb) {
@@ -259,9 +277,20 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
           tma_load_2d_pair(sb, mb, kb * Cfg::BK, brow, bar);
         } else {
           const uint32_t bar = full0 + stage * 8u;
-          mbar_arrive_expect_tx_addr(bar, Cfg::STAGE_BYTES);
-          tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
-          tma_load_2d_addr(sb, mb, kb * Cfg::BK, brow, bar);
+          if constexpr (kRagged) {
+            mbar_arrive_expect_tx_addr(bar, Cfg::B_BYTES + a32 * 4096);
+            tma_load_2d_addr(sb, mb, kb * Cfg::BK, brow, bar);
+            if (a32 == 4) {
+              tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
+            } else {
+              for (int i = 0; i < a32; ++i)
+                tma_load_2d_addr(sa + i * 4096, Policy::map_a32(p), kb * Cfg::BK, arow + i * 32, bar);
+            }
+          } else {
+            mbar_arrive_expect_tx_addr(bar, Cfg::STAGE_BYTES);
+            tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
+            tma_load_2d_addr(sb, mb, kb * Cfg::BK, brow, bar);
+          }
         }
       }
       __syncwarp();
@@ -933,8 +962,8 @@ __device__ __forceinline__ void gemm_signal(const P& p, GemmCtl<Cfg::STAGES>* ct
   }
 }
 
-// A policy may declare `static constexpr bool kGated = true`: every BN-wide accumulator tile then
-// holds BN/2 "gate" columns followed by BN/2 "up" columns of the same output columns (the
+// A policy may declare `static constexpr bool kGated = true`: every 128 columns of an accumulator tile
+// then hold 64 "gate" columns followed by the 64 "up" columns of the same outputs (the
 // weight rows are interleaved that way by the caller), and the TMA-store epilogue writes
 // silu(gate) * up - BN/2 output columns per tile - instead of the raw accumulator, so the
 // activation never makes a round trip through HBM.
@@ -985,16 +1014,17 @@ __device__ __forceinline__ void gemm_epilogue_tma(const P& p, const GemmShape& g
     static_assert(!kGated || Cfg::BN % (2 * Cfg::EPI_COLS) == 0, "whole boxes of gate and up columns");
 #pragma unroll 1
     for (int c = 0; c < kBoxes; ++c) {
-      const uint32_t taddr = tmem_base + ((q * 32u) << 16) + acc * Cfg::BN + c * Cfg::EPI_COLS;
+      const uint32_t taddr =
+          tmem_base + ((q * 32u) << 16) + acc * Cfg::BN + c * Cfg::EPI_COLS * (kGated ? 2 : 1);
       uint32_t r0[32], r1[32];
       if constexpr (kGated) {
         uint32_t up[32];
         tmem_ld_32x32(taddr, r0);
-        tmem_ld_32x32(taddr + Cfg::BN / 2, up);
+        tmem_ld_32x32(taddr + Cfg::EPI_COLS, up);
         tmem_wait_ld();
         epi_gate_32(r0, up, g.alpha);
         tmem_ld_32x32(taddr + 32u, r1);
-        tmem_ld_32x32(taddr + Cfg::BN / 2 + 32u, up);
+        tmem_ld_32x32(taddr + Cfg::EPI_COLS + 32u, up);
         tmem_wait_ld();
         epi_gate_32(r1, up, g.alpha);
       } else {
@@ -1329,6 +1359,10 @@ __device__ __forceinline__ void gemm_cta_main(const P& p, const GemmShape& g, ui
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tmem_base = gemm_setup<Cfg>(&ctl, warp);
+  if constexpr (policy_pdl<Policy>()) {
+    pdl_launch_dependents();
+    pdl_wait();
+  }
   // A pair walks the tile list as one worker; `sub` is this CTA's half of every tile.
   const int sub = Cfg::PAIR == 2 ? static_cast<int>(cluster_ctarank()) : 0;
   const int worker = cta / Cfg::PAIR, num_workers = num_ctas / Cfg::PAIR;

@@ -10,6 +10,12 @@
 // weight slab, the number of row blocks is read from device memory (it depends
 // on the routing), and the tile list is simply (row block, column block).
 //
+// Of a row block only the rows that exist are loaded, in boxes of 32 (a decode step's experts have a few rows
+// each), and both products are chained with programmatic dependent launch: one rank's layer, 4096 tokens, top-8
+// of 32, 3101 -> 3043 us, 100 tokens 558 -> 555.  Two waves of tiles or less run 128 columns wide (narrow_tiles
+// in ops/moe.py).  What bounds a large layer is the power cap: a CTA pair per two row blocks, which draws a
+// third less out of L2, takes 2450 us instead of 2540 in a burst and as long as this when calls follow each other.
+//
 // The reference's grouped GEMM for the same layer is a scalar-FMA kernel
 // (datasets/example056_thunderkitten_moe_dispatch_gemm_easy/nv/
 // empty_thunderkitten_moe_dispatch_gemm.cu:227-293); its combine sends expert
@@ -28,10 +34,11 @@ namespace cb {
 
 struct GroupedParams {
   CUtensorMap tm_a;   // [max_rows, K]
+  CUtensorMap tm_a32; // the same in boxes of 32 rows
   CUtensorMap tm_b;   // [E_local * N, K]   (expert slabs stacked along rows)
   CUtensorMap tm_c;   // [max_rows, N]      (up projection only)
   GemmShape g;        // M = max_rows (upper bound), N, K
-  const int* mblk_expert;  // [max_rows / 128]
+  const int* mblk_expert;  // [max_rows / 128] expert | groups of 32 rows << 16
   const int* n_mblocks;    // device word: row blocks in use
   // down projection: scatter to token owners
   const int2* recv_meta;               // [max_rows] {owner rank, pair index} or {-1,-1}
@@ -43,13 +50,14 @@ struct GroupedParams {
 };
 
 // kGatedUp (up projection only): the weight slab of every expert is stored with its rows
-// interleaved per column block - 128 gate rows, then the 128 up rows of the same outputs - and
+// interleaved - 64 gate rows, then the 64 up rows of the same outputs, and so on - and
 // the epilogue writes silu(gate) * up, [rows, N/2], so H1 never exists in memory.
 template <class Cfg, bool kDown, bool kGatedUp = false>
 struct GroupedPolicy {
   using P = GroupedParams;
   static constexpr bool kGated = kGatedUp;
   static_assert(!(kDown && kGatedUp), "the gated epilogue belongs to the up projection");
+  static constexpr bool kPdl = true;
   __device__ static int num_tiles(const P& p) {
     int mb = *reinterpret_cast<const volatile int*>(p.n_mblocks);
     if (mb > p.g.num_m_blocks) mb = p.g.num_m_blocks;
@@ -65,8 +73,10 @@ struct GroupedPolicy {
   __device__ static const CUtensorMap* map_b(const P& p) { return &p.tm_b; }
   __device__ static int a_row(const P&, int m_blk) { return m_blk * Cfg::BM; }
   __device__ static int b_row(const P& p, int m_blk, int n_blk) {
-    return p.mblk_expert[m_blk] * p.g.N + n_blk * Cfg::BN;
+    return (p.mblk_expert[m_blk] & 0xffff) * p.g.N + n_blk * Cfg::BN;
   }
+  __device__ static int a_rows32(const P& p, int m_blk) { return p.mblk_expert[m_blk] >> 16; }
+  __device__ static const CUtensorMap* map_a32(const P& p) { return &p.tm_a32; }
   __device__ static bool wait_a_ready(const P&, int, volatile int*) { return true; }
   static constexpr bool kDirect = kDown;
   static constexpr bool kSignalPerTile = false;  // one completion flag per kernel instead
@@ -126,8 +136,8 @@ static int launch_grouped(const GroupedParams& p, int ctas, cudaStream_t st) {
     set_last_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     return -1;
   }
-  grouped_gemm_kernel<Cfg, kDown, kGatedUp><<<ctas, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(p);
-  e = cudaGetLastError();
+  e = launch_gemm_kernel_pdl(grouped_gemm_kernel<Cfg, kDown, kGatedUp>, ctas, Cfg::THREADS,
+                             Cfg::SMEM_BYTES, st, 1, false, true, p);
   if (e != cudaSuccess) {
     set_last_error(std::string("grouped gemm launch: ") + cudaGetErrorString(e));
     return -1;
@@ -146,7 +156,8 @@ struct CbGroupedDesc {
   int down;          // 0: up projection (C local), 1: down projection with combine scatter
   int rank, world;
   int ctas;
-  int gated;         // up only: b is gate/up interleaved per 256 rows, c = silu(gate) * up
+  int gated;         // up only: b is gate/up interleaved per 64 rows, c = silu(gate) * up
+  int narrow;        // 0: tiles of a row block x 256 columns; 1: of 128 columns
   const void* a;     // [max_rows, K] bf16
   const void* b;     // [n_local_experts * N, K] bf16
   void* c;           // up only: [max_rows, N] bf16, or [max_rows, N / 2] when gated
@@ -159,9 +170,11 @@ struct CbGroupedDesc {
   void* status;
 };
 
-int cb_moe_grouped_gemm(const CbGroupedDesc* d, void* stream) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  using Cfg = GemmCfg<256, 4, false>;
+}  // extern "C"
+
+namespace cb {
+template <class Cfg>
+static int run_grouped(const CbGroupedDesc* d, int ctas, cudaStream_t st) {
   if (d->max_rows % 128 != 0 || d->K % 8 != 0 || d->N % Cfg::BN != 0) {
     set_last_error("grouped gemm: max_rows % 128 == 0, K % 8 == 0, N % 256 == 0 required");
     return -1;
@@ -169,6 +182,9 @@ int cb_moe_grouped_gemm(const CbGroupedDesc* d, void* stream) {
   GroupedParams p;
   if (make_tmap_2d(&p.tm_a, d->a, TMAP_BF16, d->K, d->max_rows, (unsigned long long)d->K * 2,
                    Cfg::BK, Cfg::BM, true))
+    return -1;
+  if (make_tmap_2d(&p.tm_a32, d->a, TMAP_BF16, d->K, d->max_rows, (unsigned long long)d->K * 2,
+                   Cfg::BK, 32, true))
     return -1;
   if (make_tmap_2d(&p.tm_b, d->b, TMAP_BF16, d->K, (unsigned long long)d->n_local_experts * d->N,
                    (unsigned long long)d->K * 2, Cfg::BK, Cfg::BN, true))
@@ -203,10 +219,19 @@ int cb_moe_grouped_gemm(const CbGroupedDesc* d, void* stream) {
   p.rank = d->rank;
   p.world = d->world;
   p.status = static_cast<uint32_t*>(d->status);
-  int ctas = d->ctas > 0 ? d->ctas : 148;
   if (d->down) return launch_grouped<Cfg, true>(p, ctas, st);
   return d->gated ? launch_grouped<Cfg, false, true>(p, ctas, st)
                   : launch_grouped<Cfg, false, false>(p, ctas, st);
+}
+}  // namespace cb
+
+extern "C" {
+
+int cb_moe_grouped_gemm(const CbGroupedDesc* d, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int ctas = d->ctas > 0 ? d->ctas : 148;
+  return d->narrow ? run_grouped<GemmCfg<128, 6, false>>(d, ctas, st)
+                   : run_grouped<GemmCfg<256, 4, false>>(d, ctas, st);
 }
 
 }  // extern "C"

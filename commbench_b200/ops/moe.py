@@ -24,6 +24,7 @@ waits on a kernel of the same phase, so nothing ever waits on a later launch.
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import torch
 
@@ -60,7 +61,7 @@ class _GroupedDesc(C.Structure):
     _fields_ = [
         ("max_rows", C.c_int), ("N", C.c_int), ("K", C.c_int), ("n_local_experts", C.c_int),
         ("down", C.c_int), ("rank", C.c_int), ("world", C.c_int), ("ctas", C.c_int),
-        ("gated", C.c_int),
+        ("gated", C.c_int), ("narrow", C.c_int),
         ("a", C.c_void_p), ("b", C.c_void_p), ("c", C.c_void_p),
         ("mblk_expert", C.c_void_p), ("n_mblocks", C.c_void_p), ("recv_meta", C.c_void_p),
         ("combine_peer", _P8), ("done_peer", _P8), ("done_ctas", C.c_void_p),
@@ -108,6 +109,26 @@ def interleave_gate_up(w1: torch.Tensor, block: int = 128) -> torch.Tensor:
     return torch.cat([g, u], dim=2).reshape(E, two_i, H).contiguous()
 
 
+GATE_BLOCK = 64      # rows of gate, then of up, in the row order of the gated up projection
+
+
+def narrow_tiles(avg_rows: float, experts: int, n: int, sms: int) -> bool:
+    """Whether a grouped GEMM with ``n`` columns runs on 128-wide tiles instead of 256-wide ones, from the
+    average rows per expert.
+
+    Only for a decode step whose 256-wide tiles do not fill two waves: the weights bound it, and with more
+    waves the SMs share the memory's rate however the last one is filled, at less cost in the wider form.
+    Measured, 256 / 128 wide for the whole layer, with three layers' weights in turn: 16 tokens, top-2 of 64,
+    hidden 2048, intermediate 1024 (1.4 waves) 135-151 / 115 us; 64 tokens, top-2 of 16, 4096 / 2048 (1.7)
+    197 / 196; 100 tokens, top-8 of 32, 7168 / 2048 (3.5) 551 / 567; 512 tokens, top-8 of 64 (6.9)
+    1085 / 1183."""
+    if avg_rows > 96:
+        return False
+    blocks = experts * (1.0 - math.exp(-avg_rows))      # experts that a token selects
+    wide, narrow = math.ceil(blocks * (n // 256) / sms), math.ceil(blocks * (n // 128) / sms)
+    return wide <= 2 and 0.51 * narrow < wide
+
+
 class _RankState:
     """Buffers of one (virtual) rank."""
 
@@ -135,7 +156,7 @@ class _RankState:
         self.w1 = (torch.randn(L.El, 2 * L.I, L.H, device=dev, generator=g) * 0.02).bfloat16()
         self.w2 = (torch.randn(L.El, L.H, L.I, device=dev, generator=g) * 0.02).bfloat16()
         # The gated up projection reads its own row order of the same weights (one more copy of w1).
-        self.w1_gated = interleave_gate_up(self.w1) if L.fused_swiglu else None
+        self.w1_gated = interleave_gate_up(self.w1, GATE_BLOCK) if L.fused_swiglu else None
 
 
 class MoELayer:
@@ -184,6 +205,9 @@ class MoELayer:
         self.states = [_RankState(self, r if self.emu else ctx.rank, dev)
                        for r in range(self.W if self.emu else 1)]
         self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        rows = tokens * topk / self.El
+        self.narrow_up = narrow_tiles(rows, self.El, 2 * intermediate, self.sms)
+        self.narrow_down = narrow_tiles(rows, self.El, hidden, self.sms)
         torch.cuda.synchronize(dev)
         if not self.emu:
             ctx.host_barrier()
@@ -295,6 +319,7 @@ class MoELayer:
                 d.gated, d.a, d.b, d.c = 1, st.a.data_ptr(), st.w1_gated.data_ptr(), st.s.data_ptr()
             else:
                 d.gated, d.a, d.b, d.c = 0, st.a.data_ptr(), st.w1.data_ptr(), st.h1.data_ptr()
+            d.narrow = int(self.narrow_up)
             d.mblk_expert, d.n_mblocks = st.mblk_expert.data_ptr(), st.n_mblocks.data_ptr()
             d.status = self._status(st)
             N.check(lib.cb_moe_grouped_gemm(C.byref(d), sp), "grouped gemm (up)")
@@ -308,6 +333,7 @@ class MoELayer:
             d2.max_rows, d2.N, d2.K, d2.n_local_experts = self.max_rows, H, I, self.El
             d2.down, d2.rank, d2.world, d2.ctas = 1, st.r, W, self.sms
             d2.a, d2.b, d2.c = st.s.data_ptr(), st.w2.data_ptr(), 0
+            d2.narrow = int(self.narrow_down)
             d2.mblk_expert, d2.n_mblocks = st.mblk_expert.data_ptr(), st.n_mblocks.data_ptr()
             d2.recv_meta = self._local(self.recv_meta, st).data_ptr()
             d2.combine_peer, d2.done_peer = _P8(*self.combine.ptrs), _P8(*self.done.ptrs)

@@ -23,7 +23,7 @@ from __future__ import annotations
 import torch
 import torch.distributed as dist
 
-from ..ops.moe import (MoELayer, dispatch_layout, expert_sort, interleave_gate_up,  # noqa: F401
+from ..ops.moe import (GATE_BLOCK, MoELayer, dispatch_layout, expert_sort, interleave_gate_up,  # noqa: F401
                        reference_moe, router_topk)
 from ..ops.p2p import rearrange_expert_weights_inplace  # noqa: F401
 from ..runtime.context import CommError
@@ -124,7 +124,7 @@ class ExpertParallelMoE(MoELayer):
         ops = rearrange_expert_weights_inplace(self.placement, new_map, [st.w1, st.w2], self.El,
                                                group=group)
         if st.w1_gated is not None:
-            st.w1_gated = interleave_gate_up(st.w1)       # the gated copy follows its source
+            st.w1_gated = interleave_gate_up(st.w1, GATE_BLOCK)       # the gated copy follows its source
         moved = sum(1 for a, b in zip(self.placement, new_map) if a != b)
         self.placement = new_map
         inv = [0] * self.E

@@ -156,3 +156,35 @@ def test_moe_layer_on_one_real_rank(native_lib, dispatch):
         assert (y.float() - ref).abs().max() <= 3e-2 * ref.abs().max()
     ctx.check_status()
     ctx.close()
+
+
+@pytest.mark.parametrize("fused_swiglu", [True, False])
+@pytest.mark.parametrize("narrow", [False, True])
+def test_grouped_gemm_at_row_counts_around_its_boxes(native_lib, narrow, fused_swiglu):
+    """Experts with 0, 1, 31 ... 385 rows (operand boxes of 32 rows, row blocks of 128), tiles of 256 and of
+    128 columns."""
+    from commbench_b200.ops.moe import MoELayer, reference_moe
+    from commbench_b200.runtime.context import CommContext
+
+    counts = [1, 31, 32, 0, 33, 127, 128, 129, 255, 256, 257, 385]
+    E, H, I, T = len(counts), 512, 512, sum(counts)
+    g = torch.Generator(device="cuda").manual_seed(11)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).int()[torch.randperm(T)]
+    idx = idx.view(T, 1).cuda()
+    w = torch.rand(T, 1, device="cuda", generator=g) + 0.5
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    ctx = CommContext(heap_bytes=64 << 20)
+    layer = MoELayer(ctx, T, H, I, E, 1, seed=3, fused_swiglu=fused_swiglu)
+    layer.narrow_up = layer.narrow_down = narrow
+    w1, w2 = layer.weights()
+    ref = reference_moe(x, idx, w, w1, w2, I)
+    for _ in range(2):
+        y = layer.forward(x, idx, w).float()
+        torch.cuda.synchronize()
+        ctx.check_status()
+        # bf16 roundings of the two products, as in the layer's other tests
+        assert (y - ref).abs().max().item() < 3e-2 * ref.abs().max().item()
+    layer.narrow_up = layer.narrow_down = not narrow
+    assert torch.equal(layer.forward(x, idx, w).float(), y)    # same K order: the same bits
+    torch.cuda.synchronize()
+    ctx.close()
