@@ -26,6 +26,8 @@ CSRC = PKG / "csrc"
 LIBDIR = PKG / "lib"
 OBJDIR = PKG.parent / "build" / "obj"
 LIBNAME = "libcommbench_b200.so"
+FAST_SRC = PKG / "host" / "fast_ops.cpp"      # Python extension: the call path of the small operators
+FASTNAME = "_fast_ops.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -125,9 +127,40 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{' '.join(cmd)}\n{r.stdout}{r.stderr}")
+    build_fast(force)
     if ptxas_verbose:
         (OBJDIR / "ptxas.log").write_text("\n".join(f"== {k}\n{v}" for k, v in logs.items()))
     return lib
+
+
+def build_fast(force: bool = False) -> Path:
+    """Compiles the extension against the installed PyTorch and Python; both are part of its cache key."""
+    import sysconfig
+
+    import torch
+
+    out = LIBDIR / FASTNAME
+    home = Path(torch.__file__).resolve().parent
+    libs = home / "lib"
+    cuda = Path(nvcc_path()).resolve().parent.parent
+    flags = ["-O2", "-std=c++20", "-fPIC", "-shared",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             "-I", sysconfig.get_paths()["include"], "-I", str(cuda / "include")]
+    for inc in (home / "include", home / "include/torch/csrc/api/include"):
+        flags += ["-isystem", str(inc)]
+    key = hashlib.sha256(FAST_SRC.read_bytes() +
+                         f"{torch.__version__} {sys.version} {flags}".encode()).hexdigest()[:24]
+    stamp = OBJDIR / (FASTNAME + ".key")
+    if not force and out.exists() and stamp.exists() and stamp.read_text() == key:
+        return out
+    OBJDIR.mkdir(parents=True, exist_ok=True)
+    cmd = [os.environ.get("CXX", "g++"), *flags, str(FAST_SRC), "-o", str(out), "-L", str(libs), "-lc10",
+           "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-Wl,-rpath,{libs}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling {FAST_SRC} failed:\n{' '.join(cmd)}\n{r.stdout}{r.stderr}")
+    stamp.write_text(key)
+    return out
 
 
 if __name__ == "__main__":

@@ -17,7 +17,9 @@ PAD_ABORT = PAD_NVLS_BASE + PAD_CHANNELS
 PAD_WORDS = PAD_ABORT + 64
 
 _LIB_PATH = Path(__file__).resolve().parent / "lib" / "libcommbench_b200.so"
+_FAST_PATH = _LIB_PATH.with_name("_fast_ops.so")
 _lib = None
+_fast = None
 
 
 class NativeError(RuntimeError):
@@ -135,6 +137,32 @@ def load():
             f"CollArgs layout mismatch: C {lib.cb_sizeof_coll_args()} vs ctypes {C.sizeof(CollArgs)}")
     _lib = lib
     return lib
+
+
+_FAST_ENTRIES = ("cb_gemm_bf16", "cb_gemm_fp8", "cb_gemm_fp8_blockscaled", "cb_gemm_fp8_mx",
+                 "cb_quant_blockscaled", "cb_quant_blockscaled_pow2", "cb_attn_fwd4",
+                 "cb_attn_split_bytes", "cb_attn_split")
+
+
+def fast():
+    """The extension with the short call path of the small operators (host/fast_ops.cpp).  Each of its
+    functions answers None for a call that it leaves to the general path."""
+    global _fast
+    if _fast is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (the extension links against its libraries)
+
+        lib = load()
+        if not _FAST_PATH.exists():
+            raise NativeError(f"{_FAST_PATH} is missing: run `python -m commbench_b200._build` first")
+        loader = importlib.machinery.ExtensionFileLoader("_fast_ops", str(_FAST_PATH))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fast_ops", loader))
+        loader.exec_module(mod)
+        mod.bind({n: C.cast(getattr(lib, n), C.c_void_p).value for n in _FAST_ENTRIES})
+        _fast = mod
+    return _fast
 
 
 def last_error() -> str:

@@ -62,6 +62,10 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, kv_offset: 
 
     ``q_offset`` / ``kv_offset`` are the global sequence positions of the first query / key;
     with ``causal`` key j is visible to query i iff kv_offset + j <= q_offset + i."""
+    if out is None and lse is None and stream is None and impl is None and get_config().attn_impl == 4:
+        r = N.fast().attention(q, k, v, causal, q_offset, kv_offset, scale, status_ptr)
+        if r is not None:
+            return r
     lib = N.load()
     for t, n in ((q, "q"), (k, "k"), (v, "v")):
         if not (t.is_cuda and t.is_contiguous() and t.dtype == torch.bfloat16 and t.dim() == 4

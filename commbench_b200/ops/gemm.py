@@ -27,6 +27,10 @@ def _check(t: torch.Tensor, name: str):
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, alpha: float = 1.0,
          bn: int = 0, max_ctas: int = 0, status_ptr: int = 0, stream=None) -> torch.Tensor:
     """``out[M,N] = alpha * a[M,K] @ b[N,K].T`` on the tcgen05 kernel (no library GEMM)."""
+    if stream is None:
+        r = N.fast().gemm(a, b, out, alpha, bn, max_ctas, status_ptr)
+        if r is not None:
+            return r
     lib = N.load()
     _check(a, "a")
     _check(b, "b")
@@ -109,6 +113,10 @@ def quantize_blockscaled_pow2(x: torch.Tensor, row_block: int = 1):
     ``2 ** (byte - 127)``) of K blocks ``4 kg .. 4 kg + 3`` of row ``r``, lowest byte first
     (missing blocks: 127).  For ``row_block=128`` every row of a block carries the block's
     byte, so ``sf`` has one column per row of ``x`` either way - what :func:`gemm_fp8_mx` takes."""
+    if row_block == 1:
+        r = N.fast().quantize_rows(x, True)
+        if r is not None:
+            return r
     lib = N.load()
     _check(x, "x")
     rows, K = x.shape
@@ -137,6 +145,10 @@ def gemm_fp8_mx(a_q, a_sf, b_q, b_sf, out=None, alpha: float = 1.0, pair: bool =
     """``out = (a_q * 2^(a_sf-127)) @ (b_q * 2^(b_sf-127)).T`` with the power-of-two block scales
     applied by the tensor cores (``tcgen05.mma.kind::mxf8f6f4.block_scale``): ``a_sf``
     [ceil(K/512), M], ``b_sf`` [ceil(K/512), N] int32 from :func:`quantize_blockscaled_pow2`."""
+    if stream is None:
+        r = N.fast().gemm_fp8_mx(a_q, a_sf, b_q, b_sf, out, alpha, pair, status_ptr)
+        if r is not None:
+            return r
     lib = N.load()
     _check(a_q, "a_q")
     _check(b_q, "b_q")
@@ -183,6 +195,10 @@ def gemm_fp8_blockscaled(a_q, a_s, b_q, b_s, out=None, alpha: float = 1.0, pair:
     cores: the quantised operands are the MMA operands, and every 128-wide K block's partial sum
     is multiplied by its two scales and accumulated in fp32 registers inside the kernel.
     ``pair`` makes no difference any more: one CTA per tile is the faster form at every size."""
+    if stream is None:
+        r = N.fast().gemm_fp8_blockscaled(a_q, a_s, b_q, b_s, out, alpha, max_ctas, status_ptr)
+        if r is not None:
+            return r
     lib = N.load()
     _check(a_q, "a_q")
     _check(b_q, "b_q")
