@@ -10,11 +10,12 @@
 // weight slab, the number of row blocks is read from device memory (it depends
 // on the routing), and the tile list is simply (row block, column block).
 //
-// Of a row block only the rows that exist are loaded, in boxes of 32 (a decode step's experts have a few rows
-// each), and both products are chained with programmatic dependent launch: one rank's layer, 4096 tokens, top-8
-// of 32, 3101 -> 3043 us, 100 tokens 558 -> 555.  Two waves of tiles or less run 128 columns wide (narrow_tiles
-// in ops/moe.py).  What bounds a large layer is the power cap: a CTA pair per two row blocks, which draws a
-// third less out of L2, takes 2450 us instead of 2540 in a burst and as long as this when calls follow each other.
+// Of a row block only the rows that exist are loaded, in boxes of 32: a decode step's experts have a few rows
+// each.  Calls in a row with three layers' weights in turn, one rank: 100 tokens, top-8 of 32, 560 -> 553 us;
+// 1000 tokens, top-4 of 32, 428 -> 418; 4096 tokens, top-8 of 32, 2960 either way.  Two waves of tiles or less
+// run 128 columns wide (narrow_tiles in ops/moe.py).  What bounds a large layer is the power cap: a CTA pair per
+// two row blocks, which draws a third less out of L2, takes 2450 us instead of 2540 in a burst and as long as
+// this when calls follow each other.  Launching the products as programmatic dependents gained nothing either.
 //
 // The reference's grouped GEMM for the same layer is a scalar-FMA kernel
 // (datasets/example056_thunderkitten_moe_dispatch_gemm_easy/nv/
@@ -57,7 +58,6 @@ struct GroupedPolicy {
   using P = GroupedParams;
   static constexpr bool kGated = kGatedUp;
   static_assert(!(kDown && kGatedUp), "the gated epilogue belongs to the up projection");
-  static constexpr bool kPdl = true;
   __device__ static int num_tiles(const P& p) {
     int mb = *reinterpret_cast<const volatile int*>(p.n_mblocks);
     if (mb > p.g.num_m_blocks) mb = p.g.num_m_blocks;
@@ -136,8 +136,8 @@ static int launch_grouped(const GroupedParams& p, int ctas, cudaStream_t st) {
     set_last_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     return -1;
   }
-  e = launch_gemm_kernel_pdl(grouped_gemm_kernel<Cfg, kDown, kGatedUp>, ctas, Cfg::THREADS,
-                             Cfg::SMEM_BYTES, st, 1, false, true, p);
+  grouped_gemm_kernel<Cfg, kDown, kGatedUp><<<ctas, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(p);
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_error(std::string("grouped gemm launch: ") + cudaGetErrorString(e));
     return -1;
