@@ -26,8 +26,9 @@ static int cp_launch_t(const FaCpParams& p, int grid, cudaStream_t st) {
     set_last_error(std::string("cudaFuncSetAttribute(fa_cp): ") + cudaGetErrorString(e));
     return -1;
   }
-  fa_cp_kernel<kPoly><<<grid, CP_THREADS, CP_SMEM, st>>>(p);
-  e = cudaGetLastError();
+  // Tickets are drawn before the kernel waits for its predecessors: only without them it may start early.
+  e = launch_gemm_kernel_pdl(fa_cp_kernel<kPoly>, grid, CP_THREADS, CP_SMEM, st, 1, false,
+                             p.sched == nullptr, p);
   if (e != cudaSuccess) {
     set_last_error(std::string("context-parallel attention launch: ") + cudaGetErrorString(e));
     return -1;

@@ -50,6 +50,7 @@
 #include <cuda_bf16.h>
 
 #include "../prim/clc.cuh"
+#include "../prim/pdl.cuh"
 #include "../prim/tcgen05.cuh"
 #include "../prim/tma.cuh"
 #include "fa_cp_types.h"
@@ -432,6 +433,8 @@ __global__ void __launch_bounds__(CP_THREADS, 1) fa_cp_kernel(const __grid_const
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    pdl_launch_dependents();
+    pdl_wait();   // queries, keys and values, and readers of the result, of the kernels before
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&ctl.tmem_base);
     // tile t: S (fp32, 128 columns; its first 64 columns hold P as bf16 pairs after the
     // softmax) at column 256 t, O at column 256 t + 128.

@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   pdl_launch_dependents();   // the merge kernel waits for this grid's completion itself
+  pdl_wait();                // operands, and readers of results and workspace, of the kernels before
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&ctl.tmem_base);
   // stream t: S (fp32, 128 columns; the first 64 hold P as bf16 pairs after the softmax) at column
   // 256 t, O at column 256 t + 128.
@@ -727,8 +728,7 @@ int cb_attn_split(const void* q, const void* k, const void* v, void* o, void* ls
   static std::atomic<uint64_t> smem_done{0};
   cudaError_t e = allow_smem(reinterpret_cast<const void*>(fa_split_kernel), SP_SMEM, smem_done);
   if (e == cudaSuccess) {
-    fa_split_kernel<<<p.pl.ctas, CP_THREADS, SP_SMEM, st>>>(p);
-    e = cudaGetLastError();
+    e = launch_pdl(fa_split_kernel, dim3(static_cast<unsigned>(p.pl.ctas)), dim3(CP_THREADS), SP_SMEM, st, p);
   }
   if (e == cudaSuccess && p.pl.merge) {
     const long long rows = static_cast<long long>(B) * Sq * Hq;

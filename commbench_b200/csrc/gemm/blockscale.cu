@@ -10,6 +10,8 @@
 
 #include <string>
 
+#include "../prim/pdl.cuh"
+
 namespace cb {
 void set_last_error(const std::string& s);
 
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(256)
     quant_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
                       float* __restrict__ scale, long long rows, int K, int pow2,
                       uint32_t* __restrict__ sf_words, int sf_ld) {
+  pdl_launch_dependents();   // the product's set-up overlaps this kernel; it waits for its end
   const int kblocks = K / 128;
   const int kgroups = (kblocks + 3) / 4;
   const long long w = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;

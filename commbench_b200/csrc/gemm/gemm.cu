@@ -72,6 +72,7 @@ struct PlainParams {
 template <class Cfg>
 struct PlainPolicy {
   using P = PlainParams;
+  static constexpr bool kPdl = true;
   static constexpr bool kDirect = false;
   static constexpr bool kSignalPerTile = false;
   static constexpr bool kScatterRows = false;
@@ -178,8 +179,8 @@ static int launch_plain(const void* a, const void* b, void* c, int M, int N, int
     set_last_error("gemm: a tile of a CTA pair needs a limit of at least two CTAs");
     return -1;
   }
-  cudaError_t e = launch_gemm_kernel(gemm_plain_kernel<Cfg>, ctas, Cfg::THREADS, Cfg::SMEM_BYTES,
-                                     st, Cfg::PAIR, false, p);
+  cudaError_t e = launch_gemm_kernel_pdl(gemm_plain_kernel<Cfg>, ctas, Cfg::THREADS, Cfg::SMEM_BYTES,
+                                         st, Cfg::PAIR, false, true, p);
   if (e != cudaSuccess) {
     set_last_error(std::string("gemm launch: ") + cudaGetErrorString(e));
     return -1;

@@ -66,6 +66,7 @@
 #include <cuda_bf16.h>
 
 #include "../prim/cluster.cuh"
+#include "../prim/pdl.cuh"
 #include "../prim/tcgen05.cuh"
 #include "../prim/tma.cuh"
 
@@ -207,6 +208,17 @@ struct GemmCtl {
 //   optional: int a_rows32(const P&, int m_blk), const CUtensorMap* map_a32(const P&)   (one CTA per tile) the
 //                                              tile has rows in its first 32 a_rows32 only, which are
 //                                              loaded in boxes of 32; the others are whatever the ring holds
+//   optional: static constexpr bool kPdl       launched with programmatic dependent launch: after set-up,
+//                                              wait for the kernels before
+template <class Policy>
+__host__ __device__ constexpr bool policy_pdl() {
+  if constexpr (requires { Policy::kPdl; }) {
+    return Policy::kPdl;
+  } else {
+    return false;
+  }
+}
+
 // Producer and MMA roles are executed by a whole, converged warp: every lane follows the loop
 // and the waits, one elected lane issues the TMA loads / MMAs / commits.  Measured on B200
 // with back-to-back MMAs of 32 pipe cycles each: 43-49 cycles per instruction issued this way
@@ -1347,6 +1359,10 @@ __device__ __forceinline__ void gemm_cta_main(const P& p, const GemmShape& g, ui
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tmem_base = gemm_setup<Cfg>(&ctl, warp);
+  if constexpr (policy_pdl<Policy>()) {
+    pdl_launch_dependents();
+    pdl_wait();   // operands, and readers of the result, of the kernels before
+  }
   // A pair walks the tile list as one worker; `sub` is this CTA's half of every tile.
   const int sub = Cfg::PAIR == 2 ? static_cast<int>(cluster_ctarank()) : 0;
   const int worker = cta / Cfg::PAIR, num_workers = num_ctas / Cfg::PAIR;

@@ -291,6 +291,12 @@ class RingAttention(_CpBase):
                 k_own.copy_(ks[i])
             if vs[i].data_ptr() != v_own.data_ptr():
                 v_own.copy_(vs[i])
+        # One rank: a plain local attention over its own slot, without pieces or counters.
+        if self.W == 1 and not self.emu and out is None and want_lse and self.B <= 64 and \
+                tuple(q.shape) == (self.B, self.Sl, self.Hq, 128):
+            res = N.fast().attention(q, self._k_own[0], self._v_own[0], causal, 0, 0, sc, self._status_ptr(0))
+            if res is not None:
+                return res
         # A plan change (causal <-> full) rewrites the piece list and renumbers the counters:
         # nothing of the old plan may still run, and the counters start again from zero.
         if self._plan_key != (bool(causal),):
