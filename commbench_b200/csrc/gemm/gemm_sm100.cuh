@@ -205,11 +205,16 @@ struct GemmCtl {
 //                                              were issued (one lane); quadrant = 4 * (CTA of
 //                                              the pair) + epilogue warp, or 4 * CTA from the
 //                                              signal warp of a direct policy
-//   optional: int a_rows32(const P&, int m_blk), const CUtensorMap* map_a32(const P&)   (one CTA per tile) the
-//                                              tile has rows in its first 32 a_rows32 only, which are
-//                                              loaded in boxes of 32; the others are whatever the ring holds
 //   optional: static constexpr bool kPdl       launched with programmatic dependent launch: after set-up,
 //                                              wait for the kernels before
+//   optional: bool early_b(const P&)           (one CTA per tile) as kPdl, but where this says so the producer
+//                                              fills the ring with B of its first tile before it waits:
+//                                              neither B nor what num_tiles, tile_coord and b_row read is
+//                                              written by a kernel that may still run then
+template <class Policy, class P>
+__host__ __device__ constexpr bool policy_early_b() {
+  return requires(const P& p) { Policy::early_b(p); };
+}
 template <class Policy>
 __host__ __device__ constexpr bool policy_pdl() {
   if constexpr (requires { Policy::kPdl; }) {
@@ -241,6 +246,26 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
   int ready_tiles = 0;
   // Pair: both CTAs' bytes are counted on the even CTA's barrier, the one its MMA warp waits on.
   const uint32_t full0_leader = Cfg::PAIR == 2 ? map_to_cta(full0, 0) : full0;
+  [[maybe_unused]] int early = 0;   // K blocks whose B is on its way already
+  if constexpr (policy_early_b<Policy, P>()) {
+    static_assert(Cfg::PAIR == 1, "see early_b");
+    const bool first = Policy::early_b(p);
+    if (first && cta < ntiles) {
+      int m_blk, n_blk;
+      Policy::tile_coord(p, cta, &m_blk, &n_blk);
+      const int brow = Policy::b_row(p, m_blk, n_blk);
+      early = g.num_k_blocks < Cfg::STAGES ? g.num_k_blocks : Cfg::STAGES;
+      if (elect_one()) {
+        for (int kb = 0; kb < early; ++kb) {
+          mbar_arrive_expect_tx_addr(full0 + kb * 8u, Cfg::STAGE_BYTES);
+          tma_load_2d_addr(ring_addr + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, Policy::map_b(p), kb * Cfg::BK,
+                           brow, full0 + kb * 8u);
+        }
+      }
+      __syncwarp();
+    }
+    if (first) pdl_wait();
+  }
   for (int tile = cta; tile < ntiles; tile += num_ctas) {
     int m_blk, n_blk;
     Policy::tile_coord(p, tile, &m_blk, &n_blk);
@@ -256,11 +281,9 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
     }
     const CUtensorMap* ma = Policy::map_a(p, m_blk);
     const CUtensorMap* mb = Policy::map_b(p);
-    constexpr bool kRagged = Cfg::PAIR == 1 && requires { Policy::a_rows32(p, m_blk); };
-    [[maybe_unused]] int a32 = 4;
-    if constexpr (kRagged) a32 = Policy::a_rows32(p, m_blk);
     const int arow = Policy::a_row(p, m_blk) + sub * Cfg::CTA_M;
     const int brow = Policy::b_row(p, m_blk, n_blk) + sub * Cfg::B_ROWS;
+    const bool some_b = policy_early_b<Policy, P>() && early > 0 && tile == cta;   // B is there in part
     for (int kb = 0; kb < g.num_k_blocks; ++kb) {
       if (!mbar_wait_traced(&ctl->empty[stage], phase ^ 1u, &ctl->abort_flag, status,
                             0x100 + stage, tracing, &w_empty))
@@ -277,15 +300,8 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
           tma_load_2d_pair(sb, mb, kb * Cfg::BK, brow, bar);
         } else {
           const uint32_t bar = full0 + stage * 8u;
-          if constexpr (kRagged) {
-            mbar_arrive_expect_tx_addr(bar, Cfg::B_BYTES + a32 * 4096);
-            tma_load_2d_addr(sb, mb, kb * Cfg::BK, brow, bar);
-            if (a32 == 4) {
-              tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
-            } else {
-              for (int i = 0; i < a32; ++i)
-                tma_load_2d_addr(sa + i * 4096, Policy::map_a32(p), kb * Cfg::BK, arow + i * 32, bar);
-            }
+          if (some_b && kb < early) {
+            tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
           } else {
             mbar_arrive_expect_tx_addr(bar, Cfg::STAGE_BYTES);
             tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
@@ -1359,7 +1375,13 @@ __device__ __forceinline__ void gemm_cta_main(const P& p, const GemmShape& g, ui
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tmem_base = gemm_setup<Cfg>(&ctl, warp);
-  if constexpr (policy_pdl<Policy>()) {
+  if constexpr (policy_early_b<Policy, P>()) {
+    // The dependents may count on what this kernel's predecessors wrote: released after the wait only.
+    if (Policy::early_b(p) && warp != 0) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
+  } else if constexpr (policy_pdl<Policy>()) {
     pdl_launch_dependents();
     pdl_wait();   // operands, and readers of the result, of the kernels before
   }

@@ -10,12 +10,15 @@
 // weight slab, the number of row blocks is read from device memory (it depends
 // on the routing), and the tile list is simply (row block, column block).
 //
-// Of a row block only the rows that exist are loaded, in boxes of 32: a decode step's experts have a few rows
-// each.  Calls in a row with three layers' weights in turn, one rank: 100 tokens, top-8 of 32, 560 -> 553 us;
-// 1000 tokens, top-4 of 32, 428 -> 418; 4096 tokens, top-8 of 32, 2960 either way.  Two waves of tiles or less
-// run 128 columns wide (narrow_tiles in ops/moe.py).  What bounds a large layer is the power cap: a CTA pair per
-// two row blocks, which draws a third less out of L2, takes 2450 us instead of 2540 in a burst and as long as
-// this when calls follow each other.  Launching the products as programmatic dependents gained nothing either.
+// A decode step (early): each product starts as a programmatic dependent and fetches weights - which no kernel of
+// the layer writes - while the kernel before ends.  One rank, three layers' weights in turn: 16 tokens, top-8 of
+// 8 experts, hidden 7168, intermediate 2048 178 -> 173 us; 24, top-8 of 32, 2048 / 2048 214 -> 209; 52, top-4 of
+// 8, 4096 / 1024 104.6 -> 89; 100, top-8 of 32, 7168 / 2048 557 -> 552.  Larger layers do not gain by it (3096
+// tokens, top-8 of 64, 2048 / 1024: 511 without, 521 to 545 with).  Two waves of tiles or less run 128 columns
+// wide (narrow_tiles in ops/moe.py).  Loading only the rows that a block has, in boxes of 32, cost the producer
+// more than it saved (511 -> 521).  What bounds a large layer is the power cap: a CTA pair per two row blocks,
+// which draws a third less out of L2, takes 2450 us instead of 2540 in a burst (4096 tokens, top-8 of 32) and as
+// long as this, 2960, when calls follow each other.
 //
 // The reference's grouped GEMM for the same layer is a scalar-FMA kernel
 // (datasets/example056_thunderkitten_moe_dispatch_gemm_easy/nv/
@@ -35,11 +38,10 @@ namespace cb {
 
 struct GroupedParams {
   CUtensorMap tm_a;   // [max_rows, K]
-  CUtensorMap tm_a32; // the same in boxes of 32 rows
   CUtensorMap tm_b;   // [E_local * N, K]   (expert slabs stacked along rows)
   CUtensorMap tm_c;   // [max_rows, N]      (up projection only)
   GemmShape g;        // M = max_rows (upper bound), N, K
-  const int* mblk_expert;  // [max_rows / 128] expert | groups of 32 rows << 16
+  const int* mblk_expert;  // [max_rows / 128]
   const int* n_mblocks;    // device word: row blocks in use
   // down projection: scatter to token owners
   const int2* recv_meta;               // [max_rows] {owner rank, pair index} or {-1,-1}
@@ -47,6 +49,7 @@ struct GroupedParams {
   uint32_t* done_peer[CB_MAX_RANKS];   // owner's done words [W]
   uint32_t* done_ctas;                 // local scratch counter
   int rank, world;
+  int early;
   uint32_t* status;
 };
 
@@ -58,6 +61,9 @@ struct GroupedPolicy {
   using P = GroupedParams;
   static constexpr bool kGated = kGatedUp;
   static_assert(!(kDown && kGatedUp), "the gated epilogue belongs to the up projection");
+  // The kernel before is the receive kernel or the other product: each releases its dependents after its own
+  // wait, so the plan has been complete since then, and none of them writes weights.
+  __device__ static bool early_b(const P& p) { return p.early != 0; }
   __device__ static int num_tiles(const P& p) {
     int mb = *reinterpret_cast<const volatile int*>(p.n_mblocks);
     if (mb > p.g.num_m_blocks) mb = p.g.num_m_blocks;
@@ -73,10 +79,8 @@ struct GroupedPolicy {
   __device__ static const CUtensorMap* map_b(const P& p) { return &p.tm_b; }
   __device__ static int a_row(const P&, int m_blk) { return m_blk * Cfg::BM; }
   __device__ static int b_row(const P& p, int m_blk, int n_blk) {
-    return (p.mblk_expert[m_blk] & 0xffff) * p.g.N + n_blk * Cfg::BN;
+    return p.mblk_expert[m_blk] * p.g.N + n_blk * Cfg::BN;
   }
-  __device__ static int a_rows32(const P& p, int m_blk) { return p.mblk_expert[m_blk] >> 16; }
-  __device__ static const CUtensorMap* map_a32(const P& p) { return &p.tm_a32; }
   __device__ static bool wait_a_ready(const P&, int, volatile int*) { return true; }
   static constexpr bool kDirect = kDown;
   static constexpr bool kSignalPerTile = false;  // one completion flag per kernel instead
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
 }
 
 template <class Cfg, bool kDown, bool kGatedUp = false>
-static int launch_grouped(const GroupedParams& p, int ctas, cudaStream_t st) {
+static int launch_grouped(const GroupedParams& p, int ctas, bool early, cudaStream_t st) {
   static std::atomic<uint64_t> smem_done{0};
   cudaError_t e = allow_smem(
       reinterpret_cast<const void*>(grouped_gemm_kernel<Cfg, kDown, kGatedUp>), Cfg::SMEM_BYTES,
@@ -136,8 +140,8 @@ static int launch_grouped(const GroupedParams& p, int ctas, cudaStream_t st) {
     set_last_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     return -1;
   }
-  grouped_gemm_kernel<Cfg, kDown, kGatedUp><<<ctas, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(p);
-  e = cudaGetLastError();
+  e = launch_gemm_kernel_pdl(grouped_gemm_kernel<Cfg, kDown, kGatedUp>, ctas, Cfg::THREADS,
+                             Cfg::SMEM_BYTES, st, 1, false, early, p);
   if (e != cudaSuccess) {
     set_last_error(std::string("grouped gemm launch: ") + cudaGetErrorString(e));
     return -1;
@@ -158,6 +162,7 @@ struct CbGroupedDesc {
   int ctas;
   int gated;         // up only: b is gate/up interleaved per 64 rows, c = silu(gate) * up
   int narrow;        // 0: tiles of a row block x 256 columns; 1: of 128 columns
+  int early;         // 1: starts while the kernel before ends and fetches weights first
   const void* a;     // [max_rows, K] bf16
   const void* b;     // [n_local_experts * N, K] bf16
   void* c;           // up only: [max_rows, N] bf16, or [max_rows, N / 2] when gated
@@ -182,9 +187,6 @@ static int run_grouped(const CbGroupedDesc* d, int ctas, cudaStream_t st) {
   GroupedParams p;
   if (make_tmap_2d(&p.tm_a, d->a, TMAP_BF16, d->K, d->max_rows, (unsigned long long)d->K * 2,
                    Cfg::BK, Cfg::BM, true))
-    return -1;
-  if (make_tmap_2d(&p.tm_a32, d->a, TMAP_BF16, d->K, d->max_rows, (unsigned long long)d->K * 2,
-                   Cfg::BK, 32, true))
     return -1;
   if (make_tmap_2d(&p.tm_b, d->b, TMAP_BF16, d->K, (unsigned long long)d->n_local_experts * d->N,
                    (unsigned long long)d->K * 2, Cfg::BK, Cfg::BN, true))
@@ -219,9 +221,11 @@ static int run_grouped(const CbGroupedDesc* d, int ctas, cudaStream_t st) {
   p.rank = d->rank;
   p.world = d->world;
   p.status = static_cast<uint32_t*>(d->status);
-  if (d->down) return launch_grouped<Cfg, true>(p, ctas, st);
-  return d->gated ? launch_grouped<Cfg, false, true>(p, ctas, st)
-                  : launch_grouped<Cfg, false, false>(p, ctas, st);
+  const bool early = d->early != 0;
+  p.early = d->early;
+  if (d->down) return launch_grouped<Cfg, true>(p, ctas, early, st);
+  return d->gated ? launch_grouped<Cfg, false, true>(p, ctas, early, st)
+                  : launch_grouped<Cfg, false, false>(p, ctas, early, st);
 }
 }  // namespace cb
 

@@ -175,8 +175,7 @@ __global__ void __launch_bounds__(kSlotWarps * 32)
 //   send_row_base[E]    first destination row of my selections of expert e (at rank e/El)
 //   recv_expected[El]   rows that will arrive for my local expert j
 //   recv_base[El+1]     padded first row of my local expert j (last = total padded rows)
-//   mblk_expert[...]    local expert of each 128-row block of my receive buffer; from bit 16 on the groups of
-//                       32 rows of the block that hold any
+//   mblk_expert[...]    local expert of each 128-row block of my receive buffer
 //   n_mblocks[1]
 // One CTA; E <= 1024.
 __global__ void __launch_bounds__(256)
@@ -222,10 +221,7 @@ __global__ void __launch_bounds__(256)
     const int b0 = base_sh[rank * El + j] / 128;
     const int nb = (rows_sh[rank * El + j] + 127) / 128;
     for (int b = 0; b < nb; ++b)
-      if ((b0 + b) * 128 < max_recv_rows) {
-        const int rows = min(rows_sh[rank * El + j] - b * 128, 128);
-        mblk_expert[b0 + b] = j | (rows + 31) / 32 << 16;
-      }
+      if ((b0 + b) * 128 < max_recv_rows) mblk_expert[b0 + b] = j;
   }
 }
 

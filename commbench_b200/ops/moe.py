@@ -61,7 +61,7 @@ class _GroupedDesc(C.Structure):
     _fields_ = [
         ("max_rows", C.c_int), ("N", C.c_int), ("K", C.c_int), ("n_local_experts", C.c_int),
         ("down", C.c_int), ("rank", C.c_int), ("world", C.c_int), ("ctas", C.c_int),
-        ("gated", C.c_int), ("narrow", C.c_int),
+        ("gated", C.c_int), ("narrow", C.c_int), ("early", C.c_int),
         ("a", C.c_void_p), ("b", C.c_void_p), ("c", C.c_void_p),
         ("mblk_expert", C.c_void_p), ("n_mblocks", C.c_void_p), ("recv_meta", C.c_void_p),
         ("combine_peer", _P8), ("done_peer", _P8), ("done_ctas", C.c_void_p),
@@ -206,6 +206,7 @@ class MoELayer:
                        for r in range(self.W if self.emu else 1)]
         self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
         rows = tokens * topk / self.El
+        self.weights_early = rows <= 96      # a decode step: the products are bound by reading weights
         self.narrow_up = narrow_tiles(rows, self.El, 2 * intermediate, self.sms)
         self.narrow_down = narrow_tiles(rows, self.El, hidden, self.sms)
         torch.cuda.synchronize(dev)
@@ -319,7 +320,7 @@ class MoELayer:
                 d.gated, d.a, d.b, d.c = 1, st.a.data_ptr(), st.w1_gated.data_ptr(), st.s.data_ptr()
             else:
                 d.gated, d.a, d.b, d.c = 0, st.a.data_ptr(), st.w1.data_ptr(), st.h1.data_ptr()
-            d.narrow = int(self.narrow_up)
+            d.narrow, d.early = int(self.narrow_up), int(self.weights_early)
             d.mblk_expert, d.n_mblocks = st.mblk_expert.data_ptr(), st.n_mblocks.data_ptr()
             d.status = self._status(st)
             N.check(lib.cb_moe_grouped_gemm(C.byref(d), sp), "grouped gemm (up)")
@@ -333,7 +334,7 @@ class MoELayer:
             d2.max_rows, d2.N, d2.K, d2.n_local_experts = self.max_rows, H, I, self.El
             d2.down, d2.rank, d2.world, d2.ctas = 1, st.r, W, self.sms
             d2.a, d2.b, d2.c = st.s.data_ptr(), st.w2.data_ptr(), 0
-            d2.narrow = int(self.narrow_down)
+            d2.narrow, d2.early = int(self.narrow_down), int(self.weights_early)
             d2.mblk_expert, d2.n_mblocks = st.mblk_expert.data_ptr(), st.n_mblocks.data_ptr()
             d2.recv_meta = self._local(self.recv_meta, st).data_ptr()
             d2.combine_peer, d2.done_peer = _P8(*self.combine.ptrs), _P8(*self.done.ptrs)

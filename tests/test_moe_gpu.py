@@ -160,9 +160,9 @@ def test_moe_layer_on_one_real_rank(native_lib, dispatch):
 
 @pytest.mark.parametrize("fused_swiglu", [True, False])
 @pytest.mark.parametrize("narrow", [False, True])
-def test_grouped_gemm_at_row_counts_around_its_boxes(native_lib, narrow, fused_swiglu):
-    """Experts with 0, 1, 31 ... 385 rows (operand boxes of 32 rows, row blocks of 128), tiles of 256 and of
-    128 columns."""
+def test_grouped_gemm_forms_at_ragged_row_counts(native_lib, narrow, fused_swiglu):
+    """Experts with 0, 1, 31 ... 385 rows, tiles of 256 and of 128 columns, weights fetched before the wait for
+    the kernel before and after it."""
     from commbench_b200.ops.moe import MoELayer, reference_moe
     from commbench_b200.runtime.context import CommContext
 
@@ -175,7 +175,7 @@ def test_grouped_gemm_at_row_counts_around_its_boxes(native_lib, narrow, fused_s
     x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
     ctx = CommContext(heap_bytes=64 << 20)
     layer = MoELayer(ctx, T, H, I, E, 1, seed=3, fused_swiglu=fused_swiglu)
-    layer.narrow_up = layer.narrow_down = narrow
+    layer.narrow_up = layer.narrow_down = layer.weights_early = narrow
     w1, w2 = layer.weights()
     ref = reference_moe(x, idx, w, w1, w2, I)
     for _ in range(2):
@@ -184,7 +184,9 @@ def test_grouped_gemm_at_row_counts_around_its_boxes(native_lib, narrow, fused_s
         ctx.check_status()
         # bf16 roundings of the two products, as in the layer's other tests
         assert (y - ref).abs().max().item() < 3e-2 * ref.abs().max().item()
-    layer.narrow_up = layer.narrow_down = not narrow
-    assert torch.equal(layer.forward(x, idx, w).float(), y)    # same K order: the same bits
+    for layer.narrow_up in (False, True):
+        for layer.weights_early in (False, True):
+            layer.narrow_down = not layer.narrow_up
+            assert torch.equal(layer.forward(x, idx, w).float(), y)    # same K order: the same bits
     torch.cuda.synchronize()
     ctx.close()
