@@ -215,6 +215,11 @@ struct GemmChoice {
   int bn;      // persistent: 64 ... 512 as in cb_gemm_bf16; small kernel: its tile width
   int split;   // 0: persistent kernel; else the small kernel's K splits
 };
+// Two limits that a loop meets together: a little above the larger one.
+static float both_us(float a, float b) {
+  const float a3 = a * a * a, b3 = b * b * b;
+  return cbrtf(sqrtf(a3 * a3 + b3 * b3));
+}
 static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
   const float nkb = static_cast<float>((kbytes + 127) / 128);
   const float l2_rate = kbytes % 128 == 0 ? 17e6f : 11e6f;   // bytes per us
@@ -261,7 +266,7 @@ static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
                                       : (split == 8 ? 3.7f : 1.7f) + tile_kb * 0.05f *
                                             static_cast<float>(split - 1) / static_cast<float>(split);
       const float steps = static_cast<float>((static_cast<int>(nkb) + split - 1) / split);
-      offer(widths[i], split, 2.7f + fmaxf(steps * per_kb, hbm_us) + reduce);
+      offer(widths[i], split, 2.7f + both_us(steps * per_kb, hbm_us) + reduce);
     }
   return best;
 }
@@ -301,6 +306,7 @@ static int run_small(const void* a, const void* b, void* c, int M, int N, int K,
   const TmapDtype dt = FP8 ? TMAP_U8 : TMAP_BF16;
   const unsigned long long pitch = static_cast<unsigned long long>(K) * (FP8 ? 1 : 2);
   p.a_rows = M < Cfg::BM ? (M + 7) / 8 * 8 : Cfg::BM;
+  p.stages = Cfg::stages(p.a_rows);
   if (make_tmap_2d(&p.tm_a, a, dt, K, M, pitch, Cfg::BK, static_cast<unsigned>(p.a_rows), true))
     return -1;
   if (make_tmap_2d(&p.tm_b, b, dt, K, N, pitch, Cfg::BK, Cfg::BN, true)) return -1;

@@ -11,7 +11,9 @@
 //     atomics, the same bits every time;
 //   * hands operands over KPS K blocks at a time: one wait, one election, one commit for 4 x KPS MMAs;
 //   * loads only the rows of A that exist (a box of M rounded up to 8), since the rows beyond are never
-//     stored;
+//     stored, into ring slots of that height: with 48 rows 7 instead of 4 slots of two 64-wide K blocks, so that
+//     more weights are on their way (bound by them: 48 x 3584 x 8192 in 64-wide tiles 16.6 -> 15.9 us, 128-wide
+//     15.5 -> 14.8, 48 x 8192 x 3584 14.3 -> 13.8, all with weights out of memory);
 //   * is chained with programmatic dependent launch, so that its set-up overlaps the tail of the
 //     kernel before.
 // One tile per cluster.  Every mbarrier wait is bounded; an abort leaves through the cluster barriers.
@@ -40,9 +42,19 @@ struct SmallCfg {
   static constexpr int KB_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGE_BYTES = KPS * KB_BYTES;
   static constexpr int PITCH = BN_ + 4;                    // floats per staged row: no bank conflicts
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
+  static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
+  static constexpr int MAX_STAGES = 12;
+  static constexpr int SMEM_BYTES = RING_BYTES + 1024;
+  // Ring slots for A boxes of a_rows rows.  The MMA reads 128 rows from an A slot's start: what follows the
+  // rows that were loaded is other operands, whose products are never stored, but it has to lie in the ring.
+  static constexpr int stages(int a_rows) {
+    const int kb = a_rows * 128 + B_BYTES;
+    const int beyond = A_BYTES > kb ? A_BYTES - kb : 0;
+    const int n = (RING_BYTES - beyond) / (KPS * kb);
+    return n < MAX_STAGES ? n : MAX_STAGES;
+  }
   static constexpr int THREADS = 192;                      // producer, MMA, 4 epilogue warps
-  static_assert(BM * PITCH * 4 <= STAGES * STAGE_BYTES, "the staged tile reuses the operand ring");
+  static_assert(BM * PITCH * 4 <= RING_BYTES, "the staged tile reuses the operand ring");
   static_assert(SMEM_BYTES <= 232448 - 256, "over the 227 KB shared-memory limit");
 };
 
@@ -51,13 +63,14 @@ struct SmallParams {
   __nv_bfloat16* c;
   int M, N, num_m, num_kb;  // K blocks of the whole product
   int a_rows;               // rows of the A box
+  int stages;               // ring slots: Cfg::stages(a_rows)
   float alpha;
   uint32_t* status;
 };
 
 template <class Cfg>
 struct SmallCtl {
-  uint64_t full[Cfg::STAGES], empty[Cfg::STAGES], done;
+  uint64_t full[Cfg::MAX_STAGES], empty[Cfg::MAX_STAGES], done;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -88,7 +101,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
   if (threadIdx.x == 0) {
     tmap_prefetch(&p.tm_a);
     tmap_prefetch(&p.tm_b);
-    for (int s = 0; s < Cfg::STAGES; ++s) {
+    for (int s = 0; s < p.stages; ++s) {
       mbar_init(&ctl.full[s], 1);
       mbar_init(&ctl.empty[s], 1);
     }
@@ -104,14 +117,16 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&ctl.tmem_base);
+  const uint32_t a_bytes = static_cast<uint32_t>(p.a_rows) * 128u;
+  const uint32_t kb_step = a_bytes + Cfg::B_BYTES, stage_step = Cfg::KPS * kb_step;
+  const uint32_t stages = static_cast<uint32_t>(p.stages);
   pdl_launch_dependents();
   pdl_wait();   // operands, and readers of C, of the kernels before
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     const uint32_t ring_addr = smem_u32(ring), full0 = smem_u32(&ctl.full[0]);
-    const uint32_t kb_bytes = static_cast<uint32_t>(p.a_rows) * 128u + Cfg::B_BYTES;
-    uint32_t stage = 0, phase = 0;
+    uint32_t stage = 0, phase = 0, slot = ring_addr;
     for (int kb = 0; kb < nkb; kb += Cfg::KPS) {
       if (!mbar_wait_traced(&ctl.empty[stage], phase ^ 1u, &ctl.abort_flag, p.status, 0x100 + stage,
                             false, nullptr))
@@ -119,19 +134,21 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
       if (elect_one()) {
         const int sub = nkb - kb < Cfg::KPS ? nkb - kb : Cfg::KPS;
         const uint32_t bar = full0 + stage * 8u;
-        mbar_arrive_expect_tx_addr(bar, kb_bytes * sub);
+        mbar_arrive_expect_tx_addr(bar, kb_step * sub);
 #pragma unroll
         for (int i = 0; i < Cfg::KPS; ++i) {
           if (i >= sub) break;
-          const uint32_t sa = ring_addr + stage * Cfg::STAGE_BYTES + i * Cfg::KB_BYTES;
+          const uint32_t sa = slot + i * kb_step;
           const int x = (kb0 + kb + i) * Cfg::BK;
-          tma_load_2d_addr(sa + Cfg::A_BYTES, &p.tm_b, x, n_blk * Cfg::BN, bar);
+          tma_load_2d_addr(sa + a_bytes, &p.tm_b, x, n_blk * Cfg::BN, bar);
           tma_load_2d_addr(sa, &p.tm_a, x, m_blk * Cfg::BM, bar);
         }
       }
       __syncwarp();
-      if (++stage == Cfg::STAGES) {
+      slot += stage_step;
+      if (++stage == stages) {
         stage = 0;
+        slot = ring_addr;
         phase ^= 1u;
       }
     }
@@ -140,6 +157,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
     constexpr uint32_t idesc = make_idesc(Cfg::BM, Cfg::BN, Cfg::FP8 ? 0u : 1u);
     const uint64_t a_desc0 = make_sw128_kmajor_desc(smem_u32(ring));
     uint32_t stage = 0, phase = 0;
+    const uint64_t kb_desc = kb_step >> 4, b_desc = a_bytes >> 4, stage_desc = stage_step >> 4;
+    uint64_t a_desc = a_desc0;
     bool ok = true;
     for (int kb = 0; kb < nkb; kb += Cfg::KPS) {
       if (!mbar_wait_traced(&ctl.full[stage], phase, &ctl.abort_flag, p.status, 0x300 + stage, false,
@@ -148,14 +167,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
         break;
       }
       tc_fence_after_sync();
-      const uint64_t a_desc = a_desc0 + stage * static_cast<uint64_t>(Cfg::STAGE_BYTES >> 4);
       const int sub = nkb - kb < Cfg::KPS ? nkb - kb : Cfg::KPS;
       if (elect_one()) {
 #pragma unroll
         for (int i = 0; i < Cfg::KPS; ++i) {
           if (i >= sub) break;
-          const uint64_t ad = a_desc + i * static_cast<uint64_t>(Cfg::KB_BYTES >> 4);
-          const uint64_t bd = ad + static_cast<uint64_t>(Cfg::A_BYTES >> 4);
+          const uint64_t ad = a_desc + i * kb_desc;
+          const uint64_t bd = ad + b_desc;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const uint32_t accum = (kb > 0 || i > 0 || k > 0) ? 1u : 0u;
@@ -168,8 +186,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
         mma_commit(&ctl.empty[stage]);
       }
       __syncwarp();
-      if (++stage == Cfg::STAGES) {
+      a_desc += stage_desc;
+      if (++stage == stages) {
         stage = 0;
+        a_desc = a_desc0;
         phase ^= 1u;
       }
     }

@@ -412,3 +412,28 @@ def test_fp8_gemm_with_hardware_block_scales_224_wide(native_lib, n):
     _check(out, _bs_reference(aq, as_, bq, bs), 1e-2)
     # the same K order on one CTA per 128 x 192 tile: the same bits
     assert torch.equal(out, gemm_fp8_mx(aq, asf, bq, bsf, pair=False))
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("m", [1, 8, 9, 40, 65, 120, 121, 128, 130])
+def test_small_gemm_ring_slots_of_every_height(native_lib, m, bn, fp8):
+    """Ring slots follow the rows of A, 10 of them at one row and 3 or 4 at 128: K long enough to go round
+    several times, and short enough to leave slots unused."""
+    from commbench_b200 import _native as N
+
+    lib = N.load()
+    for n, k in ((264, 2704), (64, 80)):
+        g = torch.Generator(device="cuda").manual_seed(m + n)
+        a = torch.randint(-3, 4, (m, k), device="cuda", generator=g).float()
+        b = torch.randint(-3, 4, (n, k), device="cuda", generator=g).float()
+        dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
+        aq, bq = a.to(dt), b.to(dt)
+        for split in (1, 4):
+            if split > (k * aq.element_size() + 127) // 128:
+                continue
+            out = torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+            N.check(lib.cb_gemm_small(aq.data_ptr(), bq.data_ptr(), out.data_ptr(), m, n, k, 1.0, int(fp8), bn,
+                                      split, 0, N.raw_stream()), "cb_gemm_small")
+            # |sums| < 9 * 2704 are exact in fp32
+            assert torch.equal(out.float(), _ref(a, b).bfloat16().float()), (n, k, split)
