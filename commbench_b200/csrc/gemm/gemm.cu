@@ -203,14 +203,14 @@ static long long pair_waves(long long m256, int N, int bn, int sms) {
 
 // Which kernel and tile a GEMM runs on, by a model of its time in microseconds.  kbytes: bytes of one
 // K row (K x element size).  Per-128-byte-K-block times of a CTA that nothing else holds up, measured on
-// one m-block: persistent pairs on 256 x 256 tiles 0.30, single CTAs 0.36, the small kernel's 64 / 128 /
-// 256-wide tiles 0.16 / 0.22 / 0.34 (0.18 / 0.30 / 0.50 where rows do not start on 128-byte lines, since
-// every box row then touches two); all CTAs together draw at most 17 TB/s out of L2 (11), weights
+// one m-block: persistent pairs on 256 x 256 tiles 0.315, single CTAs 0.33, the small kernel's 64 / 128 /
+// 256-wide tiles 0.16 / 0.21 / 0.34 (0.19 / 0.30 / 0.485 where rows do not start on 128-byte lines, since
+// every box row then touches two); all CTAs together draw at most 17 TB/s out of L2 (12.5), weights
 // arrive at 6 TB/s from memory, and a persistent tile takes 2.5 us however short its K loop
-// (its epilogue).  Over 105 random shapes (M 1-8192, N 512-16384, K 512-8192, bf16 and fp8), called in
-// a row, the choice takes 3.5 % more than the best of all variants on (geometric) average and over 10 %
-// more for 17 of them; the worst is 593 x 3696 x 1200, where it picks pairs (14.5 us) and 128-wide tiles
-// of the small kernel take 9.0.
+// (its epilogue).  Over 150 random shapes (M 1-8192, N 512-16384, K 512-8192, bf16 and fp8), called in
+// a row with three sets of operands in turn, the choice takes 1.0 % more than the best of all variants on
+// (geometric) average and over 5 % more for 9 of them (1.8 % and 18 with the constants of before: pairs 0.30,
+// single CTAs 0.36, 11 TB/s); the worst is 6 x 1792 x 5456, 8.0 us in four parts and 6.1 in eight.
 struct GemmChoice {
   int bn;      // persistent: 64 ... 512 as in cb_gemm_bf16; small kernel: its tile width
   int split;   // 0: persistent kernel; else the small kernel's K splits
@@ -222,7 +222,7 @@ static float both_us(float a, float b) {
 }
 static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
   const float nkb = static_cast<float>((kbytes + 127) / 128);
-  const float l2_rate = kbytes % 128 == 0 ? 17e6f : 11e6f;   // bytes per us
+  const float l2_rate = kbytes % 128 == 0 ? 17e6f : 12.5e6f;   // bytes per us
   const float hbm_us = static_cast<float>(N) * static_cast<float>(kbytes) / 6e6f;
   const long long m128 = (M + 127) / 128, m256 = (M + 255) / 256;
   GemmChoice best = {512, 0};
@@ -234,25 +234,25 @@ static GemmChoice choose_gemm(int M, int N, long long kbytes, int sms) {
     }
   };
   {  // persistent kernels: pairs on 256 x 256 and 256 x 224, single CTAs on 128 x 256
-    // (224 from 32 K blocks on: in short loops the epilogue counts, which gains nothing)
-    for (int bn = 256; bn >= (nkb >= 32.f ? 224 : 256); bn -= 32) {
+    // (224 from 18 K blocks on: in shorter loops the epilogue counts, which gains nothing)
+    for (int bn = 256; bn >= (nkb >= 18.f ? 224 : 256); bn -= 32) {
       const long long pairs = m256 * ((N + bn - 1) / bn);
       const float pair_ctas = 2.f * static_cast<float>(pairs < sms / 2 ? pairs : sms / 2);
       const float cta_bytes = static_cast<float>(128 + bn / 2) * 128.f;   // per CTA and K block
       const float pair_kb =
-          fmaxf(0.30f * pair_tile_cost(bn) / pair_tile_cost(256), pair_ctas * cta_bytes / l2_rate);
+          fmaxf(0.315f * pair_tile_cost(bn) / pair_tile_cost(256), pair_ctas * cta_bytes / l2_rate);
       const float waves = static_cast<float>(pair_waves(m256, N, bn, sms));
-      offer(2 * bn, 0, 7.f + fmaxf(waves * fmaxf(nkb * pair_kb, 2.5f), hbm_us));
+      offer(2 * bn, 0, 7.7f + fmaxf(waves * fmaxf(nkb * pair_kb, 2.5f), hbm_us));
     }
     const long long singles = m128 * ((N + 255) / 256), sw = (singles + sms - 1) / sms;
     const float single_ctas = static_cast<float>(singles < sms ? singles : sms);
-    const float single_kb = fmaxf(0.36f, single_ctas * 49152.f / l2_rate);
+    const float single_kb = fmaxf(0.33f, single_ctas * 49152.f / l2_rate);
     offer(256, 0, 6.5f + fmaxf(static_cast<float>(sw) * fmaxf(nkb * single_kb, 2.5f), hbm_us));
   }
   const int a_rows = M < 128 ? (M + 7) / 8 * 8 : 128;
   const int widths[3] = {64, 128, 256};
   const bool lines = kbytes % 128 == 0;
-  const float kb_us[3] = {lines ? 0.16f : 0.18f, lines ? 0.22f : 0.30f, lines ? 0.34f : 0.50f};
+  const float kb_us[3] = {lines ? 0.16f : 0.19f, lines ? 0.21f : 0.30f, lines ? 0.34f : 0.485f};
   for (int i = 0; i < 3; ++i)
     for (int split = 1; split <= 8; split *= 2) {
       if (static_cast<float>(split) > nkb) break;
