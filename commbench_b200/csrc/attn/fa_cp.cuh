@@ -201,19 +201,6 @@ __device__ __forceinline__ void cp_add_sums(const uint64_t (&sum4)[4], float& l)
   l += __uint_as_float(static_cast<uint32_t>(a)) + __uint_as_float(static_cast<uint32_t>(a >> 32));
 }
 
-// All of it on a row that is complete.  Warp-collective.
-template <int kPoly>
-__device__ __forceinline__ void cp_online_softmax(uint32_t (&s)[128], uint32_t tO, float scale_log2,
-                                                  bool need_mask, bool rescale_o, bool votes,
-                                                  float& m_ref, float& l) {
-  float mx8[8];
-  cp_row_max(s, mx8);
-  cp_update_max(mx8, tO, scale_log2, rescale_o, votes, m_ref, l);
-  uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
-  cp_probabilities<kPoly, 0, 128>(s, scale_log2, m_ref, need_mask, sum4);
-  cp_add_sums(sum4, l);
-}
-
 // Walks the key blocks that a query tile pair attends to, segment by segment.  Every role of a
 // CTA runs its own copy and sees the same sequence.  Both tiles of the pair visit the same
 // blocks: a block that lies wholly in the future of the first tile (at most one per item, the

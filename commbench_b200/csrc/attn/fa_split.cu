@@ -87,7 +87,7 @@ struct SplitCtl {
   uint64_t q_full[2], q_empty[2];
   uint64_t k_full[CP_KST], k_empty[CP_KST];
   uint64_t v_full[CP_VST], v_empty[CP_VST];
-  uint64_t s_full[2], p_full[2], pv_done[2];   // per stream
+  uint64_t s_full[2], p_first[2], p_rest[2], pv_done[2];   // per stream; P in halves of 64 keys
   uint64_t seg_full, seg_done;   // both streams' O and (max, sum) of a segment: complete, read
   float2 ml[2][CP_BM];           // (max, sum) of the segment per stream and row
   uint32_t tmem_base;
@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
       mbar_init(&ctl.q_full[i], 1);
       mbar_init(&ctl.q_empty[i], 1);
       mbar_init(&ctl.s_full[i], 1);
-      mbar_init(&ctl.p_full[i], active);
+      mbar_init(&ctl.p_first[i], active);
+      mbar_init(&ctl.p_rest[i], active);
       mbar_init(&ctl.pv_done[i], 1);
     }
     ctl.abort_flag = 0;
@@ -283,7 +284,8 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
       };
       auto issue_pv = [&](int j) -> bool {
         const int g = g0 + j, s = g % CP_VST, t = j & 1;
-        if (!wait_all(&ctl.p_full[t], pv_count[t] & 1u, 0xF20 + t)) return false;
+        const uint32_t par = pv_count[t] & 1u;
+        if (!wait_all(&ctl.p_first[t], par, 0xF20 + t)) return false;
         if (!wait_all(&ctl.v_full[s], (g / CP_VST) & 1, 0xF22)) return false;
         ++pv_count[t];
         tc_fence_after_sync();
@@ -291,9 +293,19 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
           const uint64_t va = v_desc0 + s * kTileStep;
           const uint32_t d = tmem + 256u * t + 128u;
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
+          for (int kk = 0; kk < 4; ++kk)
             mma_bf16_ts(d, tmem + 256u * t + 8u * kk, va + kk * (2048u >> 4), idesc_pv,
                         (j > 1 || kk > 0) ? 1u : 0u);
+        }
+        __syncwarp();
+        if (!wait_all(&ctl.p_rest[t], par, 0xF24 + t)) return false;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          const uint64_t va = v_desc0 + s * kTileStep;
+          const uint32_t d = tmem + 256u * t + 128u;
+#pragma unroll
+          for (int kk = 4; kk < 8; ++kk)
+            mma_bf16_ts(d, tmem + 256u * t + 8u * kk, va + kk * (2048u >> 4), idesc_pv, 1u);
           mma_commit(&ctl.pv_done[t]);
           mma_commit(&ctl.v_empty[s]);
         }
@@ -309,7 +321,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
         for (int j = 0; ok && j < 2 && j < w.n; ++j) ok = issue_qk(j);
         for (int j = 0; ok && j < w.n; ++j) {
           // A stream's first product of a segment overwrites the O of its last one: that was read
-          // before its softmax warps hand over (p_full) the first block of this segment.
+          // before its softmax warps hand over (p_first) the first block of this segment.
           ok = issue_pv(j);
           if (ok && j + 2 < w.n) ok = issue_qk(j + 2);
         }
@@ -354,9 +366,12 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
         const int kv_left = pl.Skv - kb;
         const bool need_mask = kv_left < CP_BN || (pl.causal && key0 + CP_BN - 1 > tile_first);
         if (need_mask) cp_mask_tail(s, pl.causal ? min(kv_left, q_pos - key0 + 1) : kv_left);
-        cp_online_softmax<0>(s, tO, p.scale_log2, need_mask, j > 1, r < tile_rows, m_ref, l);
+        float mx8[8];
+        cp_row_max(s, mx8);
+        cp_update_max(mx8, tO, p.scale_log2, j > 1, r < tile_rows, m_ref, l);
+        uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
+        cp_probabilities<0, 0, 64>(s, p.scale_log2, m_ref, need_mask, sum4);
         tmem_st_32x32_at(tS, &s[0]);
-        tmem_st_32x32_at(tS + 32u, &s[32]);
         tmem_wait_st();
         // Both streams' O of the segment before must have been read before this hand-over.
         if (j < 2 && seg > 0 &&
@@ -366,7 +381,14 @@ __global__ void __launch_bounds__(CP_THREADS, 1)
         }
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl.p_full[t]);
+        if (lane == 0) mbar_arrive(&ctl.p_first[t]);
+        cp_probabilities<0, 64, 128>(s, p.scale_log2, m_ref, need_mask, sum4);
+        tmem_st_32x32_at(tS + 32u, &s[32]);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.p_rest[t]);
+        cp_add_sums(sum4, l);
       }
       if (!ok) break;
       // -------------------------------------------- end of the segment: merge the streams
