@@ -43,17 +43,18 @@ namespace cb {
 static constexpr int SP_MAX_QT = 64;                                 // query tiles per batch and head
 static constexpr int SP_ITEM_COST = 3;
 static constexpr int SP_MERGE_THREADS = 128;
-// Microseconds of a unit, of the merge and of a launch's start and end on the device.
-static constexpr float SP_BLOCK_US = 1.5f, SP_MERGE_US = 5.f, SP_START_US = 6.f;
+// Microseconds of a unit, of a unit of a decode call (one tile with few rows: an item of 6 blocks took 10.7 in
+// all), of the merge and of a launch's start and end on the device.
+static constexpr float SP_BLOCK_US = 1.35f, SP_DECODE_US = 0.85f, SP_MERGE_US = 6.5f, SP_START_US = 5.7f;
 
 // What a call takes when calls follow each other: on the device, but no less than on the host, where a
-// cut costs a workspace and a second launch (measured through flash_attention, 16.5 and 21.5 us).  Calls that
+// cut costs a workspace and a second launch (measured through flash_attention, 7.1 and 11 us).  Calls that
 // are both bound by the host are told apart by the device.
 struct CallTime {
   float device;
   bool merge;
   bool better_than(const CallTime& o) const {
-    const float a = fmaxf(device, merge ? 21.f : 16.5f), b = fmaxf(o.device, o.merge ? 21.f : 16.5f);
+    const float a = fmaxf(device, merge ? 11.f : 7.5f), b = fmaxf(o.device, o.merge ? 11.f : 7.5f);
     return a < b || (a == b && device < o.device);
   }
 };
@@ -610,8 +611,8 @@ static bool split_plan(SplitPlan& pl, int B, int Sq, int Skv, int Hq, int Hkv, i
   if (pl.nqt == 1) {
     // Whole items per CTA when that costs less than the merge.
     const long long whole = (items + sms - 1) / sms * pl.nblk[0];
-    const CallTime uncut = {SP_START_US + SP_BLOCK_US * static_cast<float>(whole), false};
-    if (uncut.better_than({SP_START_US + SP_BLOCK_US * static_cast<float>(pl.per) + SP_MERGE_US, true}))
+    const CallTime uncut = {SP_START_US + SP_DECODE_US * static_cast<float>(whole), false};
+    if (uncut.better_than({SP_START_US + SP_DECODE_US * static_cast<float>(pl.per) + SP_MERGE_US, true}))
       pl.per = static_cast<int>(whole);
   }
   pl.ctas = static_cast<int>((total + pl.per - 1) / pl.per);
@@ -639,13 +640,14 @@ static int split_sms() {
 // Which kernel takes a call, from a model of both in microseconds.  The tile-pair kernel takes
 // kPairBlock for a key block of its 256 rows and is as long as its longest item or its share of all
 // of them; the split kernel takes SP_BLOCK_US for a unit of its 128 rows, plus the merge.
-// Measured on the device, split / pair (B, Sq, Skv, Hq, Hkv): (1, 64, 64, 4, 4) 7.6 / 9.0 us,
-// (1, 300, 300, 4, 1) 11 / 14 (with a merge, so a call takes 21.5 / 16.5), (1, 500, 4596, 8, 2)
-// 23 / 81, (1, 8192, 8192, 4, 4) 90 / 127; near the line (1, 1280, 1280, 16, 8) 33 / 30,
-// (1, 2000, 2777, 16, 4) 54 / 51, (1, 1000, 7000, 32, 8) 118 / 112; beyond it (2, 2000, 2000, 32, 8)
-// 125 / 88.
+// Measured, calls in a row, split / pair (B, Sq, Skv, Hq, Hkv): (1, 537, 537, 8, 2) 12.2 / 15.4 us,
+// (1, 8192, 8192, 4, 4) 93 / 128; near the line (1, 64, 64, 4, 4) 7.7 / 7.3, (1, 300, 300, 4, 1) 12.2 / 11.9,
+// (1, 896, 896, 16, 4) 20.3 / 19.4, (1, 1280, 1280, 16, 8) 27.7 / 26.3, (1, 2000, 2777, 16, 4) 52 / 47,
+// (1, 1000, 7000, 32, 8) 111 / 116; beyond it, every key visible, (2, 218, 995, 32, 8) 26.8 / 21.8.  Over 68
+// shapes of that range the choice takes 1.1 % more than the better kernel on average (2.1 % with the constants
+// of before the two kernels and their call path became faster).
 static bool split_wins(const SplitPlan& pl, int sms) {
-  constexpr float kPairBlock = 2.0f, kPairStart = 7.f;
+  constexpr float kPairBlock = 1.8f, kPairStart = 7.f;
   const float pair_tiles = static_cast<float>((pl.Sq + 2 * CP_BM - 1) / (2 * CP_BM));
   float blocks = 0.f;
   for (int i = 0; i < pl.nqt; ++i) blocks += static_cast<float>(pl.nblk[i]);
