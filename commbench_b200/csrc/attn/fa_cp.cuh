@@ -30,10 +30,10 @@
 //   * P is handed over in two halves of 64 keys: the product with the first runs while the exponentials of
 //     the second are taken.  16384 tokens, 32 / 8 heads, causal: 1790 -> 1705 us in a burst (1965 MHz), 2050 ->
 //     1965 us when such calls follow each other (1.6 GHz under the power cap).
-// What bounds the inner loop (3400 cycles for 128 keys x 256 rows against 2048 on the tensor cores): the MMA
-// warp, which is issuing for 3000 of them - 60 cycles for a product's MMA, about 115 for one of the scores,
-// whose two operands both come from shared memory, beside the 64 KB that arrive per block - and behind it a
-// tile's chain scores -> softmax (1700) -> P -> product -> next scores; without the exponentials 1670 us.
+// What bounds the inner loop: the MMA warp, and behind it a tile's chain scores -> softmax (1700) -> P ->
+// product -> next scores.  Traced before the halves, 128 keys x 256 rows took 3660 cycles against 2048 on the
+// tensor cores: the MMA warp waited 860, spent 960 on the 16 MMAs of the products and 1840 on all else up to
+// its next wait, the 16 MMAs of the scores among it; without the exponentials 1670 us instead of 1790.
 // Slower: CTA pairs, which halve the shared-memory traffic of K and V (1807 us: a pair's MMAs start too late
 // after each hand-over), three quarters of P first (1757), the loads of the scores in halves beside the
 // maximum, asking for K and V before P (1700 to 1720).
