@@ -211,6 +211,8 @@ struct GemmCtl {
 //                                              fills the ring with B of its first tile before it waits:
 //                                              neither B nor what num_tiles, tile_coord and b_row read is
 //                                              written by a kernel that may still run then
+//   optional: static constexpr int kBHalfStep  (one CTA per tile) not 0: the rows of a B tile are two runs of
+//                                              BN / 2, that far apart in map_b, whose box is BN / 2 rows high
 template <class Policy, class P>
 __host__ __device__ constexpr bool policy_early_b() {
   return requires(const P& p) { Policy::early_b(p); };
@@ -221,6 +223,15 @@ __host__ __device__ constexpr bool policy_pdl() {
     return Policy::kPdl;
   } else {
     return false;
+  }
+}
+
+template <class Policy>
+__host__ __device__ constexpr int policy_b_half_step() {
+  if constexpr (requires { Policy::kBHalfStep; }) {
+    return Policy::kBHalfStep;
+  } else {
+    return 0;
   }
 }
 
@@ -246,6 +257,13 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
   int ready_tiles = 0;
   // Pair: both CTAs' bytes are counted on the even CTA's barrier, the one its MMA warp waits on.
   const uint32_t full0_leader = Cfg::PAIR == 2 ? map_to_cta(full0, 0) : full0;
+  constexpr int kBHalfStep = policy_b_half_step<Policy>();
+  static_assert(kBHalfStep == 0 || (Cfg::PAIR == 1 && Cfg::B_BYTES / 2 % 1024 == 0),
+                "half tiles of B: one CTA per tile, on swizzle atoms");
+  const auto load_b = [&](uint32_t sb, const CUtensorMap* mb, int x, int brow, uint32_t bar) {
+    tma_load_2d_addr(sb, mb, x, brow, bar);
+    if constexpr (kBHalfStep != 0) tma_load_2d_addr(sb + Cfg::B_BYTES / 2, mb, x, brow + kBHalfStep, bar);
+  };
   [[maybe_unused]] int early = 0;   // K blocks whose B is on its way already
   if constexpr (policy_early_b<Policy, P>()) {
     static_assert(Cfg::PAIR == 1, "see early_b");
@@ -258,8 +276,8 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
       if (elect_one()) {
         for (int kb = 0; kb < early; ++kb) {
           mbar_arrive_expect_tx_addr(full0 + kb * 8u, Cfg::STAGE_BYTES);
-          tma_load_2d_addr(ring_addr + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, Policy::map_b(p), kb * Cfg::BK,
-                           brow, full0 + kb * 8u);
+          load_b(ring_addr + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, Policy::map_b(p), kb * Cfg::BK, brow,
+                 full0 + kb * 8u);
         }
       }
       __syncwarp();
@@ -305,7 +323,7 @@ __device__ __forceinline__ void gemm_producer(const P& p, const GemmShape& g, ui
           } else {
             mbar_arrive_expect_tx_addr(bar, Cfg::STAGE_BYTES);
             tma_load_2d_addr(sa, ma, kb * Cfg::BK, arow, bar);
-            tma_load_2d_addr(sb, mb, kb * Cfg::BK, brow, bar);
+            load_b(sb, mb, kb * Cfg::BK, brow, bar);
           }
         }
       }
@@ -978,8 +996,8 @@ __device__ __forceinline__ void gemm_signal(const P& p, GemmCtl<Cfg::STAGES>* ct
   }
 }
 
-// A policy may declare `static constexpr bool kGated = true`: every 128 columns of an accumulator tile
-// then hold 64 "gate" columns followed by the 64 "up" columns of the same outputs (the
+// A policy may declare `static constexpr bool kGated = true`: every BN-wide accumulator tile then
+// holds BN/2 "gate" columns followed by BN/2 "up" columns of the same output columns (the
 // weight rows are interleaved that way by the caller), and the TMA-store epilogue writes
 // silu(gate) * up - BN/2 output columns per tile - instead of the raw accumulator, so the
 // activation never makes a round trip through HBM.
@@ -1030,17 +1048,16 @@ __device__ __forceinline__ void gemm_epilogue_tma(const P& p, const GemmShape& g
     static_assert(!kGated || Cfg::BN % (2 * Cfg::EPI_COLS) == 0, "whole boxes of gate and up columns");
 #pragma unroll 1
     for (int c = 0; c < kBoxes; ++c) {
-      const uint32_t taddr =
-          tmem_base + ((q * 32u) << 16) + acc * Cfg::BN + c * Cfg::EPI_COLS * (kGated ? 2 : 1);
+      const uint32_t taddr = tmem_base + ((q * 32u) << 16) + acc * Cfg::BN + c * Cfg::EPI_COLS;
       uint32_t r0[32], r1[32];
       if constexpr (kGated) {
         uint32_t up[32];
         tmem_ld_32x32(taddr, r0);
-        tmem_ld_32x32(taddr + Cfg::EPI_COLS, up);
+        tmem_ld_32x32(taddr + Cfg::BN / 2, up);
         tmem_wait_ld();
         epi_gate_32(r0, up, g.alpha);
         tmem_ld_32x32(taddr + 32u, r1);
-        tmem_ld_32x32(taddr + Cfg::EPI_COLS + 32u, up);
+        tmem_ld_32x32(taddr + Cfg::BN / 2 + 32u, up);
         tmem_wait_ld();
         epi_gate_32(r1, up, g.alpha);
       } else {

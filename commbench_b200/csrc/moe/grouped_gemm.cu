@@ -54,12 +54,15 @@ struct GroupedParams {
 };
 
 // kGatedUp (up projection only): the weight slab of every expert is stored with its rows
-// interleaved - 64 gate rows, then the 64 up rows of the same outputs, and so on - and
-// the epilogue writes silu(gate) * up, [rows, N/2], so H1 never exists in memory.
+// interleaved - 128 gate rows, then the 128 up rows of the same outputs, and so on - and
+// the epilogue writes silu(gate) * up, [rows, N/2], so H1 never exists in memory.  A 256-wide tile
+// is such a block; a 128-wide one takes the same half of its gate and of its up rows, in two boxes.
 template <class Cfg, bool kDown, bool kGatedUp = false>
 struct GroupedPolicy {
   using P = GroupedParams;
   static constexpr bool kGated = kGatedUp;
+  static constexpr int kBHalfStep = kGatedUp && Cfg::BN == 128 ? 128 : 0;
+  static_assert(!kGatedUp || Cfg::BN == 128 || Cfg::BN == 256, "half a block of gate and up rows, or a whole one");
   static_assert(!(kDown && kGatedUp), "the gated epilogue belongs to the up projection");
   // The kernel before is the receive kernel or the other product: each releases its dependents after its own
   // wait, so the plan has been complete since then, and none of them writes weights.
@@ -79,7 +82,9 @@ struct GroupedPolicy {
   __device__ static const CUtensorMap* map_b(const P& p) { return &p.tm_b; }
   __device__ static int a_row(const P&, int m_blk) { return m_blk * Cfg::BM; }
   __device__ static int b_row(const P& p, int m_blk, int n_blk) {
-    return p.mblk_expert[m_blk] * p.g.N + n_blk * Cfg::BN;
+    const int first = p.mblk_expert[m_blk] * p.g.N;
+    if constexpr (kBHalfStep != 0) return first + (n_blk >> 1) * 256 + (n_blk & 1) * 64;
+    return first + n_blk * Cfg::BN;
   }
   __device__ static bool wait_a_ready(const P&, int, volatile int*) { return true; }
   static constexpr bool kDirect = kDown;
@@ -160,7 +165,7 @@ struct CbGroupedDesc {
   int down;          // 0: up projection (C local), 1: down projection with combine scatter
   int rank, world;
   int ctas;
-  int gated;         // up only: b is gate/up interleaved per 64 rows, c = silu(gate) * up
+  int gated;         // up only: b is gate/up interleaved per 256 rows, c = silu(gate) * up
   int narrow;        // 0: tiles of a row block x 256 columns; 1: of 128 columns
   int early;         // 1: starts while the kernel before ends and fetches weights first
   const void* a;     // [max_rows, K] bf16
@@ -180,8 +185,10 @@ struct CbGroupedDesc {
 namespace cb {
 template <class Cfg>
 static int run_grouped(const CbGroupedDesc* d, int ctas, cudaStream_t st) {
-  if (d->max_rows % 128 != 0 || d->K % 8 != 0 || d->N % Cfg::BN != 0) {
-    set_last_error("grouped gemm: max_rows % 128 == 0, K % 8 == 0, N % 256 == 0 required");
+  const int n_multiple = d->gated ? 256 : Cfg::BN;
+  if (d->max_rows % 128 != 0 || d->K % 8 != 0 || d->N % n_multiple != 0) {
+    set_last_error("grouped gemm: max_rows % 128 == 0, K % 8 == 0, N % " + std::to_string(n_multiple) +
+                   " == 0 required");
     return -1;
   }
   GroupedParams p;
@@ -189,7 +196,8 @@ static int run_grouped(const CbGroupedDesc* d, int ctas, cudaStream_t st) {
                    Cfg::BK, Cfg::BM, true))
     return -1;
   if (make_tmap_2d(&p.tm_b, d->b, TMAP_BF16, d->K, (unsigned long long)d->n_local_experts * d->N,
-                   (unsigned long long)d->K * 2, Cfg::BK, Cfg::BN, true))
+                   (unsigned long long)d->K * 2, Cfg::BK,
+                   d->gated && Cfg::BN == 128 ? Cfg::BN / 2 : Cfg::BN, true))
     return -1;
   if (d->gated && d->down) {
     set_last_error("grouped gemm: the gated epilogue belongs to the up projection");

@@ -95,11 +95,15 @@ def dispatch_layout(topk_idx: torch.Tensor, num_ranks: int, num_experts: int):
     return per_e, per_r, in_r
 
 
-def interleave_gate_up(w1: torch.Tensor, block: int = 128) -> torch.Tensor:
+GATE_BLOCK = 128     # rows of gate, then of up, in the row order of the gated up projection
+
+
+def interleave_gate_up(w1: torch.Tensor, block: int = GATE_BLOCK) -> torch.Tensor:
     """[E, 2I, H] with rows (gate | up) -> the same rows ordered per output block:
     gate rows j*block..(j+1)*block, then the up rows of the same outputs, for j = 0, 1, ...
-    One 2*block-row tile of the product then holds both halves of `block` outputs, which is what
-    the gated epilogue of the grouped GEMM combines into silu(gate) * up."""
+    In the default order a 256-row tile of the product, or the two 64-row halves that a 128-row tile loads,
+    holds both halves of its outputs, which is what the gated epilogue of the grouped GEMM combines into
+    silu(gate) * up."""
     E, two_i, H = w1.shape
     I = two_i // 2
     if I % block:
@@ -107,9 +111,6 @@ def interleave_gate_up(w1: torch.Tensor, block: int = 128) -> torch.Tensor:
     g = w1[:, :I].reshape(E, I // block, 1, block, H)
     u = w1[:, I:].reshape(E, I // block, 1, block, H)
     return torch.cat([g, u], dim=2).reshape(E, two_i, H).contiguous()
-
-
-GATE_BLOCK = 64      # rows of gate, then of up, in the row order of the gated up projection
 
 
 def narrow_tiles(avg_rows: float, experts: int, n: int, sms: int) -> bool:
@@ -156,7 +157,7 @@ class _RankState:
         self.w1 = (torch.randn(L.El, 2 * L.I, L.H, device=dev, generator=g) * 0.02).bfloat16()
         self.w2 = (torch.randn(L.El, L.H, L.I, device=dev, generator=g) * 0.02).bfloat16()
         # The gated up projection reads its own row order of the same weights (one more copy of w1).
-        self.w1_gated = interleave_gate_up(self.w1, GATE_BLOCK) if L.fused_swiglu else None
+        self.w1_gated = interleave_gate_up(self.w1) if L.fused_swiglu else None
 
 
 class MoELayer:

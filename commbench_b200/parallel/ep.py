@@ -124,7 +124,7 @@ class ExpertParallelMoE(MoELayer):
         ops = rearrange_expert_weights_inplace(self.placement, new_map, [st.w1, st.w2], self.El,
                                                group=group)
         if st.w1_gated is not None:
-            st.w1_gated = interleave_gate_up(st.w1, GATE_BLOCK)       # the gated copy follows its source
+            st.w1_gated = interleave_gate_up(st.w1)       # the gated copy follows its source
         moved = sum(1 for a, b in zip(self.placement, new_map) if a != b)
         self.placement = new_map
         inv = [0] * self.E

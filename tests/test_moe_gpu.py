@@ -190,3 +190,27 @@ def test_grouped_gemm_forms_at_ragged_row_counts(native_lib, narrow, fused_swigl
             assert torch.equal(layer.forward(x, idx, w).float(), y)    # same K order: the same bits
     torch.cuda.synchronize()
     ctx.close()
+
+
+@pytest.mark.parametrize("narrow", [False, True])
+def test_weights_in_the_default_gate_up_order(native_lib, narrow):
+    """interleave_gate_up's default order is the one that the gated product reads, whatever its tile width.
+    3e-2 of the largest value, as in the layer tests above."""
+    from commbench_b200.ops.moe import MoELayer, interleave_gate_up, reference_moe, router_topk
+    from commbench_b200.runtime.context import CommContext
+
+    T, H, I, E, K = 40, 512, 768, 8, 2
+    ctx = CommContext(heap_bytes=64 << 20)
+    layer = MoELayer(ctx, T, H, I, E, K, seed=5)
+    layer.narrow_up = narrow
+    g = torch.Generator(device="cuda").manual_seed(6)
+    w1, w2 = layer.weights()
+    w1.copy_(torch.randn(w1.shape, device="cuda", generator=g) * 0.02)
+    layer.states[0].w1_gated = interleave_gate_up(w1)
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    idx, w = router_topk(torch.randn(T, E, device="cuda", generator=g), K)
+    y = layer.forward(x, idx, w)
+    ref = reference_moe(x, idx, w, w1, w2, I)
+    assert (y.float() - ref).abs().max() <= 3e-2 * ref.abs().max()
+    ctx.check_status()
+    ctx.close()
