@@ -133,6 +133,13 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
     return lib
 
 
+def built_for() -> str:
+    """What the extension depends on besides its source: it uses PyTorch's C++ headers."""
+    import torch
+
+    return f"PyTorch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
 def build_fast(force: bool = False) -> Path:
     """Compiles the extension against the installed PyTorch and Python; both are part of its cache key."""
     import sysconfig
@@ -145,6 +152,7 @@ def build_fast(force: bool = False) -> Path:
     cuda = Path(nvcc_path()).resolve().parent.parent
     flags = ["-O2", "-std=c++20", "-fPIC", "-shared",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             f'-DCB_BUILT_FOR="{built_for()}"',
              "-I", sysconfig.get_paths()["include"], "-I", str(cuda / "include")]
     for inc in (home / "include", home / "include/torch/csrc/api/include"):
         flags += ["-isystem", str(inc)]

@@ -144,24 +144,42 @@ _FAST_ENTRIES = ("cb_gemm_bf16", "cb_gemm_fp8", "cb_gemm_fp8_blockscaled", "cb_g
                  "cb_attn_split_bytes", "cb_attn_split")
 
 
+class _NoFast:
+    """Stands in for an extension that is not there: takes no call."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def fast():
     """The extension with the short call path of the small operators (host/fast_ops.cpp).  Each of its
-    functions answers None for a call that it leaves to the general path."""
+    functions answers None for a call that it leaves to the general path.  So do all of them, after one
+    warning, where the extension is missing or was built for another PyTorch: the kernels are in the
+    library that :func:`load` opens, and only the host's share of a call gets longer."""
     global _fast
     if _fast is None:
         import importlib.machinery
         import importlib.util
+        import warnings
 
-        import torch  # noqa: F401  (the extension links against its libraries)
+        from . import _build
 
         lib = load()
-        if not _FAST_PATH.exists():
-            raise NativeError(f"{_FAST_PATH} is missing: run `python -m commbench_b200._build` first")
-        loader = importlib.machinery.ExtensionFileLoader("_fast_ops", str(_FAST_PATH))
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fast_ops", loader))
-        loader.exec_module(mod)
-        mod.bind({n: C.cast(getattr(lib, n), C.c_void_p).value for n in _FAST_ENTRIES})
-        _fast = mod
+        try:
+            if not _FAST_PATH.exists():
+                raise ImportError(f"{_FAST_PATH} is missing")
+            loader = importlib.machinery.ExtensionFileLoader("_fast_ops", str(_FAST_PATH))
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fast_ops", loader))
+            loader.exec_module(mod)
+            made_for = getattr(mod, "built_for", lambda: "an unknown PyTorch")()
+            if made_for != _build.built_for():
+                raise ImportError(f"{_FAST_PATH} was built for {made_for}, this is {_build.built_for()}")
+            mod.bind({n: C.cast(getattr(lib, n), C.c_void_p).value for n in _FAST_ENTRIES})
+            _fast = mod
+        except ImportError as e:
+            _fast = _NoFast()
+            warnings.warn(f"short call path off ({e}); `python -m commbench_b200._build` builds it",
+                          RuntimeWarning, stacklevel=2)
     return _fast
 
 

@@ -315,7 +315,11 @@ PyObject* fast_bind(PyObject*, PyObject* d) {
   Py_RETURN_NONE;
 }
 
+// built_for(): the PyTorch and Python whose headers this file was compiled with; asked before anything else.
+PyObject* fast_built_for(PyObject*, PyObject*) { return PyUnicode_FromString(CB_BUILT_FOR); }
+
 PyMethodDef methods[] = {
+    {"built_for", fast_built_for, METH_NOARGS, nullptr},
     {"bind", fast_bind, METH_O, nullptr},
     {"gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(fast_gemm)), METH_FASTCALL, nullptr},
     {"gemm_fp8_mx", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(fast_gemm_mx)), METH_FASTCALL, nullptr},
