@@ -94,6 +94,10 @@ def gemm_role_trace(a: torch.Tensor, b: torch.Tensor, bn: int = 512) -> dict:
 def quantize_blockscaled(x: torch.Tensor, row_block: int = 1):
     """bf16 [rows, K] -> (e4m3 [rows, K], fp32 scales).  ``row_block=1``: one scale per row and
     128 columns (activations, "1x128"); ``row_block=128``: one per 128x128 block (weights)."""
+    if row_block == 1:
+        r = N.fast().quantize_rows(x, False)
+        if r is not None:
+            return r
     lib = N.load()
     _check(x, "x")
     rows, K = x.shape

@@ -143,3 +143,36 @@ def test_short_path_follows_the_current_stream_and_is_captured(native_lib):
     cap.zero_()
     graph.replay()
     assert torch.equal(cap, ref)
+
+
+@pytest.mark.parametrize("i", range(11))
+def test_short_path_is_asked_and_answers(native_lib, monkeypatch, i):
+    """Every call that is compared with the general path above is one that the extension takes."""
+    from commbench_b200 import _native as N
+
+    ext, answers = N.fast(), []
+
+    class Spy:
+        def __getattr__(self, name):
+            def call(*args):
+                answers.append(getattr(ext, name)(*args))
+                return answers[-1]
+            return call
+
+    call = _calls()[i]
+    monkeypatch.setattr(N, "_fast", Spy())
+    call()
+    assert len(answers) == 1 and answers[0] is not None
+
+
+@pytest.mark.parametrize("rows,k", [(1, 128), (37, 256), (129, 640), (1000, 3584)])
+def test_row_quantiser_of_the_short_path(native_lib, monkeypatch, rows, k):
+    """Scales in fp32, at one row, ragged rows, K groups that are not whole, and rows of zeros."""
+    from commbench_b200.ops.gemm import quantize_blockscaled
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, k, device="cuda", generator=g).bfloat16()
+    x[rows // 2] = 0
+    fast = quantize_blockscaled(x, 1)
+    _general(monkeypatch)
+    _same(fast, quantize_blockscaled(x, 1))
