@@ -64,8 +64,9 @@ struct GroupedPolicy {
   static constexpr int kBHalfStep = kGatedUp && Cfg::BN == 128 ? 128 : 0;
   static_assert(!kGatedUp || Cfg::BN == 128 || Cfg::BN == 256, "half a block of gate and up rows, or a whole one");
   static_assert(!(kDown && kGatedUp), "the gated epilogue belongs to the up projection");
-  // The kernel before is the receive kernel or the other product: each releases its dependents after its own
-  // wait, so the plan has been complete since then, and none of them writes weights.
+  // The kernel before is the receive kernel, the other product or the SwiGLU kernel of the unfused form: each
+  // releases its dependents after its own wait or only by its end, so the plan has been complete since then,
+  // and none of them writes weights (prim/pdl.cuh).
   __device__ static bool early_b(const P& p) { return p.early != 0; }
   __device__ static int num_tiles(const P& p) {
     int mb = *reinterpret_cast<const volatile int*>(p.n_mblocks);

@@ -208,7 +208,6 @@ struct MoeRecvArgs {
 __global__ void __launch_bounds__(256)
     moe_recv_dequant_kernel(const __grid_constant__ MoeRecvArgs a) {
   pdl_wait();                // chained with programmatic dependent launch: see prim/pdl.cuh
-  pdl_launch_dependents();
   const int j = blockIdx.x;
   const int expect = a.recv_expected[j];
   const int base = a.recv_base[j];
@@ -234,6 +233,7 @@ __global__ void __launch_bounds__(256)
                           PH_MOE_ARRIVE2, j);
   }
   const bool all_ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  pdl_launch_dependents();   // not before: the product behind this kernel takes every SM's shared memory
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int nvec = a.H / 8;
@@ -329,12 +329,13 @@ __global__ void __launch_bounds__(256)
                               uint32_t* done_ctas, const __nv_bfloat16* __restrict__ bias0,
                               const __nv_bfloat16* __restrict__ bias1) {
   pdl_wait();                // chained with programmatic dependent launch: see prim/pdl.cuh
-  pdl_launch_dependents();
   bool ok = true;
   if (threadIdx.x < static_cast<unsigned>(world))
     ok = wait_flag_ge_sys(done + threadIdx.x, 1u, timeout_ns, status, PH_MOE_COMBINE2,
                           threadIdx.x);
-  if (__syncthreads_and(ok ? 1 : 0) != 0) {
+  const bool all_ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  pdl_launch_dependents();   // not before: what follows may take every SM's shared memory
+  if (all_ok) {
     // A warp takes 32 vectors of one token; eight of the token's K rows are loaded before the
     // first is added (a masked selection's row is loaded too and left out of the sum), so the
     // kernel is bound by bandwidth instead of by K dependent loads.  Measured at 4096 tokens, K = 8,

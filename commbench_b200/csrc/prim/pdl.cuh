@@ -4,8 +4,21 @@
 // writes are visible).  `pdl_launch_dependents()` lets the NEXT kernel of the stream be
 // scheduled from that point on, so its launch latency and prologue overlap this kernel.
 //
-// Every kernel of a chain calls pdl_wait() first thing, by every thread: a kernel that
-// skipped it could let its own dependents start before its predecessors have finished.
+// What a kernel may do before and after the two:
+//   * Every thread of a kernel launched this way calls pdl_wait() before it touches what an earlier kernel
+//     writes, or writes what one reads, and before the kernel ends: its end then stands for the end of all
+//     kernels before it.
+//   * Release first, wait then (GEMM, attention; the row quantiser, an ordinary launch, only releases): the next
+//     kernel may start before those further back have ended.  Right only because that kernel in its turn touches
+//     nothing of theirs before its own wait.
+//   * Wait first, release then (all kernels of the expert layer): the next kernel may rely, before its own wait,
+//     on all that the releasing kernel's predecessors wrote.  The expert products do: they read the plan and
+//     fetch weights first (early_b in gemm/gemm_sm100.cuh).  A kernel that is put before them keeps this order.
+//   * A kernel that waits for another rank releases after that wait.  The next kernel may hold the shared memory
+//     of every SM from its start on, and then the kernel that the other rank waits for, on another stream of
+//     this one, would find no room while both wait.
+// A released kernel's blocks occupy SMs while they wait: another stream's kernels get what is left until the
+// kernel in front has ended.
 //
 // The reference chains its small expert-parallel kernels the same way
 // (`cudaTriggerProgrammaticLaunchCompletion`: datasets/example079_deepep_jit_dispatch_notify/nv/

@@ -254,7 +254,9 @@ class MoELayer:
 
         The small kernels of the layer (slots, plan, dispatch, receive, combine reduction) are chained
         with programmatic dependent launch: each may be scheduled while its predecessor still runs
-        and waits on the device for it."""
+        and waits on the device for it.  A decode step's products take the shared memory of all SMs
+        while the kernel before them ends, but not while that one waits for other ranks, so layers on
+        several streams do not keep each other from running."""
         lib, W, E, K, T, H, I = self.lib, self.W, self.E, self.K, self.T, self.H, self.I
         if not self.emu:
             xs, topk_idx, topk_w = [xs], [topk_idx], [topk_w]
