@@ -43,13 +43,14 @@ namespace cb {
 static constexpr int SP_MAX_QT = 64;                                 // query tiles per batch and head
 static constexpr int SP_ITEM_COST = 3;
 static constexpr int SP_MERGE_THREADS = 128;
-// Microseconds of a unit, of a unit of a decode call (one tile with few rows: an item of 6 blocks took 10.7 in
-// all), of the merge and of a launch's start and end on the device.
-static constexpr float SP_BLOCK_US = 1.35f, SP_DECODE_US = 0.85f, SP_MERGE_US = 6.5f, SP_START_US = 5.7f;
+// Microseconds of a unit, of a unit where a batch and head has one query tile (an item of 6 blocks with few rows
+// took 10.7 in all), of the merge and of a launch's start and end on the device.
+static constexpr float SP_BLOCK_US = 1.35f, SP_ONE_TILE_US = 0.85f, SP_MERGE_US = 6.5f, SP_START_US = 5.7f;
 
 // What a call takes when calls follow each other: on the device, but no less than on the host, where a
-// cut costs a workspace and a second launch (measured through flash_attention, 7.1 and 11 us).  Calls that
-// are both bound by the host are told apart by the device.
+// cut costs a workspace and a second launch (measured through flash_attention, 7.1 and 11 us; with 7.5 a call
+// that is not cut and takes no longer on the device counts as bound by the host).  Calls that are both bound by
+// the host are told apart by the device.
 struct CallTime {
   float device;
   bool merge;
@@ -570,6 +571,9 @@ __global__ void __launch_bounds__(SP_MERGE_THREADS, 6)
         l > 0.f ? m * 0.6931471805599453f + logf(l) : -INFINITY;
 }
 
+// A call is cut, and given to this kernel, at one and the same price of a unit.
+static float unit_us(const SplitPlan& pl) { return pl.nqt == 1 ? SP_ONE_TILE_US : SP_BLOCK_US; }
+
 // Fills the plan; false when the call does not fit this kernel (or has no key block at all).
 static bool split_plan(SplitPlan& pl, int B, int Sq, int Skv, int Hq, int Hkv, int q_offset,
                        int kv_offset, int causal, int sms) {
@@ -611,8 +615,8 @@ static bool split_plan(SplitPlan& pl, int B, int Sq, int Skv, int Hq, int Hkv, i
   if (pl.nqt == 1) {
     // Whole items per CTA when that costs less than the merge.
     const long long whole = (items + sms - 1) / sms * pl.nblk[0];
-    const CallTime uncut = {SP_START_US + SP_DECODE_US * static_cast<float>(whole), false};
-    if (uncut.better_than({SP_START_US + SP_DECODE_US * static_cast<float>(pl.per) + SP_MERGE_US, true}))
+    const CallTime uncut = {SP_START_US + unit_us(pl) * static_cast<float>(whole), false};
+    if (uncut.better_than({SP_START_US + unit_us(pl) * static_cast<float>(pl.per) + SP_MERGE_US, true}))
       pl.per = static_cast<int>(whole);
   }
   pl.ctas = static_cast<int>((total + pl.per - 1) / pl.per);
@@ -639,11 +643,13 @@ static int split_sms() {
 
 // Which kernel takes a call, from a model of both in microseconds.  The tile-pair kernel takes
 // kPairBlock for a key block of its 256 rows and is as long as its longest item or its share of all
-// of them; the split kernel takes SP_BLOCK_US for a unit of its 128 rows, plus the merge.
+// of them; the split kernel takes unit_us for a unit of its 128 rows, plus the merge.
 // Measured, calls in a row, split / pair (B, Sq, Skv, Hq, Hkv): (1, 537, 537, 8, 2) 12.2 / 15.4 us,
 // (1, 8192, 8192, 4, 4) 93 / 128; near the line (1, 64, 64, 4, 4) 7.7 / 7.3, (1, 300, 300, 4, 1) 12.2 / 11.9,
 // (1, 896, 896, 16, 4) 20.3 / 19.4, (1, 1280, 1280, 16, 8) 27.7 / 26.3, (1, 2000, 2777, 16, 4) 52 / 47,
-// (1, 1000, 7000, 32, 8) 111 / 116; beyond it, every key visible, (2, 218, 995, 32, 8) 26.8 / 21.8.  Over 68
+// (1, 1000, 7000, 32, 8) 111 / 116; beyond it, every key visible, (2, 218, 995, 32, 8) 26.8 / 21.8; one query
+// tile, more items than SMs: (20, 1, 1275, 8, 8) 29 / 42, (24, 4, 1403, 8, 8) 36 / 47, (25, 128, 1275, 8, 8)
+// 37 / 47.  Over 68
 // shapes of that range the choice takes 1.1 % more than the better kernel on average (2.1 % with the constants
 // of before the two kernels and their call path became faster).
 static bool split_wins(const SplitPlan& pl, int sms) {
@@ -657,7 +663,7 @@ static bool split_wins(const SplitPlan& pl, int sms) {
   const float longest = static_cast<float>(pl.nblk[pl.nqt - 1]);
   const CallTime pair = {kPairStart + kPairBlock * (share > longest ? share : longest), false};
   const CallTime split = {SP_START_US + (pl.merge ? SP_MERGE_US : 0.f) +
-                              SP_BLOCK_US * static_cast<float>(pl.per),
+                              unit_us(pl) * static_cast<float>(pl.per),
                           pl.merge != 0};
   return split.better_than(pair);
 }

@@ -283,3 +283,15 @@ def test_attention_is_not_cut_where_the_host_bounds_the_call(native_lib, shape, 
     B, Sq, Skv, Hq, Hkv = shape
     nbytes = native_lib.cb_attn_split_bytes(B, Sq, Skv, Hq, Hkv, Skv - Sq, 0, 1)
     assert (nbytes == -1) if cut is None else (nbytes > 0) == cut and nbytes >= 0
+
+
+@pytest.mark.parametrize("rows", [1, 4, 32, 128])
+@pytest.mark.parametrize("items", [148, 149, 152, 176, 200, 295, 304, 1000])
+def test_one_query_tile_never_goes_to_the_tile_pair_kernel(native_lib, items, rows):
+    """The tile-pair kernel takes an item per SM at a time, with most of its 256 rows idle, and its heads do not
+    share keys: with one query tile for each batch and head the split-key kernel is the faster one however
+    many items there are."""
+    for blocks in range(1, 129):
+        for hq in (1, 4):
+            if rows % hq == 0:
+                assert native_lib.cb_attn_split_bytes(items, rows // hq, 128 * blocks - 5, hq, 1, 0, 0, 0) >= 0
