@@ -437,3 +437,22 @@ def test_small_gemm_ring_slots_of_every_height(native_lib, m, bn, fp8):
                                       split, 0, N.raw_stream()), "cb_gemm_small")
             # |sums| < 9 * 2704 are exact in fp32
             assert torch.equal(out.float(), _ref(a, b).bfloat16().float()), (n, k, split)
+
+
+@pytest.mark.parametrize("shape", [(8100, 3584, 1024), (8100, 3544, 1152), (8100, 3400, 1024), (1718, 4296, 640),
+                                   (1718, 4272, 128)])
+def test_hardware_block_scales_224_wide_where_the_choice_takes_them(native_lib, shape):
+    """At the shortest K of the rule and below it; the last column tile whole, ending inside its half box, inside
+    a whole box and nearly empty.  The same K order as on one CTA per 128 x 192 tile: the same bits."""
+    from commbench_b200.ops.gemm import gemm_fp8_mx, quantize_blockscaled_pow2
+
+    M, n, K = shape
+    assert native_lib.cb_gemm_mx_choice(M, n, K) == 224
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.randn(M, K, device="cuda", generator=g) * (1.0 + (torch.arange(M, device="cuda") % 7))[:, None]
+    b = torch.randn(n, K, device="cuda", generator=g) * 0.02 * (1 + torch.arange(n, device="cuda") // 128)[:, None]
+    aq, as_, asf = quantize_blockscaled_pow2(a.bfloat16().contiguous(), 1)
+    bq, bs, bsf = quantize_blockscaled_pow2(b.bfloat16().contiguous(), 128)
+    out = gemm_fp8_mx(aq, asf, bq, bsf)
+    _check(out, _bs_reference(aq, as_, bq, bs), 1e-2)
+    assert torch.equal(out, gemm_fp8_mx(aq, asf, bq, bsf, pair=False))

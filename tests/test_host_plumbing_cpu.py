@@ -295,3 +295,12 @@ def test_one_query_tile_never_goes_to_the_tile_pair_kernel(native_lib, items, ro
         for hq in (1, 4):
             if rows % hq == 0:
                 assert native_lib.cb_attn_split_bytes(items, rows // hq, 128 * blocks - 5, hq, 1, 0, 0, 0) >= 0
+
+
+@pytest.mark.parametrize("shape,width", [((4347, 8104, 768), 192), ((6993, 7504, 768), 192), ((6541, 5032, 128), 192),
+                                         ((1718, 4296, 768), 224), ((4347, 8104, 1024), 224),
+                                         ((8192, 3584, 8192), 224), ((2048, 4096, 4096), 192)])
+def test_short_products_with_block_scales_count_store_boxes(native_lib, shape, width):
+    """Tile width at 148 SMs, on either side of the rule for short K: 10 / 9 and 16 / 13 waves of 192 / 224
+    columns are slower in the wider form there, 3 / 2 are not."""
+    assert native_lib.cb_gemm_mx_choice(*shape) == width
