@@ -24,7 +24,7 @@
 //     from the CTA before and the one it hands on - so the workspace is two tiles per CTA, 20 MB
 //     at most, whatever the batch.
 // Measured, tile-pair kernel -> this, kernels alone: 16 sequences x 1 query over 6001 keys, 32 / 8 heads:
-// 398 -> 69 us (5.7 TB/s of 6.6; the call takes 78); 32 x 16384 keys, 64 / 8 heads: 3783 -> 325 us
+// 398 -> 69 us (5.7 TB/s of 6.6; calls in a row 76 to 78); 32 x 16384 keys, 64 / 8 heads: 3783 -> 325 us
 // (6.6 TB/s); 1 x 16384 keys, 8 / 8 heads: 259 -> 20 us.
 //
 // Every mbarrier wait is bounded (see mbarrier.cuh).

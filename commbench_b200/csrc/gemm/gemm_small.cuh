@@ -11,7 +11,7 @@
 //     atomics, the same bits every time;
 //   * hands operands over KPS K blocks at a time: one wait, one election, one commit for 4 x KPS MMAs;
 //   * loads only the rows of A that exist (a box of M rounded up to 8), since the rows beyond are never
-//     stored, into ring slots of that height: with 48 rows 7 instead of 4 slots of two 64-wide K blocks, so that
+//     stored, into ring slots of that height: with 48 rows 6 instead of 4 slots of two 64-wide K blocks, so that
 //     more weights are on their way (bound by them: 48 x 3584 x 8192 in 64-wide tiles 16.6 -> 15.9 us, 128-wide
 //     15.5 -> 14.8, 48 x 8192 x 3584 14.3 -> 13.8, all with weights out of memory);
 //   * is chained with programmatic dependent launch, so that its set-up overlaps the tail of the
@@ -43,7 +43,7 @@ struct SmallCfg {
   static constexpr int STAGE_BYTES = KPS * KB_BYTES;
   static constexpr int PITCH = BN_ + 4;                    // floats per staged row: no bank conflicts
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
-  static constexpr int MAX_STAGES = 12;
+  static constexpr int MAX_STAGES = 12;   // barriers of a ring: 10 slots with 8 rows of A in 64-wide tiles, 5 in others
   static constexpr int SMEM_BYTES = RING_BYTES + 1024;
   // Ring slots for A boxes of a_rows rows.  The MMA reads 128 rows from an A slot's start: what follows the
   // rows that were loaded is other operands, whose products are never stored, but it has to lie in the ring.

@@ -11,10 +11,12 @@
 // on the routing), and the tile list is simply (row block, column block).
 //
 // A decode step (early): each product starts as a programmatic dependent and fetches weights - which no kernel of
-// the layer writes - while the kernel before ends.  One rank, three layers' weights in turn: 16 tokens, top-8 of
-// 8 experts, hidden 7168, intermediate 2048 178 -> 173 us; 24, top-8 of 32, 2048 / 2048 214 -> 209; 52, top-4 of
-// 8, 4096 / 1024 104.6 -> 89; 100, top-8 of 32, 7168 / 2048 557 -> 552.  Larger layers do not gain by it (3096
-// tokens, top-8 of 64, 2048 / 1024: 511 without, 521 to 545 with).  Two waves of tiles or less run 128 columns
+// the layer writes - while the kernel before ends.  That saves 3 to 8 us of a layer, calls in a row, three layers'
+// weights in turn: 16 tokens, top-8 of 8 experts, hidden 7168, intermediate 2048 (16 rows per expert) 174 -> 168;
+// 52, top-4 of 8, 4096 / 1024 (26) 86 -> 81; 200, top-8 of 32, 2048 / 1024 (50) 143 -> 136; 380 of the same (95)
+// 143 -> 136; 1500, top-4 of 32 (188) 182 -> 178.  Layers of 300 us and more do not show it: 100, top-8 of 32,
+// 7168 / 2048 514 to 529 without, 517 to 539 with; 740, top-8 of 64, 2048 / 2048 (93) 341, 348 to 354; 3096,
+// top-8 of 64, 2048 / 1024 (387) 455 to 510, 505 to 513.  Two waves of tiles or less run 128 columns
 // wide (narrow_tiles in ops/moe.py).  Loading only the rows that a block has, in boxes of 32, cost the producer
 // more than it saved (511 -> 521).  What bounds a large layer is the power cap: a CTA pair per two row blocks,
 // which draws a third less out of L2, takes 2450 us instead of 2540 in a burst (4096 tokens, top-8 of 32) and as

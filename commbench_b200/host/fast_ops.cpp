@@ -1,8 +1,9 @@
 // Call path of the small operators without the Python work around a launch: argument checks, the result's
 // allocation, the current stream and the C entry point in one extension call.
 //
-// A decode-sized GEMM takes 5.9 us on the device; through Python attribute checks, `new_empty` and ctypes its
-// call took 8.9 us on the host, of which the entry point (tensor maps and launch) is 4.2.  Every function here
+// A decode-sized GEMM (16 x 8192 x 1024) takes 5.2 us with calls in a row; through Python attribute checks,
+// `new_empty` and ctypes its call took 8.9 us on the host, of which the entry point (tensor maps and launch) is 4.2.
+// A row quantisation takes 5.5 us on the host instead of 10.2.  Every function here
 // answers None for whatever it does not recognise - another type, layout or device, a tensor subclass, an
 // active dispatch or function mode, a launch that failed - and its caller in ops/ goes on with the general
 // path, which knows the errors.  The GIL is released around allocations and launches, which may block.

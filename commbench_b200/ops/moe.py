@@ -122,7 +122,8 @@ def narrow_tiles(avg_rows: float, experts: int, n: int, sms: int) -> bool:
     Measured, 256 / 128 wide for the whole layer, with three layers' weights in turn: 16 tokens, top-2 of 64,
     hidden 2048, intermediate 1024 (1.4 waves) 135-151 / 115 us; 64 tokens, top-2 of 16, 4096 / 2048 (1.7)
     197 / 196; 100 tokens, top-8 of 32, 7168 / 2048 (3.5) 551 / 567; 512 tokens, top-8 of 64 (6.9)
-    1085 / 1183."""
+    1085 / 1183.  A 128-wide tile is taken to cost 0.51 of a 256-wide one, so that of two widths with the same
+    last wave the wider one is kept."""
     if avg_rows > 96:
         return False
     blocks = experts * (1.0 - math.exp(-avg_rows))      # experts that a token selects
@@ -207,7 +208,7 @@ class MoELayer:
                        for r in range(self.W if self.emu else 1)]
         self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
         rows = tokens * topk / self.El
-        self.weights_early = rows <= 96      # a decode step: the products are bound by reading weights
+        self.weights_early = rows <= 96      # a decode step; csrc/moe/grouped_gemm.cu has both sides
         self.narrow_up = narrow_tiles(rows, self.El, 2 * intermediate, self.sms)
         self.narrow_down = narrow_tiles(rows, self.El, hidden, self.sms)
         torch.cuda.synchronize(dev)
