@@ -52,7 +52,7 @@ def _dense(sync):
     def start():
         x.copy_(x0)
 
-    return start, round_, lambda: (x, q, k, v, o, y, lse)
+    return start, round_, (x, q, k, v, o, y, lse), []
 
 
 def _experts(sync):
@@ -91,7 +91,7 @@ def _experts(sync):
     def start():
         x.copy_(x0)
 
-    return start, round_, lambda: (x, *seen)
+    return start, round_, (x, *seen), [layer.ctx for layer, _, _ in layers]
 
 
 @pytest.mark.parametrize("captured", [False, True])
@@ -99,7 +99,7 @@ def _experts(sync):
 def test_chain_gives_the_bits_of_single_calls(native_lib, chain, captured):
     results = []
     for sync in (torch.cuda.synchronize, lambda: None):
-        start, round_, buffers = chain(sync)
+        start, round_, buffers, contexts = chain(sync)
         start()
         round_()                                          # attributes of the kernels are set outside a capture
         start()
@@ -115,7 +115,10 @@ def test_chain_gives_the_bits_of_single_calls(native_lib, chain, captured):
         for _ in range(6):
             step()
         torch.cuda.synchronize()
-        results.append([t.clone() for t in buffers()])
+        results.append([t.clone() for t in buffers])
+        for ctx in contexts:
+            ctx.check_status()
+            ctx.close()
     for a, b in zip(*results):
         assert bool(torch.isfinite(a.float()).all())
         assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
